@@ -44,8 +44,8 @@ NCU_TRAFFIC = {
 }
 VARIANT_NAMES = {0: "auto", 1: "generic", 2: "tiled", 4: "tensor", 5: "tensor16"}
 ARITH = {"tensor16": "3xFP16 split on the tensor cores (x_hi*w_hi + x_lo*w_hi + x_hi*w_lo, 11-bit halves), FP32 "
-                     "accumulate, partial sums added on the CUDA cores every 48 MMAs; out-of-range activations "
-                     "recomputed in 3xTF32",
+                     "accumulate, partial sums added on the CUDA cores every 48 MMAs; tiles with out-of-range "
+                     "activations computed again with fitted scales",
          "tensor": "3xTF32 split on the tensor cores (x_hi*w_hi + x_lo*w_hi + x_hi*w_lo), FP32 accumulate, "
                    "partial sums added on the CUDA cores every 48 MMAs",
          "tiled": "FP32 FMA on the CUDA cores, taps added in the reference's (ic, r, s) order",

@@ -63,10 +63,10 @@ enum {
                                  16-byte aligned input                                    */
   TETRIS_VARIANT_TENSOR16 = 5 /* the same contraction in split FP16 (two 11-bit halves per
                                  operand, FP32 accumulate: FP32-accurate at twice the tensor
-                                 rate); stride 1, in_channel a multiple of 4 and >= 8, 16-byte
-                                 aligned input.  A launch whose largest |activation| is 2048
-                                 or more (NaN, infinity) or below 2^-8 is recomputed on the
-                                 device by the split-TF32 variant queued behind it         */
+                                 rate); strides 1-4, in_channel a multiple of 4 and >= 8,
+                                 16-byte aligned input.  Tiles whose largest |activation| is
+                                 2048 or more (infinity) or below 2^-8 are computed a second
+                                 time by the same launch with scales fitted to them        */
 };
 
 typedef struct tetris_filter tetris_filter_t; /* opaque; owns device buffers */
@@ -133,12 +133,13 @@ int tetris_filter_check(const tetris_filter_t *f);
  * Pointers need 4-byte alignment only; 16-byte aligned tensors take the vector paths (the
  * tensor-core variant needs a 16-byte aligned input and is not chosen without one).
  * Reproducibility: the list, generic and depthwise kernels add each output's taps in a fixed
- * order.  The tensor-core variant, on layers whose tiles fill the last wave of SMs badly, cuts
+ * order, and the split-FP16 tensor-core variant adds the slices of a K range it has cut in slice
+ * order.  The split-TF32 variant, on layers whose tiles fill the last wave of SMs badly, cuts
  * every tile's K range into 2-8 work items that ADD their partial results into the zeroed output
  * with floating-point atomics, in whatever order they finish: such a launch is not bit-identical
  * from run to run (differences of a few 1e-7 relative).  A filter created with
- * tetris_filter_opts_t.deterministic = 1 never splits and is bit-reproducible, at the cost of
- * the badly filled wave.
+ * tetris_filter_opts_t.deterministic = 1 never splits that way and is bit-reproducible, at the
+ * cost of the badly filled wave.
  */
 int tetris_conv2d_launch(const tetris_filter_t *f, const float *d_input_nhwc,
                          float *d_output_nhwc, int batch_size, int img_h, int img_w,

@@ -1,0 +1,99 @@
+"""GPU: the split-FP16 tensor-core kernel at the edges of its tile geometries -- strides 1 to 4 (input
+phases), stacked tiles (at most 64 channels), K ranges cut over a cluster, tiles of consecutive
+pixels, of whole padded rows and of 8-column blocks with several images, channel counts around
+the tiles' -- and its second pass for activations outside FP16's window."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # n, ic, h, w, oc, ks, stride, pad
+    (1, 64, 56, 56, 64, 3, 1, 1),      # stacked, small tiles
+    (2, 32, 65, 33, 63, 3, 2, 1),      # stacked, stride 2, one channel short
+    (3, 8, 17, 19, 65, 3, 3, 1),       # one channel past a stacked tile, stride 3
+    (2, 12, 31, 30, 130, 5, 4, 2),     # stride 4, 5x5, partial K chunk and channel tile
+    (1, 512, 14, 14, 256, 3, 1, 1),    # K range over a cluster of 8
+    (1, 100, 7, 7, 64, 3, 1, 1),       # stacked and cut into slices of unequal length
+    (9, 256, 7, 7, 128, 3, 1, 1),      # several images per tile, the last tile with one
+    (8, 1024, 13, 13, 255, 1, 1, 0),   # 1x1, 255 channels, slices
+    (2, 64, 9, 300, 96, 3, 1, 1),      # wide and flat
+    (2, 64, 300, 5, 40, 3, 1, 1),      # tall and thin
+    (5, 32, 28, 28, 128, 1, 2, 0),     # strided projection: one phase has a tap
+    (4, 16, 1, 1, 16, 1, 1, 0),        # one pixel per image
+    (2, 40, 12, 12, 260, 7, 1, 3),     # 7x7
+]
+
+
+def _run(tb, torch, f, x, stride, pad, relu):
+    n, ic, h, w = x.shape
+    oh, ow = tb.out_extent(h, f.kernel_size_, stride, pad), tb.out_extent(w, f.kernel_size_, stride, pad)
+    xin = torch.from_numpy(np.ascontiguousarray(x.transpose(0, 2, 3, 1))).cuda()
+    out = torch.full((n, oh, ow, f.out_channel_), float("nan"), device="cuda")
+    tb.sparse_conv2d_fused(f, xin, out, n, h, w, stride, pad, variant=tb.VARIANT_TENSOR16, relu=relu)
+    torch.cuda.synchronize()
+    f.check()
+    return out.cpu().numpy().transpose(0, 3, 1, 2)
+
+
+def _layer(case, seed):
+    n, ic, h, w, oc, ks, stride, pad = case
+    rng = np.random.default_rng(seed)
+    filt = rng.normal(0, 0.05, (oc, ic, ks, ks)).astype(np.float32)
+    filt[rng.random(filt.shape) < 0.8] = 0
+    return filt, rng.random((n, ic, h, w), dtype=np.float32) - 0.3
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "n%d_ic%d_%dx%d_oc%d_k%d_s%d_p%d" % c)
+def test_tile_geometries(tb, torch_cuda, oracle, case):
+    n, ic, h, w, oc, ks, stride, pad = case
+    filt, x = _layer(case, sum(case))
+    f = tb.SparseFilter(filt, ic, oc, ks)
+    want = oracle.host_conv2d(x, filt, stride, pad, threads=True, skip_zero=True)
+    got = _run(tb, torch_cuda, f, x, stride, pad, False)
+    assert not np.isnan(got).any(), "output elements were left unwritten"
+    assert oracle.compare(got, want)[0] == 0
+    again = _run(tb, torch_cuda, f, x, stride, pad, False)
+    assert np.array_equal(got, again)  # slices are added in slice order
+    assert oracle.compare(_run(tb, torch_cuda, f, x, stride, pad, True), np.maximum(want, 0))[0] == 0
+    f.close()
+
+
+@pytest.mark.parametrize("case", [(2, 96, 20, 20, 72, 3, 1, 1), (1, 64, 24, 24, 48, 3, 2, 1), (1, 512, 14, 14, 128, 1, 1, 0)],
+                         ids=lambda c: "n%d_ic%d_%dx%d_oc%d_k%d_s%d_p%d" % c)
+def test_activations_outside_the_window(tb, torch_cuda, oracle, case):
+    """All large, all tiny, and 2^-30 beside 2^13 in one tile: the bar of the path (1e-4 relative,
+    1e-5 absolute), with the absolute floor scaled like the data -- and for the mixed input like
+    the large values, whose FP32 rounding in the oracle itself is of that size."""
+    n, ic, h, w, oc, ks, stride, pad = case
+    filt, x = _layer(case, 7)
+    f = tb.SparseFilter(filt, ic, oc, ks)
+    for scale in (2.0 ** 14, 2.0 ** 60, 2.0 ** -12, 2.0 ** -70):
+        y = (x * np.float32(scale)).astype(np.float32)
+        want = oracle.host_conv2d(y, filt, stride, pad, threads=True)
+        got = _run(tb, torch_cuda, f, y, stride, pad, False)
+        assert oracle.compare(got / np.float32(scale), want / np.float32(scale))[0] == 0, scale
+    # channels of very different magnitude; an output that reads only the tiny ones keeps its
+    # relative accuracy although its tile holds the large ones (three bands of 16 binades)
+    mixed = x.copy()
+    mixed[:, : ic // 2] *= np.float32(2.0 ** 13)
+    mixed[:, ic // 2:] *= np.float32(2.0 ** -18)
+    split = filt.copy()
+    split[: oc // 2, ic // 2:] = 0      # reads the large channels
+    split[oc // 2:, : ic // 2] = 0      # reads the tiny ones
+    g = tb.SparseFilter(split, ic, oc, ks)
+    want = oracle.host_conv2d(mixed, split, stride, pad, threads=True)
+    got = _run(tb, torch_cuda, g, mixed, stride, pad, False)
+    for part, s in ((slice(0, oc // 2), 2.0 ** 13), (slice(oc // 2, oc), 2.0 ** -18)):
+        assert oracle.compare(got[:, part] / np.float32(s), want[:, part] / np.float32(s))[0] == 0
+    # an infinity spoils the outputs that read it, and no others
+    spiked = x.copy()
+    spiked[0, 3, 5, 5] = np.inf
+    got = _run(tb, torch_cuda, f, spiked, stride, pad, False)
+    want = oracle.host_conv2d(x, filt, stride, pad, threads=True)
+    far = np.ones(got.shape, bool)
+    far[0, :, max(0, 5 + pad - ks) // stride: (5 + pad) // stride + 1, max(0, 5 + pad - ks) // stride: (5 + pad) // stride + 1] = False
+    assert not np.isfinite(got[~far]).all()
+    assert oracle.compare(got[far], want[far])[0] == 0
+    f.close()
+    g.close()

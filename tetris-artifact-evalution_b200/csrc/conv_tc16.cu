@@ -1,115 +1,121 @@
-// Dense contraction on the 5th-generation tensor cores in SPLIT FP16: the stride-1 layers' fast
-// variant (tcgen05.mma kind::f16 + tcgen05.cp + TMEM + TMA).
+// Dense contraction on the 5th-generation tensor cores in SPLIT FP16: the fast variant of the
+// layers with 8 or more input channels (tcgen05.mma kind::f16 + TMEM + TMA).
 //
-// Arithmetic.  x = x_hi + x_lo and w' = w * 2^sh = w_hi + w_lo with *_hi the value rounded to
-// FP16 (11 significant bits) and *_lo the FP16-rounded remainder; D += x_hi*w_hi + x_lo*w_hi +
-// x_hi*w_lo in FP32 accumulators, scaled back by 2^-sh (exact) at the store; sh is chosen per
-// OUTPUT CHANNEL, so channels of very different magnitude keep their own full precision.  The products are
-// exact in FP32; what is dropped is x_lo*w_lo and the rounding of the remainders, about 2^-22 of
-// a product each -- the same as the split-TF32 variant (conv_tc.cu), at twice the tensor-core
-// rate and half the operand bytes.  sh puts a channel's largest |w'| at about 2^13: weights down
-// to 2^-17 of the channel's largest keep a normal FP16 remainder.  Activations are
-// scaled by a fixed 16 (their range is not known before the launch), which puts FP16's window at
-// |x| < 2048 with remainders exact down to |x| = 2^-7 and an absolute error of at most 2e-9 per
-// activation below that.  The conversion warps record the largest magnitude of the launch in
-// global memory; the launcher has queued the split-TF32 variant behind this kernel, which
-// starts, reads that maximum and recomputes the whole layer when it is 2048 or more (or NaN or
-// infinity) -- FP16 would overflow -- or below 2^-8 -- all activations so small that the
-// absolute error above would show in the relative accuracy -- and returns at once otherwise.
-// Results are therefore FP32-accurate for any input.
+// Arithmetic.  x' = 16 x = x_hi + x_lo and w' = w * 2^sh = w_hi + w_lo with *_hi the value rounded
+// to FP16 (11 significant bits) and *_lo the FP16-rounded remainder; D += w_hi*x_hi + w_hi*x_lo +
+// w_lo*x_hi in FP32 accumulators, scaled back by 2^-sh / 16 (exact) at the store; sh is chosen per
+// OUTPUT CHANNEL, so channels of very different magnitude keep their own full precision.  The
+// products are exact in FP32; what is dropped is w_lo*x_lo and the rounding of the remainders,
+// about 2^-22 of a product each -- the same as the split-TF32 variant (conv_tc.cu), at twice the
+// tensor-core rate.  sh puts a channel's largest |w'| at about 2^13.
 //
-// As in the split-TF32 variant the tensor core accumulates 48 MMAs (8 K steps) from zero into a
-// partial accumulator and CUDA-core warps add the partials to a running sum in registers (the
-// tensor core truncates when it adds into its accumulator; see conv_tc.cu).
+// Range.  FP16 has a window: |x| < 2048 after the fixed scale, absolute error of at most 2e-9 per
+// activation.  The converter warps of a CTA record the largest |x| they see; a CTA that finds it
+// outside [2^-8, 2048) runs its work items a second time with a scale taken from that maximum and
+// the activations cut into three bands of 16 binades, one pass over K per band, whose sums are
+// added up in FP32 (see kBands).  No second launch and no state between launches: what a CTA
+// recomputes is its own output.
 //
-// Structure.  GEMM view: M = 128 pixels = 16 groups of 8 consecutive output columns, N = 128
-// (64) output channels, K = (32-channel chunk, filter tap).  What differs from conv_tc.cu is how
-// the M-side operand reaches tensor memory.  There, converter warps rebuild the operand of every
-// tap from the activation patch (nine times per patch for a 3x3 filter) and that conversion, not
-// the tensor pipe, set the pace.  Here the patch is converted ONCE, in place, in shared memory
-// (each 128-byte row of 32 FP32 channels becomes 32 x_hi and 32 x_lo FP16 values), and the
-// operand of a tap is a WINDOW of the converted patch: tcgen05.cp copies 128 rows x 32 bytes from
-// shared to tensor memory through a matrix descriptor whose start address is shifted by the
-// tap's (row, column) offset and whose 8-row groups are PW rows apart (PW = patch width).  The
-// 128-byte swizzle is a function of the shared-memory address, so a window that starts at any
-// 128-byte row reads back exactly what the TMA load and the in-place conversion wrote.
-//   * warp 0 (one thread): one TMA load per 32-channel chunk of the tile's pixels with their
-//     halo (4-D box, out-of-range coordinates zero-filled = the padding) into a ring of stages;
-//   * warps 4-7: convert a landed patch in place, one 128-byte row per thread, conflict-free;
-//   * warp 3 (one elected lane): per K step four tcgen05.cp (x_hi and x_lo, two K slices each)
-//     into one of the operand blocks; per GROUP of U K steps (U = 2, or 4 for 64-channel tiles
-//     under filters larger than 1x1) one wait (the MMAs that read the block a lap ago are done)
-//     and one commit;
-//   * warp 2 (one thread): one bulk copy per group of K steps of prepared {w_hi, w_lo} tile images;
-//   * warp 1 (one elected lane): 6 tcgen05.mma per K step; per group two waits (operands copied,
-//     weights landed) and one commit.  The pipeline's unit is a group of K steps because a wait
-//     costs a warp ~200 clocks and a commit ~250, against ~450 for the twelve MMAs of a pair;
-//   * warps 8-15: partial accumulators -> running sum in registers -> staged, coalesced stores.
+// The tensor core truncates when it adds into its FP32 accumulator, so the accumulation chain is
+// cut every 8 K steps (48 MMAs): the tensor core accumulates from zero into one of two partial
+// accumulators and CUDA-core warps add the partials to a running sum in registers.
+//
+// Structure.  D[channel][pixel]: the M side is 128 output channels (the weights), the N side up to
+// 256 output pixels (the activations), K = (32-channel chunk, filter tap).  Both operands are read
+// from shared memory.  Why this way round and this size: an MMA of M = 128 reads 128 x 32 bytes of
+// A and N x 32 bytes of B from shared memory (128 bytes/clock) and computes for N/2 clocks, so
+// N = 128 needs the whole shared-memory pipe while N = 256 leaves a quarter of it for the weight
+// copies and the conversion; with the weights on the M side one 16 KB weight image serves 256
+// pixels (L2 -> SM weight traffic halved against 128-pixel tiles), and an accumulator row is an
+// output channel, so a warp stores one pixel's 32 consecutive channels as one 128-byte line
+// without staging, whatever the channel count or alignment.
+//   * warp 0 (one thread): TMA loads of activation patches (tile + halo, 32 channels, out-of-range
+//     coordinates zero-filled = the padding) and bulk copies of weight images, each into a ring;
+//   * converter warps: a landed patch, once, in place: each 128-byte row of 32 FP32 channels
+//     becomes {x_hi[32], x_lo[32]} FP16;
+//   * warp 1 (one elected lane): the MMAs.  The B operand of a tap is a WINDOW of the converted
+//     patch: a descriptor whose start is shifted by the tap's (row, column) and whose 8-pixel
+//     groups are one patch row apart.  The 128-byte swizzle is a function of the shared-memory
+//     address, so a window that starts at any 128-byte row reads back what TMA wrote;
+//   * eight summing warps: partial accumulators -> running sums -> global memory.
+// At stride S the input splits into S x S phases; each phase is a patch of its own (TMA element
+// strides) whose taps read it at stride 1, so a phase is loaded and converted once per chunk.
+// Filters with at most 64 output channels stack {w_hi, w_lo} on the M side: one MMA multiplies
+// both halves, 4 MMAs per K step instead of 6; the halves are added in the epilogue.
+// Few tiles (small batches, deep layers): the K range of a tile is cut over a cluster of up to 8
+// CTAs, whose sums meet in distributed shared memory and are added in slice order (bit-reproducible,
+// no zeroing of the output, ReLU-fusable).
 // Every barrier wait is bounded; on a timeout an error flag is raised, all roles drain, TMEM is
 // freed and the kernel returns; the host reports TETRIS_ERR_CUDA.
-//
-// 1x1 filters take the same pipeline with M = 128 consecutive pixels of the flattened image
-// (no halo, 100 % full tiles).  Mid-size images (28 x 28, 52 x 52 ...), which 8 x 16 tiles cut
-// badly, are walked in their padded-width layout instead (`flat`, see launch_conv_tc16).  Covers stride 1, IC % 4 == 0 (TMA strides), KS <= 7.
-// No cluster launch: every load is issued by one CTA for itself.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
-#include <cstdlib>
+#include <cstring>
 #include <mutex>
+#include <new>
 
 #include "internal.h"
 
 namespace tetris {
 namespace {
 
-constexpr int BM = 128, KC = 32;         // tile rows (pixels); K chunk (32 channels)
-constexpr int kTW = 8, kTH = 16;         // a tile is 16 groups of 8 output columns
-constexpr int kAStagesMax = 4;           // operand blocks in tensor memory: one per group of U K steps, 256 / (32 U) of them
-constexpr int kStepCols = 32;            // per K step {x_hi k0, x_hi k1, x_lo k0, x_lo k1} x 8 columns
-constexpr int kTmemCols = 512;           // 2 partial accumulators (<= 128 columns each) + 8 x 32 operand columns
-constexpr int kTmemA = 256;
-constexpr int kWStagesMax = 4, kXStagesMax = 6;   // weight stages hold a group of K steps
-constexpr int kGroups = 16;              // "group done" barriers in rotation (a power of two, 2^4: see wait_group)
-constexpr int kSuperSteps = 8;           // K steps (48 MMAs) accumulated on the tensor core before the FP32 add outside
-constexpr int kThreads = 512;            // warp 0 x loads, 1 MMA, 2 w loads, 3 cp, 4-7 convert, 8-15 sum + store
-constexpr int kStoreBytes = 8 * 4096;    // store staging: per summing warp 32 rows x 32 channels
-constexpr int kNumBars = 3 * kXStagesMax + kWStagesMax + kAStagesMax + kGroups + 2 + 2;   // (... + two drain barriers + two partial-sum barriers)
+constexpr int BM = 128, KC = 32;         // channels of a tile; K chunk (32 input channels)
+constexpr int kTW = 8;                   // a pixel group is 8 consecutive output columns
+constexpr int kXStagesMax = 6, kWStagesMax = 8;
+constexpr int kSuper = 8;                // K steps accumulated on the tensor core before the FP32 add outside
+constexpr int kSumWarps = 8;
+constexpr int kBands = 3, kBandBits = 16;  // second pass: bands of 16 binades below the largest activation
+// Per summing warp: two blocks of 16 pixels x 32 channels on their way to the output, and for
+// stacked tiles 32 pixels x 32 accumulator lanes handed to the warp with the other half.
+__host__ __device__ constexpr int stage_bytes(bool stack) { return kSumWarps * (4096 + (stack ? 4096 : 0)); }
+constexpr int kNumBars = 3 * kXStagesMax + 2 * kWStagesMax + 6;  // (even: what follows is read 16 bytes at a time)
 constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr float kXScale = 16.f;          // activations are multiplied by this before the split (undone in out_scale)
 
+enum { kLinear = 0, kFlat = 1, kGrid = 2 };
+
+// Division of 0 <= n < 2^31 by a launch constant: q = (umulhi(n, mul) + n) >> shift with
+// shift = ceil(log2 d) and mul = floor(2^32 (2^shift - d) / d) + 1 (the items' coordinates are worked
+// out by every role; an integer division costs a warp ~100 clocks).
+struct FastDiv {
+  uint32_t d, mul, shift;
+};
+FastDiv fast_div(uint32_t d) {
+  FastDiv f;
+  f.d = d; f.shift = 0;
+  while ((1ull << f.shift) < d) ++f.shift;
+  f.mul = (uint32_t)(((1ull << 32) * ((1ull << f.shift) - d)) / d + 1);
+  return f;
+}
+__device__ __forceinline__ int quot(int n, const FastDiv &f) { return (int)((__umulhi((uint32_t)n, f.mul) + (uint32_t)n) >> f.shift); }
+
 struct Tc16Params {
   float *out;
-  int N, OH, OW, OC, P, KS;
-  int linear;                  // 1x1 filters: a tile is 128 consecutive pixels of the flattened N*OH*OW image
-  int flat;                    // a tile is 128 consecutive positions of one image laid out with its padded width
-                               // PW = W + 2P (positions past OW in a row are computed and dropped)
-  int PW;                      // patch width in pixels (kTW + KS - 1; flat mode: W + 2P); 8 in linear mode
-  int PHI;                     // patch rows one image occupies in a stage
-  int TH, NB;                  // output rows and images of a tile
+  int N, OH, OW, OC, S, P, KS;
+  int mode;                    // kLinear: 1x1 filters at stride 1, a tile is `npx` consecutive pixels of the batch;
+                               // kFlat: `npx` consecutive positions of one image laid out with its padded width PW
+                               // (positions past OW in a row are computed and dropped);
+                               // kGrid: 8 columns x TH rows x NB images
+  int npx;                     // pixels of a tile = N of the MMAs, a multiple of 16
+  int PW;                      // patch width in pixels
+  int PHI;                     // patch rows of one image
+  int TH, NB;                  // kGrid: output rows and images of a tile
   int box_rows;                // 128-byte rows a patch load delivers
-  int x_stage_bytes, n_x;      // activation stage size and ring depth
-  int n_w;                     // weight ring depth
-  int tiles_w, tiles_h, tiles_n;
-  int n_chunks, ksplit;
-  // Tail split: the tiles that would form a last, nearly empty wave of CTAs (tiles tail_tile0 ...)
-  // are cut into tail_d K slices each (work items tail_start ...); the slices leave their sums in
-  // `scratch`, and whichever finishes last (tail_count) adds them up in slice order and stores.
-  int tail_start, tail_tile0, tail_d;
-  float *scratch;
-  int *tail_count;
-  int relu;                    // max(y, 0) at the store (never together with a split K range)
-  long long total_pixels;      // N * OH * OW (linear mode)
+  int x_stage_bytes, n_x, n_w;
+  int tiles_w, tiles_h, tiles_n, oc_tiles, total_tiles;
+  FastDiv by_oc_tiles, by_tiles_w, by_tiles_h, by_PW, by_PHI;
+  int n_chunks;
+  int d;                       // CTAs of a cluster = slices of a tile's K range
+  int relu;                    // max(y, 0) at the store
+  int tma_store;               // pixel groups leave through TMA stores (channel count and alignment allow it)
+  long long total_pixels;      // N * OH * OW
   const float *out_scale;      // per output channel: 2^-sh[oc] / 16 (undoes the weight and activation scaling)
   int *error_flag;
-  unsigned *gate;              // gate[0]: largest |activation| of the launch, as FP32 bits (see launch_conv_tc_gated)
   const __half *w_tiles;
   unsigned spin_limit;         // polls after which a barrier wait gives up (0: kSpinLimit)
   int withhold_first_load;     // failure-detection test only: every CTA leaves out its first activation load
-  long long *prof;             // per-role clock totals of CTA 0 for TETRIS_TC16_PROF=1 (nullptr = off)
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -125,6 +131,13 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+// (does not suspend the thread: for the loader, which polls two rings)
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
@@ -162,9 +175,11 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-// K-major operand, 128-byte rows, 128B swizzle; 8-row groups `sbo_bytes` apart.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t sbo_bytes) {
-  return (uint64_t)((saddr >> 4) & 0x3FFF) | (1ull << 16) | ((uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32) | (1ull << 46) | (2ull << 61);
+// K-major operand; 8-row groups `sbo_bytes` apart; layout 2 = 128-byte rows with the 128B swizzle,
+// 4 = 64-byte rows with the 64B swizzle.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t sbo_bytes, uint32_t layout) {
+  return (uint64_t)((saddr >> 4) & 0x3FFF) | (1ull << 16) | ((uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32) | (1ull << 46) |
+         ((uint64_t)layout << 61);
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -174,15 +189,13 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(pred));
   return pred != 0;
 }
-// shared -> tensor memory: 128 rows x 32 bytes into 8 columns
-__device__ __forceinline__ void tmem_cp(uint32_t taddr, uint32_t d_lo, uint32_t d_hi) {
-  asm volatile("{\n.reg .b64 d;\nmov.b64 d, {%1, %2};\ntcgen05.cp.cta_group::1.128x256b [%0], d;\n}" ::"r"(taddr), "r"(d_lo), "r"(d_hi) : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem descriptor], FP16 operands, FP32 accumulate
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t db_lo, uint32_t db_hi, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\n.reg .b64 d;\nmov.b64 d, {%2, %3};\nsetp.ne.b32 p, %5, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %4, p;\n}"
-               ::"r"(tmem_d), "r"(tmem_a), "r"(db_lo), "r"(db_hi), "r"(idesc), "r"(accumulate) : "memory");
+// D[tmem] (+)= A[smem] * B[smem], FP16 operands, FP32 accumulate.  The descriptors are passed as
+// words: the high ones are constants, the low ones a start address plus a constant.
+__device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint32_t da_lo, uint32_t da_hi, uint32_t db_lo, uint32_t db_hi,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p;\n.reg .b64 da, db;\nmov.b64 da, {%1, %2};\nmov.b64 db, {%3, %4};\nsetp.ne.b32 p, %6, 0;\n"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}"
+               ::"r"(tmem_d), "r"(da_lo), "r"(da_hi), "r"(db_lo), "r"(db_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -191,49 +204,74 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
                : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+                 "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<const uint32_t *>(&h);
 }
+__device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(min(127, max(-126, e)) + 127) << 23); }
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr, uint32_t rank) {
+  float4 v;
+  asm volatile("{\n.reg .b32 r;\nmapa.shared::cluster.u32 r, %4, %5;\nld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [r];\n}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
 
-// BN: output channels of a tile.  U: K steps per pipeline group -- the unit the copy warp and the
-// MMA warp wait, issue and commit by (2 for BN = 128; 4 for BN = 64, whose MMAs are short enough
-// that a wait and a commit per pair of steps would set the pace).
-template <int BN, int U>
-__global__ void __launch_bounds__(kThreads, 1)
-conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const Tc16Params p) {
+// NMAX: most pixels of a tile.  A summing warp keeps NMAX / 2 running sums per thread, which sets
+// the register count: 12 warps (2 of them converters) for 256 pixels, 16 warps (6 converters) for
+// 128.  STACK: at most 64 output channels, {w_hi, w_lo} stacked on the M side.
+template <int NMAX> struct Roles {
+  static constexpr int kConv = NMAX == 256 ? 2 : 6;
+  static constexpr int kFirstSum = 2 + kConv;
+  static constexpr int kThreads = 32 * (kFirstSum + kSumWarps);
+};
+
+template <int NMAX, bool STACK>
+__global__ void __launch_bounds__(Roles<NMAX>::kThreads, 1)
+conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_out, const Tc16Params p) {
+  constexpr int kConv = Roles<NMAX>::kConv, kFirstSum = Roles<NMAX>::kFirstSum, kThreads = Roles<NMAX>::kThreads;
+  constexpr int kWBytes = STACK ? 8192 : 16384;   // weights of one K step
+  constexpr int kOcTile = STACK ? 64 : 128;       // output channels of a tile
+  constexpr int NC = NMAX / 2;                    // running sums (pixels) per summing thread, at most
+  constexpr int kTmemCols = 2 * NMAX;             // two partial accumulators
   extern __shared__ unsigned char smem_raw[];
   unsigned char *xbase = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
   unsigned char *wbase = xbase + (size_t)p.n_x * p.x_stage_bytes;
-  constexpr int kWBytes = BN * 128;      // weights of one K step: BN rows of {w_hi (64 B), w_lo (64 B)}; a stage holds U
-  constexpr int kAStages = 256 / (kStepCols * U);   // operand blocks in rotation (a power of two)
-  constexpr int kSuper = kSuperSteps / U;           // groups per partial sum
-  static_assert(kAStages <= kAStagesMax && kAStages * kStepCols * U == 256 && kSuper * U == kSuperSteps, "group size");
-  unsigned char *store_base = wbase + (size_t)p.n_w * U * kWBytes;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(store_base + kStoreBytes);
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + kNumBars);
+  unsigned char *exch = wbase + (size_t)p.n_w * kWBytes;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(exch + stage_bytes(STACK));
+  int4 *gtabs = reinterpret_cast<int4 *>(bars + kNumBars);  // per summing warp: where each of its 8-pixel groups goes
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(gtabs + kSumWarps * (NC / 8));
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  unsigned *seen_slot = tmem_slot + 3;            // largest |activation| of this CTA, FP32 bits
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   auto bar_xfull = [&](int s) { return smem_u32(&bars[s]); };
   auto bar_xconv = [&](int s) { return smem_u32(&bars[kXStagesMax + s]); };
   auto bar_xempty = [&](int s) { return smem_u32(&bars[2 * kXStagesMax + s]); };
   auto bar_wfull = [&](int s) { return smem_u32(&bars[3 * kXStagesMax + s]); };
-  auto bar_afull = [&](int s) { return smem_u32(&bars[3 * kXStagesMax + kWStagesMax + s]); };
-  auto bar_gdone = [&](int c) { return smem_u32(&bars[3 * kXStagesMax + kWStagesMax + kAStagesMax + c]); };
-  auto bar_pempty = [&](int b) { return smem_u32(&bars[kNumBars - 2 + b]); };
-  auto bar_drain = [&](int b) { return smem_u32(&bars[kNumBars - 4 + b]); };
+  auto bar_wempty = [&](int s) { return smem_u32(&bars[3 * kXStagesMax + kWStagesMax + s]); };
+  auto bar_pfull = [&](int b) { return smem_u32(&bars[kNumBars - 6 + b]); };
+  auto bar_pempty = [&](int b) { return smem_u32(&bars[kNumBars - 4 + b]); };
+  auto bar_drain = [&]() { return smem_u32(&bars[kNumBars - 2]); };
 
   if (tid == 0) {
-    for (int s = 0; s < kXStagesMax; ++s) { mbar_init(bar_xfull(s), 1); mbar_init(bar_xconv(s), 4); mbar_init(bar_xempty(s), 1); }
-    for (int s = 0; s < kWStagesMax; ++s) mbar_init(bar_wfull(s), 1);
-    for (int s = 0; s < kAStages; ++s) mbar_init(bar_afull(s), 1);
-    for (int c = 0; c < kGroups; ++c) mbar_init(bar_gdone(c), 1);
-    for (int b = 0; b < 2; ++b) { mbar_init(bar_pempty(b), 8); mbar_init(bar_drain(b), 1); }
+    for (int s = 0; s < kXStagesMax; ++s) { mbar_init(bar_xfull(s), 1); mbar_init(bar_xconv(s), kConv); mbar_init(bar_xempty(s), 1); }
+    for (int s = 0; s < kWStagesMax; ++s) { mbar_init(bar_wfull(s), 1); mbar_init(bar_wempty(s), 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(bar_pfull(b), 1); mbar_init(bar_pempty(b), kSumWarps); }
+    mbar_init(bar_drain(), 1);
     abort_flag[0] = 0;
     abort_flag[1] = (int)(p.spin_limit ? p.spin_limit : kSpinLimit);
+    *seen_slot = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
   }
-  if (warp == 1) {  // the whole tensor memory of the SM: this kernel runs one CTA per SM
+  if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -241,497 +279,550 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const Tc16Params p) 
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  // Timeline aid, compiled in with -DTETRIS_TC16_PROF only: clocks per role of CTA 0, in total
-  // and inside its waits, printed by the launcher when the environment has TETRIS_TC16_PROF=1.
-#ifdef TETRIS_TC16_PROF
-  const bool prof_on = p.prof != nullptr && blockIdx.x == 0;
-  long long pw[7] = {0, 0, 0, 0, 0, 0, 0};
-  const long long prof_t0 = prof_on ? clock64() : 0;
-#define TIMED(slot, expr) ([&]() { const long long t0_ = prof_on ? clock64() : 0; const bool r_ = (expr); if (prof_on) pw[slot] += clock64() - t0_; return r_; }())
-#define PROF_OUT(role) do { if (prof_on && lane == 0) { p.prof[(role) * 8] = clock64() - prof_t0; for (int i_ = 0; i_ < 7; ++i_) p.prof[(role) * 8 + 1 + i_] = pw[i_]; } } while (0)
-#define PROF_LAP(slot) do { if (prof_on) { const long long n_ = clock64(); pw[slot] += n_ - ts0; ts0 = n_; } } while (0)
-#define PROF_START() long long ts0 = prof_on ? clock64() : 0
-#else
-#define TIMED(slot, expr) (expr)
-#define PROF_OUT(role) do { } while (0)
-#define PROF_LAP(slot) do { } while (0)
-#define PROF_START() do { } while (0)
-#endif
 
-  // Persistent CTA: work items blockIdx.x, blockIdx.x + gridDim.x, ...; the channel tile is the
-  // fastest index, so CTAs that run side by side read the same activation patch.
+  // Work items: tile blockIdx.x / d, + gridDim.x / d, ... (d > 1: exactly one).  The channel tile
+  // is the fastest index, so CTAs that run side by side read the same activation patch.
+  const int rank = p.d > 1 ? (int)(blockIdx.x % p.d) : 0;
+  const int tile0 = blockIdx.x / p.d, tile_step = gridDim.x / p.d;
+  const int chunk0 = p.n_chunks * rank / p.d, chunk1 = p.n_chunks * (rank + 1) / p.d;
   const int taps = p.KS * p.KS;
-  const int oc_tiles = (p.OC + BN - 1) / BN;
-  const int total_tiles = p.tiles_w * p.tiles_h * p.tiles_n * oc_tiles;
-  const int total_items = p.tail_start + (total_tiles - p.tail_tile0) * p.tail_d;
-  // A work item is a tile, or one of ksplit equal slices of a tile's K range (all tiles), or --
-  // for the tiles of the last wave -- one of tail_d slices.  The pipeline's unit is a GROUP of U K
-  // steps (the last of an item may be shorter).
-  struct Item { int tile, chunk0, chunks, iters, ngroups, supers; bool tail; int slice; };
-  auto item_of = [&](int t) {
-    Item it;
-    it.tail = t >= p.tail_start;
-    const int d = it.tail ? p.tail_d : p.ksplit, u = it.tail ? t - p.tail_start : t;
-    it.slice = u % d;
-    it.tile = (it.tail ? p.tail_tile0 : 0) + u / d;
-    it.chunks = p.n_chunks / d;
-    it.chunk0 = it.slice * it.chunks;
-    it.iters = taps * it.chunks;
-    it.ngroups = (it.iters + U - 1) / U;
-    it.supers = (it.ngroups + kSuper - 1) / kSuper;
-    return it;
+  const int iters = taps * (chunk1 - chunk0);       // K steps of an item (per band)
+  const int supers = (iters + kSuper - 1) / kSuper;
+  const int phases = min(p.S, p.KS);                // input phases per axis that a tap falls into
+  auto decode = [&](int t, int &oc0, int &w0, int &h0, int &n0) {
+    int u = quot(t, p.by_oc_tiles);
+    oc0 = (t - u * p.oc_tiles) * kOcTile;
+    t = quot(u, p.by_tiles_w);
+    w0 = u - t * p.tiles_w;                         // kLinear, kFlat: number of the tile; kGrid: tile column
+    u = quot(t, p.by_tiles_h);
+    h0 = (t - u * p.tiles_h) * p.TH;
+    n0 = u * p.NB;
   };
-  auto decode = [&](int t, int &w0, int &h0, int &n0, int &oc0) {
-    oc0 = (t % oc_tiles) * BN; t /= oc_tiles;
-    w0 = (t % p.tiles_w) * kTW; t /= p.tiles_w;       // (linear mode: tiles_w = number of 128-pixel tiles)
-    h0 = (t % p.tiles_h) * p.TH;
-    n0 = (t / p.tiles_h) * p.NB;
+  // output pixel of column j of a tile, -1 where it is none
+  auto pixel_of = [&](int j, int w0, int h0, int n0) -> int {
+    if (p.mode == kLinear) {
+      const long long px = (long long)w0 * p.npx + j;
+      return px < p.total_pixels ? (int)px : -1;
+    }
+    int oh, ow, n = n0;
+    bool in = true;
+    if (p.mode == kFlat) {
+      const int pos = w0 * p.npx + j;
+      oh = quot(pos, p.by_PW); ow = pos - oh * p.PW;
+    } else {
+      const int g = j >> 3, i = p.NB > 1 ? quot(g, p.by_PHI) : 0;
+      oh = g - i * p.PHI; ow = w0 * kTW + (j & 7); n = n0 + i;
+      in = i < p.NB && oh < p.TH;
+      oh += h0;
+    }
+    return in && oh < p.OH && ow < p.OW && n < p.N ? (n * p.OH + oh) * p.OW + ow : -1;
   };
-  // Group G of this CTA (counted across work items) signals bar_gdone(G % kGroups) when its MMAs
-  // have completed.  Nobody looks at a group's barrier later than 16 groups after it: the rings are
-  // at most 4 groups deep and the MMAs run at most two partial sums (8 groups) ahead of the summing warps.
-  auto wait_group = [&](int G) { return mbar_wait(bar_gdone(G & (kGroups - 1)), (G >> 4) & 1, abort_flag); };
-  auto wait_group_warp = [&](int G) { return mbar_wait_warp(bar_gdone(G & (kGroups - 1)), (G >> 4) & 1, abort_flag); };
 
-  if (warp == 0) {
-    // ---- activation loads: one patch (tile + halo) per 32-channel chunk ----
-    if (lane == 0) {
-      const uint32_t box_bytes = (uint32_t)p.box_rows * 128u;
-      int s = 0, loads = 0;
-      uint32_t phase = 1;  // (a fresh barrier lets the first lap through)
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x) {
-        const Item it = item_of(t);
-        int w0, h0, n0, oc0;
-        decode(it.tile, w0, h0, n0, oc0);
-        for (int chunk = it.chunk0; chunk < it.chunk0 + it.chunks; ++chunk) {
-          if (!(ok = TIMED(0, mbar_wait(bar_xempty(s), phase, abort_flag)))) break;
-          if (loads++ == 0 && p.withhold_first_load) {  // (test: this patch never arrives, its readers give up)
-            if (++s == p.n_x) { s = 0; phase ^= 1u; }
-            continue;
+  // Pipeline positions; they run on through the passes.
+  int sx = 0, sw = 0;                 // stage of the activation ring / weight ring
+  uint32_t px = 0, pw = 0;            // parity of the current lap of either ring
+  int sp = 0;                         // partial sums so far
+  int trades = 0;                     // blocks given and taken (stacked tiles)
+  int x_loads = 0, w_loads = 0;
+  bool ok = true;
+  // Pass 0: scale 16.  If it saw an infinity, pass 1 repeats it looking for the largest FINITE
+  // activation.  If the largest one lies outside FP16's window a last, banded pass follows.
+  bool first = true, banded = false;
+  int emax = 0;                       // exponent of the largest activation (banded pass)
+  for (;;) {
+    const int bands = banded ? kBands : 1;
+    auto band_exp = [&](int b) { return banded ? min(127, 14 - emax + kBandBits * b) : 4; };  // scale of band b: 2^that
+    if (warp == 0) {
+      // ---- loads: two independent cursors (patches, weight images) polled in turn ----
+      if (lane == 0) {
+        const uint32_t box_bytes = (uint32_t)p.box_rows * 128u;
+        int xt = tile0, xb = 0, xc = chunk0, xr = 0, xq = 0, oc_, w0, h0, n0;
+        int wt = tile0, wb = 0, wc = chunk0, wpr = 0, wpq = 0, wr = 0, wq = 0;
+        bool x_left = xt < p.total_tiles && iters > 0, w_left = x_left;
+        if (x_left) decode(xt, oc_, w0, h0, n0);
+        const __half *wsrc = p.w_tiles + (size_t)(wt - quot(wt, p.by_oc_tiles) * p.oc_tiles) * p.n_chunks * taps * (kWBytes / 2);
+        uint32_t idle = 0;
+        const uint32_t limit = (uint32_t)abort_flag[1];
+        while (x_left || w_left) {
+          bool moved = false;
+          if (x_left && mbar_test(bar_xempty(sx), px ^ 1u)) {
+            moved = true;
+            if (x_loads++ != 0 || !p.withhold_first_load) {  // (test: that patch never arrives, its readers give up)
+              const uint32_t dst = smem_u32(xbase + (size_t)sx * p.x_stage_bytes);
+              mbar_expect_tx(bar_xfull(sx), box_bytes);
+              if (p.mode == kLinear)
+                tma_load_4d(dst, &map_x, bar_xfull(sx), xc * KC, w0 * p.npx, 0, 0);
+              else if (p.mode == kFlat)  // whole padded rows, from the row of the tile's first position
+                tma_load_4d(dst, &map_x, bar_xfull(sx), xc * KC, xq - p.P, quot(w0 * p.npx, p.by_PW) * p.S + xr - p.P, n0);
+              else
+                tma_load_4d(dst, &map_x, bar_xfull(sx), xc * KC, w0 * kTW * p.S + xq - p.P, h0 * p.S + xr - p.P, n0);
+            }
+            if (++sx == p.n_x) { sx = 0; px ^= 1u; }
+            if (++xq == phases) {
+              xq = 0;
+              if (++xr == phases) {
+                xr = 0;
+                if (++xc == chunk1) {
+                  xc = chunk0;
+                  if (++xb == bands) {
+                    xb = 0;
+                    xt += tile_step;
+                    x_left = xt < p.total_tiles;
+                    if (x_left) decode(xt, oc_, w0, h0, n0);
+                  }
+                }
+              }
+            }
           }
-          mbar_expect_tx(bar_xfull(s), box_bytes);
-          if (p.linear)
-            tma_load_4d(smem_u32(xbase + (size_t)s * p.x_stage_bytes), &map_x, bar_xfull(s), chunk * KC, (w0 / kTW) * BM, 0, 0);
-          else if (p.flat)  // whole padded rows, from the row above the tile's first output row
-            tma_load_4d(smem_u32(xbase + (size_t)s * p.x_stage_bytes), &map_x, bar_xfull(s), chunk * KC, -p.P,
-                        ((w0 / kTW) * BM) / p.PW - p.P, n0);
-          else
-            tma_load_4d(smem_u32(xbase + (size_t)s * p.x_stage_bytes), &map_x, bar_xfull(s), chunk * KC, w0 - p.P, h0 - p.P, n0);
-          if (++s == p.n_x) { s = 0; phase ^= 1u; }
-        }
-      }
-      if (!ok || *abort_flag) {  // the loads of the last lap may still be in flight
-        for (int v = max(loads - p.n_x, p.withhold_first_load ? 1 : 0); v < loads; ++v)
-          mbar_drain(bar_xfull(v % p.n_x), (uint32_t)(v / p.n_x) & 1u);
-      }
-      PROF_OUT(0);
-    }
-  } else if (warp == 2) {
-    // ---- weight loads: one bulk copy per group (the {w_hi, w_lo} images of its K steps lie
-    //      back to back in global memory) ----
-    if (lane == 0) {
-      int G = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x) {
-        const Item it = item_of(t);
-        const int iters = it.iters, ngroups = it.ngroups;
-        int w0, h0, n0, oc0;
-        decode(it.tile, w0, h0, n0, oc0);
-        const __half *item = p.w_tiles + ((size_t)(oc0 / BN) * p.n_chunks + it.chunk0) * taps * (size_t)(BN * 64);
-        for (int j = 0; j < ngroups; ++j, ++G) {
-          const int s = G % p.n_w;
-          if (G >= p.n_w && !(ok = TIMED(0, wait_group(G - p.n_w)))) break;
-          const uint32_t bytes = (uint32_t)(min(U, iters - U * j) * kWBytes);
-          mbar_expect_tx(bar_wfull(s), bytes);
-          bulk_load(smem_u32(wbase + (size_t)s * U * kWBytes), item + (size_t)(U * j) * (BN * 64), bytes, bar_wfull(s));
-        }
-      }
-      if (!ok || *abort_flag) {  // the copies of the last lap may still be in flight
-        for (int v = max(G - p.n_w, 0); v < G; ++v) mbar_drain(bar_wfull(v % p.n_w), (uint32_t)(v / p.n_w) & 1u);
-      }
-      PROF_OUT(1);
-    }
-  } else if (warp == 3) {
-    // ---- operand copies (converged warp, one elected lane issues, so that descriptors and
-    //      addresses stay in uniform registers): per K step four tcgen05.cp -- the tap's window of
-    //      the converted patch -> the step's operand block in tensor memory; one wait and one
-    //      commit per pair.  Everything that depends on the K step is counted along: the issuing
-    //      thread's own instructions, not the tensor unit, set the pace otherwise. ----
-    const uint32_t sbo = (uint32_t)((p.linear || p.flat) ? 1024 : p.PW * 128);
-    const uint32_t da_hi = (uint32_t)(smem_desc(0, sbo) >> 32);
-    const uint32_t x0 = (uint32_t)smem_desc(smem_u32(xbase), sbo);       // descriptor (low word) of stage 0, tap (0, 0)
-    const uint32_t stage_step = (uint32_t)(p.x_stage_bytes >> 4);        // ... one stage further
-    const uint32_t row_step = (uint32_t)((p.PW - p.KS + 1) * 128 >> 4);  // ... from the end of a filter row to the next row
-    int G = 0, sx = 0;
-    uint32_t xd = x0, td = 0;  // descriptor of the current stage; offset of the current tap
-    uint32_t xphase = 0;       // phase of the "converted" barrier of stage sx
-    bool fresh_patch = true;   // the patch in stage sx has not been waited for yet
-    bool ok = true;
-    for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x) {
-      int r = 0, q = 0;  // tap of the next K step
-      // flat mode: the tile's first position lies (P0 mod PW) rows into its first padded row
-      const Item it = item_of(t);
-      const int iters = it.iters, ngroups = it.ngroups;
-      uint32_t td0 = 0;
-      if (p.flat) {
-        const int P0 = ((it.tile / oc_tiles) % p.tiles_w) * BM;
-        td0 = (uint32_t)((P0 - (P0 / p.PW) * p.PW) * 8);
-      }
-      td = td0;
-      for (int j = 0; j < ngroups; ++j, ++G) {
-        const int sa = G & (kAStages - 1);
-        const int ns = min(U, iters - U * j);
-        // the MMAs that read this operand block (kAStages groups ago) are done
-        if (G >= kAStages && !(ok = TIMED(0, wait_group_warp(G - kAStages)))) break;
-        // per step: the window of its tap in the converted patch (waited for once per patch), and
-        // the barrier that releases the patch if this step is its last
-        uint32_t a[U], freed[U];
-#pragma unroll
-        for (int e = 0; e < U; ++e) {
-          a[e] = 0; freed[e] = 0;
-          if (e < ns && ok) {
-            if (fresh_patch) {
-              ok = TIMED(1, mbar_wait_warp(bar_xconv(sx), xphase, abort_flag));
-              fresh_patch = false;
+          if (w_left && mbar_test(bar_wempty(sw), pw ^ 1u)) {
+            moved = true;
+            mbar_expect_tx(bar_wfull(sw), (uint32_t)kWBytes);
+            bulk_load(smem_u32(wbase + (size_t)sw * kWBytes), wsrc + ((size_t)wc * taps + wr * p.KS + wq) * (kWBytes / 2), (uint32_t)kWBytes, bar_wfull(sw));
+            ++w_loads;
+            if (++sw == p.n_w) { sw = 0; pw ^= 1u; }
+            if ((wq += p.S) >= p.KS) {
+              if ((wr += p.S) >= p.KS) {
+                if (++wpq == phases) {
+                  wpq = 0;
+                  if (++wpr == phases) {
+                    wpr = 0;
+                    if (++wc == chunk1) {
+                      wc = chunk0;
+                      if (++wb == bands) {
+                        wb = 0;
+                        wt += tile_step;
+                        w_left = wt < p.total_tiles;
+                        wsrc = p.w_tiles + (size_t)(wt - quot(wt, p.by_oc_tiles) * p.oc_tiles) * p.n_chunks * taps * (kWBytes / 2);
+                      }
+                    }
+                  }
+                }
+                wr = wpr;
+              }
+              wq = wpq;
             }
-            a[e] = xd + td;
-            if (r == p.KS - 1 && q == p.KS - 1) {
-              freed[e] = bar_xempty(sx);
-              r = 0; q = 0; td = td0; fresh_patch = true;
-              if (++sx == p.n_x) { sx = 0; xd = x0; xphase ^= 1u; } else xd += stage_step;
-            }
-            else if (++q == p.KS) { q = 0; ++r; td += row_step; }
-            else td += 8;
+          }
+          if (moved) { idle = 0; continue; }
+          if ((++idle & 31) == 0) {
+            if (*abort_flag) { ok = false; break; }
+            if (idle >= limit) { *abort_flag = 1; ok = false; break; }
+            __nanosleep(20);
           }
         }
-        if (!ok) break;
+      }
+    } else if (warp == 1) {
+      // ---- MMA issue (converged warp, one elected lane, so that descriptors stay in uniform
+      //      registers): per K step one wait, 6 (4) MMAs, one commit ----
+      // A K step of the smallest tiles takes the tensor core 200 clocks, about what this warp needs
+      // to wait, issue and commit, so the loop is kept short: no early exits (a wait that gave up
+      // raises the abort flag, later waits then return at once and the loop runs dry), 3x3 taps
+      // unrolled, ring positions counted along.
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(p.npx >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      const uint32_t sbo_x = (uint32_t)(p.mode == kGrid ? p.PW * 128 : 1024);
+      const uint64_t dx0 = smem_desc(smem_u32(xbase), sbo_x, 2), dw0 = smem_desc(smem_u32(wbase), STACK ? 512 : 1024, STACK ? 4 : 2);
+      const uint32_t dx_hi = (uint32_t)(dx0 >> 32), dw_hi = (uint32_t)(dw0 >> 32);
+      const uint32_t x_step = (uint32_t)(p.x_stage_bytes >> 4), row_step = (uint32_t)(p.PW * 8);
+      auto wait = [&](uint32_t bar, uint32_t parity) {
+        if (!mbar_try_wait(bar, parity)) mbar_wait(bar, parity, abort_flag);
+        __syncwarp();
+      };
+      int k = 0;                  // K step of the band
+      auto step = [&](uint32_t xd, bool patch_end) {
+        const bool fresh = (k & (kSuper - 1)) == 0;
+        if (fresh) wait(bar_pempty(sp & 1), ((sp >> 1) & 1) ^ 1);  // first step of a partial sum: its accumulator has been drained
+        wait(bar_wfull(sw), pw);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t ta = tmem_base + (uint32_t)(kTmemA + sa * (kStepCols * U));
+        const uint32_t tmem_d = tmem_base + (uint32_t)((sp & 1) * NMAX);
+        const uint32_t wd = (uint32_t)dw0 + (uint32_t)(sw * (kWBytes >> 4));
+        ++k;
+        const bool super_end = k == iters || (k & (kSuper - 1)) == 0;
         if (elect_one()) {
-          // operand block of a K step: columns 0-7 / 8-15 x_hi of channels 0-15 / 16-31, 16-23 / 24-31 x_lo
-          // (32 bytes along K = 2 in a descriptor's address field)
+          // K slices of 16 channels are 32 bytes = 2 in the address field; x_lo (w_lo) lies 64 bytes after x_hi (w_hi)
+          if (STACK) {
+            umma_f16_ss(tmem_d, wd, dw_hi, xd, dx_hi, idesc, fresh ? 0u : 1u);
+            umma_f16_ss(tmem_d, wd, dw_hi, xd + 4, dx_hi, idesc, 1u);
+            umma_f16_ss(tmem_d, wd + 2, dw_hi, xd + 2, dx_hi, idesc, 1u);
+            umma_f16_ss(tmem_d, wd + 2, dw_hi, xd + 6, dx_hi, idesc, 1u);
+          } else {
+            umma_f16_ss(tmem_d, wd, dw_hi, xd, dx_hi, idesc, fresh ? 0u : 1u);
+            umma_f16_ss(tmem_d, wd, dw_hi, xd + 4, dx_hi, idesc, 1u);
+            umma_f16_ss(tmem_d, wd + 4, dw_hi, xd, dx_hi, idesc, 1u);
+            umma_f16_ss(tmem_d, wd + 2, dw_hi, xd + 2, dx_hi, idesc, 1u);
+            umma_f16_ss(tmem_d, wd + 2, dw_hi, xd + 6, dx_hi, idesc, 1u);
+            umma_f16_ss(tmem_d, wd + 6, dw_hi, xd + 2, dx_hi, idesc, 1u);
+          }
+          umma_commit(bar_wempty(sw));
+          if (super_end) umma_commit(bar_pfull(sp & 1));
+          if (patch_end) umma_commit(bar_xempty(sx));
+        }
+        __syncwarp();
+        if (super_end) ++sp;
+        if (++sw == p.n_w) { sw = 0; pw ^= 1u; }
+      };
+      for (int t = tile0; t < p.total_tiles; t += tile_step) {
+        uint32_t td0 = (uint32_t)dx0;  // kFlat: the tile's first position lies some columns into its first padded row
+        if (p.mode == kFlat) {
+          int oc0, w0, h0, n0;
+          decode(t, oc0, w0, h0, n0);
+          td0 += (uint32_t)((w0 * p.npx - quot(w0 * p.npx, p.by_PW) * p.PW) * 8);
+        }
+        for (int b = 0; b < bands; ++b) {
+          k = 0;
+          for (int u = (chunk1 - chunk0) * phases * phases, ph = 0; u > 0; --u) {
+            wait(bar_xconv(sx), px);
+            const uint32_t xd = td0 + (uint32_t)sx * x_step;
+            if (p.KS == 3 && p.S == 1) {
 #pragma unroll
-          for (int e = 0; e < U; ++e) {
-            if (e < ns) {
-              const uint32_t te = ta + (uint32_t)(e * kStepCols);
-              tmem_cp(te, a[e], da_hi); tmem_cp(te + 8, a[e] + 2, da_hi); tmem_cp(te + 16, a[e] + 4, da_hi); tmem_cp(te + 24, a[e] + 6, da_hi);
-              if (freed[e]) umma_commit(freed[e]);  // the patch has been read for the last time
+              for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int q = 0; q < 3; ++q) step(xd + (uint32_t)r * row_step + 8u * q, r == 2 && q == 2);
+            } else {
+              const int pr = ph / phases, pq = ph - pr * phases;
+              if (++ph == phases * phases) ph = 0;
+              uint32_t xrow = xd;
+              for (int r = pr; r < p.KS; r += p.S, xrow += row_step) {
+                uint32_t xt = xrow;
+                for (int q = pq; q < p.KS; q += p.S, xt += 8) step(xt, r + p.S >= p.KS && q + p.S >= p.KS);
+              }
             }
+            if (++sx == p.n_x) { sx = 0; px ^= 1u; }
           }
-          umma_commit(bar_afull(sa));
         }
-        __syncwarp();
       }
-    }
-    if (!ok || *abort_flag) {  // the copies issued so far may still be running
-      if (elect_one()) umma_commit(bar_drain(0));
-      __syncwarp();
-      mbar_drain(bar_drain(0), 0);
-    }
-    PROF_OUT(2);
-  } else if (warp == 1) {
-    // ---- MMA issue (converged warp, one elected lane): six tcgen05.mma per K step, one wait and
-    //      one commit per group ----
-    const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-    const uint32_t dw_hi = (uint32_t)(smem_desc(0, 1024) >> 32);
-    const uint32_t w0 = (uint32_t)smem_desc(smem_u32(wbase), 1024);
-    int G = 0, sw = 0, sbase = 0, sp = 0;
-    uint32_t wd = w0, wphase = 0;
-    bool ok = true;
-    for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x) {
-      const Item it = item_of(t);
-      const int iters = it.iters, ngroups = it.ngroups;
-      const int sbase0 = sbase;
-      sbase += it.supers;
-      for (int j = 0, jj = 0, si = 0; j < ngroups; ++j, ++G) {
-        const int sa = G & (kAStages - 1);
-        const uint32_t acc0 = jj == 0 ? 0u : 1u;  // the first MMA of a partial overwrites it
-        const uint32_t tmem_d = tmem_base + (uint32_t)(((sbase0 + si) & 1) * BN);
-        if (jj == 0) {  // first group of a partial sum: its accumulator has been drained (two partials ago)
-          if (!(ok = TIMED(1, mbar_wait_warp(bar_pempty(sp & 1), ((sp >> 1) & 1) ^ 1, abort_flag)))) break;
-          ++sp;
-        }
-        if (++jj == kSuper) { jj = 0; ++si; }
-        if (!(ok = TIMED(2, mbar_wait_warp(bar_wfull(sw), wphase, abort_flag)))) break;  // the group's weights have landed
-        if (!(ok = TIMED(0, mbar_wait_warp(bar_afull(sa), (G / kAStages) & 1, abort_flag)))) break;  // ... and its operand blocks
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        PROF_START();
-        const int ns = min(U, iters - U * j);
-        const uint32_t ta = tmem_base + (uint32_t)(kTmemA + sa * (kStepCols * U));
-        const uint32_t dlo = wd;
-        if (++sw == p.n_w) { sw = 0; wd = w0; wphase ^= 1u; } else wd += (uint32_t)(U * kWBytes >> 4);
-        if (elect_one()) {
-          // K slices of 16 channels: 32 bytes = 2 in the address field; w_lo sits 64 bytes after w_hi
+    } else if (warp < kFirstSum) {
+      // ---- converters: a landed patch, in place, one row per thread: the 16-byte pieces of row r
+      //      sit at piece ^ (r & 7) before and after, so the eight lanes of a quarter-warp touch
+      //      eight different bank groups ----
+      const int ct = (warp - 2) * 32 + lane;
+      float seen = 0.f;
+      auto split = [](const float (&x)[4], uint32_t *hi, uint32_t *lo) {
+        const __half2 h01 = __floats2half2_rn(x[0], x[1]), h23 = __floats2half2_rn(x[2], x[3]);
+        const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
+        hi[0] = *reinterpret_cast<const uint32_t *>(&h01);
+        hi[1] = *reinterpret_cast<const uint32_t *>(&h23);
+        lo[0] = pack_half2(x[0] - f01.x, x[1] - f01.y);
+        lo[1] = pack_half2(x[2] - f23.x, x[3] - f23.y);
+      };
+      for (int t = tile0; t < p.total_tiles && ok; t += tile_step)
+        for (int b = bands - 1; b >= 0 && ok; --b) {
+          const float scale = pow2f(band_exp(b));
+          for (int u = (chunk1 - chunk0) * phases * phases; u > 0; --u) {
+            if (!(ok = mbar_wait_warp(bar_xfull(sx), px, abort_flag))) break;
+            unsigned char *stage = xbase + (size_t)sx * p.x_stage_bytes;
+            for (int row = ct; row < p.box_rows; row += 32 * kConv) {
+              float4 *rp = reinterpret_cast<float4 *>(stage + (size_t)row * 128);
+              const int swz = row & 7;
+              float4 v[8];
 #pragma unroll
-          for (int e = 0; e < U; ++e) {
-            if (e < ns) {
-              const uint32_t te = ta + (uint32_t)(e * kStepCols), de = dlo + (uint32_t)(e * (kWBytes >> 4));
-              umma_f16_ts(tmem_d, te, de, dw_hi, idesc, e == 0 ? acc0 : 1u);
-              umma_f16_ts(tmem_d, te + 16, de, dw_hi, idesc, 1u);
-              umma_f16_ts(tmem_d, te, de + 4, dw_hi, idesc, 1u);
-              umma_f16_ts(tmem_d, te + 8, de + 2, dw_hi, idesc, 1u);
-              umma_f16_ts(tmem_d, te + 24, de + 2, dw_hi, idesc, 1u);
-              umma_f16_ts(tmem_d, te + 8, de + 6, dw_hi, idesc, 1u);
+              for (int c = 0; c < 8; ++c) v[c] = rp[c ^ swz];
+              uint32_t hi[16], lo[16];
+              if (first) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                  seen = fmaxf(seen, fmaxf(fabsf(v[c].x), fabsf(v[c].y)));
+                  seen = fmaxf(seen, fmaxf(fabsf(v[c].z), fabsf(v[c].w)));
+                  const float x[4] = {kXScale * v[c].x, kXScale * v[c].y, kXScale * v[c].z, kXScale * v[c].w};
+                  split(x, hi + 2 * c, lo + 2 * c);
+                }
+              } else {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                  float x[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) {
+                    const int ex = (int)((__float_as_uint(x[e]) >> 23) & 0xFFu) - 127;  // 128: infinity or NaN, kept in band 0
+                    if (ex < 128) seen = fmaxf(seen, fabsf(x[e]));
+                    const int mine = banded ? min(kBands - 1, max(0, emax - ex) / kBandBits) : 0;
+                    x[e] = mine == b ? x[e] * scale : 0.f;
+                  }
+                  split(x, hi + 2 * c, lo + 2 * c);
+                }
+              }
+              uint4 *wp = reinterpret_cast<uint4 *>(rp);
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                wp[c ^ swz] = make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]);
+                wp[(c + 4) ^ swz] = make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]);
+              }
             }
-          }
-          PROF_LAP(3);
-          umma_commit(bar_gdone(G & (kGroups - 1)));
-          PROF_LAP(4);
-        }
-        __syncwarp();
-      }
-    }
-    if (!ok || *abort_flag) {  // the MMAs issued so far may still be running
-      if (elect_one()) umma_commit(bar_drain(1));
-      __syncwarp();
-      mbar_drain(bar_drain(1), 0);
-    }
-    PROF_OUT(3);
-  } else if (warp >= 4 && warp < 8) {
-    // ---- warps 4..7: a landed patch, in place: each 128-byte row of 32 FP32 channels becomes
-    //      {x_hi[32], x_lo[32]} FP16.  One row per thread: the 16-byte chunks of row r sit at
-    //      chunk ^ (r & 7) before and after, so the eight lanes of a quarter-warp touch eight
-    //      different bank groups. ----
-    const int ct = (warp - 4) * 32 + lane;
-    int u = 0;
-    bool ok = true;
-    uint32_t seen_max = 0;
-    for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x) {
-      const int item_chunks = item_of(t).chunks;
-      for (int chunk = 0; chunk < item_chunks; ++chunk, ++u) {
-        const int sx = u % p.n_x;
-        if (!(ok = TIMED(0, mbar_wait_warp(bar_xfull(sx), (u / p.n_x) & 1, abort_flag)))) break;
-        unsigned char *stage = xbase + (size_t)sx * p.x_stage_bytes;
-        for (int row = ct; row < p.box_rows; row += 128) {
-          uint4 *rp = reinterpret_cast<uint4 *>(stage + (size_t)row * 128);
-          const int sw = row & 7;
-          uint4 v[8];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) v[c] = rp[c ^ sw];
-          uint32_t hi[16], lo[16];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const float x0 = kXScale * __uint_as_float(v[c].x), x1 = kXScale * __uint_as_float(v[c].y),
-                        x2 = kXScale * __uint_as_float(v[c].z), x3 = kXScale * __uint_as_float(v[c].w);
-            seen_max = max(seen_max, max(max(v[c].x & 0x7FFFFFFFu, v[c].y & 0x7FFFFFFFu), max(v[c].z & 0x7FFFFFFFu, v[c].w & 0x7FFFFFFFu)));
-            const __half2 h01 = __floats2half2_rn(x0, x1), h23 = __floats2half2_rn(x2, x3);
-            const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
-            hi[2 * c] = *reinterpret_cast<const uint32_t *>(&h01);
-            hi[2 * c + 1] = *reinterpret_cast<const uint32_t *>(&h23);
-            lo[2 * c] = pack_half2(x0 - f01.x, x1 - f01.y);
-            lo[2 * c + 1] = pack_half2(x2 - f23.x, x3 - f23.y);
-          }
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            rp[c ^ sw] = make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]);
-            rp[(c + 4) ^ sw] = make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]);
+            // the writes above go through the generic proxy, the MMAs read through the async proxy
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_xconv(sx));
+            if (++sx == p.n_x) { sx = 0; px ^= 1u; }
           }
         }
-        // the writes above go through the generic proxy, tcgen05.cp reads through the async proxy
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      unsigned m = __float_as_uint(seen);
+      for (int s = 16; s; s >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, s));
+      if (lane == 0) atomicMax(seen_slot, m);
+    } else {
+      // ---- summing warps: partials -> running sums -> output.  A warp may touch the TMEM lanes of
+      //      its quarter; two warps share a quarter and take half of the pixels each.  (After a
+      //      wait that gave up this role, too, runs dry: its warps meet at barriers.) ----
+      const int me = warp - kFirstSum, quarter = me & 3, half = me >> 2;
+      const int hc = ((p.npx >> 4) + 1) / 2 * 16;                 // pixels of the first half
+      const int j0 = half * hc, ncols = half ? p.npx - hc : hc;   // this warp's pixels
+      const int ocl = STACK ? (quarter & 1) * 32 + lane : quarter * 32 + lane;  // channel inside the tile
+      int4 *gtab = gtabs + me * (NC / 8);
+      float *blocks = reinterpret_cast<float *>(exch) + me * 1024;             // two blocks of 16 pixels x 32 channels
+      float *give = reinterpret_cast<float *>(exch) + kSumWarps * 1024 + me * 1024;  // stacked tiles
+      const float *take = reinterpret_cast<const float *>(exch) + kSumWarps * 1024 + (me ^ 2) * 1024;
+      int nblk = 0;
+      const bool vec = (p.OC & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;  // 16-byte stores
+      const float unscale = banded ? pow2f(4 - band_exp(0)) : 1.f;
+      for (int t = tile0; t < p.total_tiles; t += tile_step) {
+        int oc0, w0, h0, n0;
+        decode(t, oc0, w0, h0, n0);
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_xconv(sx));
-      }
-    }
-    // the launch's largest magnitude: the guard kernel behind this one decides on it
-    for (int d = 16; d; d >>= 1) seen_max = max(seen_max, __shfl_xor_sync(0xffffffffu, seen_max, d));
-    if (lane == 0 && seen_max) atomicMax(p.gate, seen_max);
-    if (warp == 4) PROF_OUT(4);
-  } else if (warp >= 8) {
-    // ---- warps 8..15: running sum in registers, store at the end of the work item ----
-    constexpr int NC = BN / 2;             // channels per thread
-    const int quarter = warp & 3, half = (warp - 8) >> 2;
-    const int row = quarter * 32 + lane;   // tile row = pixel = TMEM lane
-    const bool vec = (p.OC & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
-    const bool small_out = (unsigned long long)p.N * p.OH * p.OW * p.OC < (1ull << 34);  // 32-bit offsets in 16-byte units
-    // output pixel of tile row r of the tile at (w0, h0, n0), in the launch's tile geometry
-    auto row_pixel = [&](int r, int w0, int h0, int n0, bool &okr, size_t &pix) {
-      if (p.linear) {
-        const long long px = (long long)(w0 / kTW) * BM + r;
-        okr = px < p.total_pixels;
-        pix = (size_t)px;
-      } else if (p.flat) {
-        const int pos = (w0 / kTW) * BM + r, oh = pos / p.PW, ow = pos - oh * p.PW;
-        okr = ow < p.OW && oh < p.OH && n0 < p.N;
-        pix = ((size_t)n0 * p.OH + oh) * p.OW + ow;
-      } else {
-        const int g = r >> 3, in = g / p.PHI, ih = g - in * p.PHI;
-        const int ow = w0 + (r & 7), oh = h0 + ih, n = n0 + in;
-        okr = in < p.NB && ih < p.TH && ow < p.OW && oh < p.OH && n < p.N;
-        pix = ((size_t)n * p.OH + oh) * p.OW + ow;
-      }
-    };
-    int gbase = 0, sp = 0;  // first group of the item; partial sum, counted across items
-    bool ok = true;
-    for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x) {
-      int ngroups, tile_supers;
-      { const Item head = item_of(t); ngroups = head.ngroups; tile_supers = head.supers; }
-      const int gbase0 = gbase;
-      gbase += ngroups;
-      float acc[NC];
+        if (p.d == 1 && lane < NC / 8) {
+          // where this warp's pixel group `lane` goes: {x, row, image} of a box of 8 pixels in the
+          // output tensor (what lies past the tensor is dropped), or pixel by pixel
+          int4 e = make_int4(0, 0, n0, 0);  // w: 0 nowhere, 1 a box, 2 pixel by pixel
+          const int j = j0 + 8 * lane;
+          if (8 * lane < ncols) {
+            if (p.mode == kLinear) {
+              e.x = w0 * p.npx + j;
+              e.w = e.x < p.total_pixels ? 1 : 0;
+            } else if (p.mode == kFlat) {
+              const int pos = w0 * p.npx + j;
+              e.y = quot(pos, p.by_PW); e.x = pos - e.y * p.PW;
+              e.w = e.y >= p.OH ? 0 : e.x + 8 > p.PW ? 2 : e.x < p.OW ? 1 : 0;
+            } else {
+              const int g = j >> 3, i = p.NB > 1 ? quot(g, p.by_PHI) : 0;
+              e.x = w0 * kTW; e.y = g - i * p.PHI; e.z = n0 + i;
+              e.w = i < p.NB && e.y < p.TH && h0 + e.y < p.OH && e.z < p.N ? 1 : 0;
+              e.y += h0;
+            }
+            if (e.w == 1 && !p.tma_store) e.w = 2;
+          }
+          gtab[lane] = e;
+        }
+        __syncwarp();
+        // Sum the partials in registers; the total goes back into the last partial's columns of
+        // tensor memory, from where a short loop takes it on (16 pixels at a time, the same code
+        // every time: 128 registers can only be walked by unrolled code, which ran at the rate of
+        // the instruction fetches -- 9000 clocks per tile).  An item of one partial is taken as it is.
+        const int partials = supers * bands;
+        auto partial = [&]() {  // this warp's first column of the next partial, once the tensor core is done with it
+          if (!mbar_try_wait(bar_pfull(sp & 1), (sp >> 1) & 1)) mbar_wait(bar_pfull(sp & 1), (sp >> 1) & 1, abort_flag);
+          __syncwarp();
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          return tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((sp & 1) * NMAX + j0);
+        };
+        uint32_t ttotal;
+        if (partials > 1) {
+          float acc[NC];
 #pragma unroll
-      for (int j = 0; j < NC; ++j) acc[j] = 0.f;
-      for (int si = 0; si < tile_supers; ++si, ++sp) {
-        const int b = sp & 1;
-        if (!(ok = TIMED(0, wait_group_warp(gbase0 + min((si + 1) * kSuper, ngroups) - 1)))) break;  // the partial's last group
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN + half * NC);
+          for (int j = 0; j < NC; ++j) acc[j] = 0.f;
+          int left = supers, band = bands - 1;
+#pragma unroll 1
+          for (int i = 1; i < partials; ++i, ++sp) {
+            const uint32_t taddr = partial();
 #pragma unroll
-        for (int c0 = 0; c0 < NC; c0 += 16) {
-          uint32_t v[16];
-          tmem_ld16(taddr + c0, v);
-          if (c0 + 16 == NC) {  // everything is in registers: the tensor core may overwrite the partial
+            for (int c0 = 0; c0 < NC; c0 += 16) {
+              if (c0 < ncols) {
+                uint32_t v[16];
+                tmem_ld16(taddr + c0, v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[c0 + j] += __uint_as_float(v[j]);
+              }
+            }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_pempty(b));
-          }
+            if (lane == 0) mbar_arrive(bar_pempty(sp & 1));  // the tensor core may overwrite the partial
+            if (--left == 0) {  // from this band's scale to the next larger one's
+              const float f = pow2f(band_exp(band - 1) - band_exp(band));
+              left = supers; --band;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) acc[c0 + j] += __uint_as_float(v[j]);
-        }
-      }
-      if (!ok) break;
-      // (the item is worked out again here rather than kept in registers across the sums above:
-      // with 64 running sums per thread this role is the one that sets the kernel's register count)
-      int t_again = t;
-      asm volatile("" : "+r"(t_again));
-      const Item it = item_of(t_again);
-      int w0, h0, n0, oc0;
-      decode(it.tile, w0, h0, n0, oc0);
-      PROF_START();
-      if (it.tail) {
-        // A slice of a last-wave tile: leave the partial sums in the scratch block of (tile,
-        // slice); the CTA that finishes a tile last adds the slices up in slice order (so the
-        // result does not depend on who that is) and carries on to the store.
-        float4 *mine = reinterpret_cast<float4 *>(p.scratch + ((size_t)((it.tile - p.tail_tile0) * p.tail_d + it.slice) * BM + row) * BN + half * NC);
-#pragma unroll
-        for (int j = 0; j < NC; j += 4) mine[j >> 2] = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-        __threadfence();
-        PROF_LAP(2);
-        asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight summing warps
-        int *verdict = reinterpret_cast<int *>(store_base);  // (the staging block is free between items)
-        if (warp == 8 && lane == 0) {
-          const int seen = atomicAdd(p.tail_count + (it.tile - p.tail_tile0), 1);
-          *verdict = seen == p.tail_d - 1 ? 1 : 0;
-          if (seen == p.tail_d - 1) p.tail_count[it.tile - p.tail_tile0] = 0;  // ready for the next launch
-        }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        const bool reducer = *verdict != 0;
-        asm volatile("bar.sync 1, 256;" ::: "memory");  // (the staging block is written again below)
-        PROF_LAP(3);
-        if (!reducer) continue;
-        __threadfence();
-        // The slices are added position by position (a warp walks one row of the tile: coalesced
-        // reads of the eight scratch blocks, coalesced stores) rather than into the per-thread
-        // running sums: with those 64 registers held, the loads of the slices would go out one
-        // at a time (measured: 36 us for one tile).
-        constexpr int V = BN / 4;  // 16-byte pieces per tile row
-        const float4 *blocks = reinterpret_cast<const float4 *>(p.scratch + (size_t)(it.tile - p.tail_tile0) * p.tail_d * BM * BN);
-        const bool vec_out = (p.OC & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
-        for (int idx = (warp - 8) * 32 + lane; idx < BM * V; idx += 256) {
-          float4 v[8];
-#pragma unroll
-          for (int sl = 0; sl < 8; ++sl)
-            v[sl] = sl < p.tail_d ? __ldcg(blocks + (size_t)sl * BM * V + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
-          float4 sum = v[0];
-#pragma unroll
-          for (int sl = 1; sl < 8; ++sl) { sum.x += v[sl].x; sum.y += v[sl].y; sum.z += v[sl].z; sum.w += v[sl].w; }
-          const int r2 = idx / V, oc = oc0 + 4 * (idx - r2 * V);
-          bool ok2;
-          size_t pix2;
-          row_pixel(r2, w0, h0, n0, ok2, pix2);
-          if (!ok2 || oc >= p.OC || *abort_flag) continue;
-          float res[4] = {sum.x, sum.y, sum.z, sum.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            res[e] *= (oc + e < p.OC) ? __ldg(p.out_scale + oc + e) : 0.f;
-            if (p.relu) res[e] = fmaxf(res[e], 0.f);
-          }
-          float *dst = p.out + pix2 * p.OC + oc;
-          if (vec_out) *reinterpret_cast<float4 *>(dst) = make_float4(res[0], res[1], res[2], res[3]);
-          else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (oc + e < p.OC) dst[e] = res[e];
-          }
-        }
-        PROF_LAP(4);
-        continue;
-      }
-      const bool add_up = !it.tail && p.ksplit > 1;  // a slice of a uniformly split K range: add into the zeroed output
-      bool row_ok;
-      size_t pix;
-      row_pixel(row, w0, h0, n0, row_ok, pix);
-      row_ok = row_ok && !*abort_flag;
-      const int ocb = oc0 + half * NC;
-      float *o = p.out + pix * p.OC + ocb;
-      const bool coalesced = vec && ocb + NC <= p.OC && small_out;
-      if (!coalesced) {  // (the coalesced path scales after the rows are turned: two loads per thread instead of NC)
-#pragma unroll
-        for (int j = 0; j < NC; ++j) acc[j] *= (ocb + j < p.OC) ? __ldg(p.out_scale + ocb + j) : 0.f;
-        if (p.relu) {
-#pragma unroll
-          for (int j = 0; j < NC; ++j) acc[j] = fmaxf(acc[j], 0.f);
-        }
-      }
-      if (coalesced) {
-        // Coalesced path: a thread holds 32..64 channels of ONE pixel; through a 4 KiB staging
-        // block per warp the rows are turned so that eight lanes write one pixel's 128
-        // contiguous bytes (4 passes through the memory pipe per store instead of 32).
-        float4 *stage = reinterpret_cast<float4 *>(store_base + (warp - 8) * 4096);
-        const uint32_t off16 = row_ok ? (uint32_t)((o - p.out) >> 2) : 0xFFFFFFFFu;
-#pragma unroll
-        for (int h = 0; h < NC / 32; ++h) {
-#pragma unroll
-          for (int qq = 0; qq < 8; ++qq)  // 16-byte piece qq of row `lane` sits at piece qq ^ (lane & 7)
-            stage[lane * 8 + (qq ^ (lane & 7))] = make_float4(acc[h * 32 + 4 * qq], acc[h * 32 + 4 * qq + 1],
-                                                               acc[h * 32 + 4 * qq + 2], acc[h * 32 + 4 * qq + 3]);
-          __syncwarp();
-          float4 v[8];
-          const int qq = lane & 7;
-          // this lane's four channels of every row: the per-channel scale (a power of two, exact)
-          const float4 sc = __ldg(reinterpret_cast<const float4 *>(p.out_scale + ocb + h * 32 + 4 * qq));
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int r = 4 * i + (lane >> 3);
-            v[i] = stage[r * 8 + (qq ^ (r & 7))];
-            v[i].x *= sc.x; v[i].y *= sc.y; v[i].z *= sc.z; v[i].w *= sc.w;
-            if (p.relu) { v[i].x = fmaxf(v[i].x, 0.f); v[i].y = fmaxf(v[i].y, 0.f); v[i].z = fmaxf(v[i].z, 0.f); v[i].w = fmaxf(v[i].w, 0.f); }
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const uint32_t off = __shfl_sync(0xffffffffu, off16, 4 * i + (lane >> 3));
-            float *dst = p.out + ((size_t)off << 2) + h * 32 + 4 * qq;
-            if (off != 0xFFFFFFFFu) {
-              if (add_up)
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v[i].x), "f"(v[i].y), "f"(v[i].z), "f"(v[i].w) : "memory");
-              else
-                *reinterpret_cast<float4 *>(dst) = v[i];
+              for (int j = 0; j < NC; ++j) acc[j] *= f;
             }
           }
-          __syncwarp();
+          ttotal = partial();
+#pragma unroll
+          for (int c0 = 0; c0 < NC; c0 += 16) {
+            if (c0 < ncols) {
+              uint32_t v[16];
+              tmem_ld16(ttotal + c0, v);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(acc[c0 + j] + __uint_as_float(v[j]));
+              tmem_st16(ttotal + c0, v);
+            }
+          }
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        } else {
+          ttotal = partial();
         }
-        continue;
+        ++sp;
+        const int oc = oc0 + ocl;
+        if (p.d > 1) {
+          // a slice of a tile: its sums into this CTA's shared memory (the rings are idle: every MMA
+          // of the only item has completed), one row of 128 accumulator lanes per pixel
+          float *rows = reinterpret_cast<float *>(xbase) + quarter * 32 + lane;
+#pragma unroll 1
+          for (int c0 = 0; c0 < ncols; c0 += 16) {
+            uint32_t v[16];
+            tmem_ld16(ttotal + c0, v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) rows[(j0 + c0 + j) * BM] = __uint_as_float(v[j]) * unscale;
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (a further pass loads over it)
+        } else {
+          // Store: a thread holds one channel of many pixels, an 8-pixel group of a warp is a box of
+          // 32 channels x 8 pixels of the output.  16 pixels at a time go into a staging block (one
+          // conflict-free 4-byte store per value), which TMA stores carry on from there while the
+          // warp stages the next block.
+          const float sc = oc < p.OC ? p.out_scale[oc] * unscale : 0.f;
+          const int ocw = oc - lane;  // first channel of the warp
+          auto put16 = [&](int c0, const float (&v)[16]) {  // pixels c0 .. c0 + 15 of this warp
+            float *blk = blocks + (nblk & 1) * 512;
+            ++nblk;
+            if (lane < 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the stores of the block before last have read it
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) blk[j * 32 + lane] = p.relu ? fmaxf(v[j] * sc, 0.f) : v[j] * sc;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            const int4 mine = gtab[(c0 >> 3) + (lane & 1)];  // (even lanes: first group, odd lanes: second)
+            __syncwarp();
+            if (lane < 2) {
+              if (mine.w == 1 && ocw < p.OC)
+                asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+                             ::"l"(&map_out), "r"(smem_u32(blk + lane * 256)), "r"(ocw), "r"(mine.x), "r"(mine.y), "r"(mine.z) : "memory");
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+            if (__any_sync(0xffffffffu, mine.w == 2)) {
+              const int wa = __shfl_sync(0xffffffffu, mine.w, 0), wb = __shfl_sync(0xffffffffu, mine.w, 1);
+#pragma unroll 1
+              for (int j = wa == 2 ? 0 : 8; j < (wb == 2 ? 16 : 8); ++j) {
+                const int pix = pixel_of(j0 + c0 + j, w0, h0, n0);
+                if (pix >= 0 && oc < p.OC) p.out[(size_t)pix * p.OC + oc] = blk[j * 32 + lane];
+              }
+            }
+          };
+          if (STACK) {
+            // Lanes 64..127 hold the w_lo halves of the channels of lanes 0..63.  The two warps of a
+            // channel group and half give each other 16 pixels at a time through shared memory -- the
+            // w_lo warp from the first half of the pixels, the other one from the second -- and store
+            // the rest.  Two blocks in turn: one barrier per round.
+            const int split = ((ncols >> 4) + 1) / 2 * 16;
+            const int out0 = quarter >= 2 ? 0 : split, nout = quarter >= 2 ? split : ncols - split;  // pixels given away
+            const int in0 = quarter >= 2 ? split : 0, nin = ncols - nout;                            // pixels kept
+#pragma unroll 1
+            for (int c = 0; c < split; c += 16) {
+              uint32_t v[16];
+              const int slot = (trades++ & 1) * 512 + lane;
+              if (c < nout) {
+                tmem_ld16(ttotal + out0 + c, v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) give[slot + j * 32] = __uint_as_float(v[j]);
+              }
+              asm volatile("bar.sync %0, 64;" ::"r"(1 + half * 2 + (quarter & 1)) : "memory");
+              if (c < nin) {
+                tmem_ld16(ttotal + in0 + c, v);
+                float y[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) y[e] = __uint_as_float(v[e]) + take[slot + e * 32];
+                put16(in0 + c, y);
+              }
+            }
+          } else {
+#pragma unroll 1
+            for (int c0 = 0; c0 < ncols; c0 += 16) {
+              uint32_t v[16];
+              tmem_ld16(ttotal + c0, v);
+              float y[16];
+#pragma unroll
+              for (int j = 0; j < 16; ++j) y[j] = __uint_as_float(v[j]);
+              put16(c0, y);
+            }
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_pempty((sp - 1) & 1));
       }
-      if (!row_ok) continue;
-      if (add_up) {
+      if (lane < 2) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // this warp's stores are complete
+    }
+    // ---- end of a pass: does this CTA's largest activation ask for another one? ----
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned m = *reinterpret_cast<volatile unsigned *>(seen_slot);
+    const bool stop = *abort_flag != 0 || banded || (m < 0x45000000u && (m == 0u || m >= 0x3B800000u));
+    if (stop) break;
+    banded = m < 0x7F800000u;
+    emax = (int)(m >> 23) - 127;
+    first = false;
+    __syncthreads();
+    if (tid == 0 && !banded) *seen_slot = 0u;
+    __syncthreads();
+  }
+
+  if (*abort_flag) {  // what this CTA has in flight must land before it leaves
+    if (tid == 0) {
+      for (int v = max(x_loads - p.n_x, p.withhold_first_load ? 1 : 0); v < x_loads; ++v) mbar_drain(bar_xfull(v % p.n_x), (uint32_t)(v / p.n_x) & 1u);
+      for (int v = max(w_loads - p.n_w, 0); v < w_loads; ++v) mbar_drain(bar_wfull(v % p.n_w), (uint32_t)(v / p.n_w) & 1u);
+    }
+    if (warp == 1) {
+      if (elect_one()) umma_commit(bar_drain());
+      __syncwarp();
+      mbar_drain(bar_drain(), 0);
+    }
+    if (tid == 0) atomicExch(p.error_flag, 1);
+  }
+  if (p.d > 1) {
+    // The slices of a tile meet: CTA `rank` adds up its share of the pixels over the cluster, in
+    // slice order, and stores them (a warp takes one pixel's 32 channels at a time).
+    cluster_sync_all();
+    const int per = (p.npx + p.d - 1) / p.d, ja = rank * per, jb = min(p.npx, ja + per);
+    int oc0, w0, h0, n0;
+    decode(tile0, oc0, w0, h0, n0);
+    // A lane adds up four channels of a pixel, 16 bytes per slice; four pixels in flight.
+    constexpr int kPix = STACK ? 2 : 1;                // pixels of a warp's row of loads
+    const int sub = STACK ? lane >> 4 : 0, oc = oc0 + 4 * (STACK ? lane & 15 : lane);
+    const uint32_t rows = smem_u32(xbase) + (uint32_t)(STACK ? lane & 15 : lane) * 16u;
+    const bool vec = (p.OC & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+    for (int j = ja + warp * 4 * kPix + sub; j < jb; j += kThreads / 32 * 4 * kPix) {
+      float4 y[4];
 #pragma unroll
-        for (int j = 0; j < NC; ++j)
-          if (ocb + j < p.OC) atomicAdd(o + j, acc[j]);
-      } else if (vec && ocb + NC <= p.OC) {
+      for (int e = 0; e < 4; ++e) y[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+      for (int s = 0; s < p.d; ++s) {
+        float4 u[4], l[4];
 #pragma unroll
-        for (int j = 0; j < NC; j += 4) *reinterpret_cast<float4 *>(o + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-      } else {
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t a = rows + (uint32_t)(min(j + e * kPix, jb - 1) * BM) * 4u;
+          u[e] = ld_cluster4(a, (uint32_t)s);
+          if (STACK) l[e] = ld_cluster4(a + 256u, (uint32_t)s);
+        }
 #pragma unroll
-        for (int j = 0; j < NC; ++j)
-          if (ocb + j < p.OC) o[j] = acc[j];
+        for (int e = 0; e < 4; ++e) {
+          if (STACK) { u[e].x += l[e].x; u[e].y += l[e].y; u[e].z += l[e].z; u[e].w += l[e].w; }
+          y[e].x += u[e].x; y[e].y += u[e].y; y[e].z += u[e].z; y[e].w += u[e].w;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int pix = j + e * kPix < jb && !*abort_flag ? pixel_of(j + e * kPix, w0, h0, n0) : -1;
+        if (pix < 0 || oc >= p.OC) continue;
+        float v[4] = {y[e].x, y[e].y, y[e].z, y[e].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[i] *= oc + i < p.OC ? __ldg(p.out_scale + oc + i) : 0.f;
+          if (p.relu) v[i] = fmaxf(v[i], 0.f);
+        }
+        float *o = p.out + (size_t)pix * p.OC + oc;
+        if (vec) *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+        else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (oc + i < p.OC) o[i] = v[i];
+        }
       }
     }
+    cluster_sync_all();  // (nobody leaves while its shared memory is being read)
   }
-  if (warp == 8) PROF_OUT(5);
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (tid == 0 && *abort_flag) atomicExch(p.error_flag, 1);
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
 }
 
@@ -761,25 +852,27 @@ __global__ void tc16_scales_kernel(const float *__restrict__ w, int per_oc, floa
   }
 }
 
-// Dense OIHW -> the images the weight loader copies: for every (32-channel chunk, tap, channel
-// tile) BN rows of 128 bytes, row = output channel = {w_hi[32], w_lo[32]} FP16 of w * scale[oc], in
-// the 128-byte-swizzled order the tensor core reads (16-byte piece j of row r sits at piece
-// j ^ (r & 7)).  Channels past IC or OC are zero.
+// Dense OIHW -> the images the weight loader copies, one per (channel tile, 32-channel chunk, tap),
+// in the swizzled order the tensor core reads.  Plain: 128 rows of 128 bytes, row = output channel
+// = {w_hi[32], w_lo[32]} FP16 of w * scale[oc], 16-byte piece j of row r at piece j ^ (r & 7).
+// Stacked (at most 64 channels): 128 rows of 64 bytes, rows 0..63 w_hi and 64..127 w_lo of channel
+// r & 63, piece j at piece j ^ ((r >> 1) & 3).  Channels past IC or OC are zero.
 __global__ void tc16_weight_tiles_kernel(const float *__restrict__ filt, __half *__restrict__ tiles,
-                                         int OC, int IC, int KS, int n_chunks, int oc_tiles, int BN, const float *__restrict__ scale) {
-  const long long total = (long long)KS * KS * n_chunks * oc_tiles * BN * 64;
+                                         int OC, int IC, int KS, int n_chunks, int oc_tiles, int stack, const float *__restrict__ scale) {
+  const int cols = stack ? 32 : 64;
+  const long long total = (long long)KS * KS * n_chunks * oc_tiles * BM * cols;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int col = (int)(i % 64);                 // FP16 position inside the stored row
-    const int row = (int)((i / 64) % BN);
-    long long tile = i / ((long long)64 * BN);     // images are stored [channel tile][chunk][tap]: the K steps of
-    const int tap = (int)(tile % (KS * KS));       // a work item lie back to back
+    const int col = (int)(i % cols);               // FP16 position inside the stored row
+    const int row = (int)((i / cols) % BM);
+    long long tile = i / ((long long)cols * BM);
+    const int tap = (int)(tile % (KS * KS));
     tile /= KS * KS;
     const int chunk = (int)(tile % n_chunks);
     const int oct = (int)(tile / n_chunks);
-    const int piece = (col >> 3) ^ (row & 7);      // logical 16-byte piece stored at this position
+    const int piece = (col >> 3) ^ (stack ? (row >> 1) & 3 : row & 7);  // logical 16-byte piece stored at this position
     const int k = ((piece & 3) << 3) | (col & 7);  // channel inside the chunk
-    const bool is_lo = piece >= 4;
-    const int oc = oct * BN + row, ic = chunk * KC + k;
+    const bool is_lo = stack ? row >= 64 : piece >= 4;
+    const int oc = stack ? row & 63 : oct * BM + row, ic = chunk * KC + k;
     float w = 0.f;
     if (ic < IC && oc < OC) w = filt[((size_t)oc * IC + ic) * KS * KS + tap] * scale[oc];
     const __half h = __float2half_rn(w);
@@ -802,39 +895,186 @@ EncodeFn get_encode() {
   return fn;
 }
 
+// How one conv shape runs: tile geometry, K slices, rings.
+struct Geometry {
+  int mode = -1, npx = 0, PW = 0, PHI = 0, TH = 1, NB = 1;
+  int tiles_w = 1, tiles_h = 1, tiles_n = 1;
+  int box_w = 1, box_h = 1, box_n = 1, reach = 0;  // patch load; furthest row a window touches
+  int d = 1, nmax = 128, n_x = 2, n_w = 3, x_stage = 0;
+  size_t smem = 0;
+  double cost = 0.;  // estimated clocks
+};
+
 struct Tc16State {
   __half *d_tiles = nullptr;
   int *d_error = nullptr;
-  unsigned *d_gate = nullptr;
-  int n_chunks = 0, bn = 128;
   float *d_out_scale = nullptr;  // per output channel
-  float *d_scratch = nullptr;    // tail split: one 128 x BN block of partial sums per CTA (allocated when a shape first needs it)
-  int *d_tail_count = nullptr;   // tail split: finished slices per last-wave tile (all zero between launches)
-  int sms = 0;
+  int n_chunks = 0, oc_tiles = 1, sms = 0;
+  bool stack = false;            // at most 64 output channels: {w_hi, w_lo} stacked on the M side
+  // Launch set-ups (tensor map, tile plan, grid), one per (input pointer, conv shape) seen lately.
   struct Setup {
     bool valid = false;
     const float *in = nullptr;
+    const float *out = nullptr;
     ConvShape shape{};
-    CUtensorMap map_x;
+    CUtensorMap map_x, map_out;
     Tc16Params params{};
-    dim3 grid;
+    unsigned grid = 0;
+    int nmax = 128;
     size_t smem = 0;
   };
   static constexpr int kSetups = 8;
   std::mutex mutex;
   Setup setups[kSetups];
   int next_setup = 0;
+  Geometry last_geo;             // geometry of the last shape planned (independent of the pointers)
+  ConvShape last_shape{};
 };
 
 constexpr size_t kSmemBudget = 227 * 1024;
+
+bool same_conv(const ConvShape &a, const ConvShape &b) {
+  return a.N == b.N && a.H == b.H && a.W == b.W && a.S == b.S && a.P == b.P;
+}
+
+// Rings and estimated time of a geometry whose tile is settled; false if it does not fit.
+bool finish_geometry(const Tc16State &t, const ConvShape &s, Geometry *g) {
+  const int taps = s.KS * s.KS, phases = std::min(s.S, s.KS);
+  const size_t wb = t.stack ? 8192 : 16384;
+  const int box_rows = g->box_w * g->box_h * g->box_n;
+  if (g->box_w * s.S > 256 || g->box_h * s.S > 256 || g->box_n > 256) return false;
+  g->nmax = g->npx > 128 ? 256 : 128;
+  g->x_stage = (std::max(g->reach, box_rows) * 128 + 1023) / 1024 * 1024;
+  const size_t fixed = 1024 + stage_bytes(t.stack) + kNumBars * 8 + kSumWarps * (g->nmax / 16) * 16 + 64;
+  auto fits = [&](int nx, int nw) { return fixed + (size_t)nx * g->x_stage + nw * wb <= kSmemBudget; };
+  if (!fits(2, 3)) return false;
+  // a patch feeds taps / phases^2 K steps: filters larger than 1x1 need few patches and many weight
+  // images in flight, 1x1 filters one of each per K step
+  const int steps = std::max(1, taps / (phases * phases));
+  const int x_want = steps >= 4 ? 3 : kXStagesMax;
+  g->n_x = 2; g->n_w = 3;
+  for (bool grew = true; grew;) {
+    grew = false;
+    if (g->n_x < std::min(x_want, 3) && fits(g->n_x + 1, g->n_w)) { ++g->n_x; grew = true; }
+    if (g->n_w < kWStagesMax && fits(g->n_x, g->n_w + 1)) { ++g->n_w; grew = true; }
+    if (g->n_x < x_want && fits(g->n_x + 1, g->n_w)) { ++g->n_x; grew = true; }
+  }
+  g->smem = fixed + (size_t)g->n_x * g->x_stage + g->n_w * wb;
+  if (g->d > 1 && (size_t)g->npx * BM * 4 > (size_t)g->n_x * g->x_stage + g->n_w * wb) return false;  // (the sums of a slice)
+  // clocks per K step: the MMAs themselves, the shared-memory pipe (MMA operands, weight copy,
+  // patch landing, read and written by the conversion), the conversion, the issuing warp
+  const int nm = t.stack ? 4 : 6, conv = g->nmax == 256 ? 2 : 6;
+  const double operand = 4096. + 32. * g->npx;
+  const double mma = nm * std::max(0.52 * g->npx, operand / 128.);
+  const double pipe = (nm * operand + wb + 384. * box_rows / steps) / 128.;
+  const double cvt = std::ceil(box_rows / (32. * conv)) * 420. / steps;
+  const double step = std::max(std::max(mma, pipe), std::max(cvt, 330.));
+  const double k_steps = (double)taps * ((t.n_chunks + g->d - 1) / g->d);
+  const double tiles = (double)g->tiles_w * g->tiles_h * g->tiles_n * t.oc_tiles;
+  // (clusters of d CTAs live inside a GPC: on the 148-SM part 148 CTAs in pairs, 132 in fours, 120 in eights)
+  const double slots = g->d <= 2 ? t.sms : g->d * std::floor(t.sms * (g->d == 4 ? 0.225 : 0.1015));
+  const double waves = std::ceil(tiles * g->d / slots);
+  const double item = std::max(k_steps * step, 12. * g->npx) + 400.;
+  g->cost = waves * item + 5000. + 10. * g->npx + 0.3 * box_rows * 10. + (g->d > 1 ? 2500. + 8. * g->npx + (waves - 1.) * 5000. : 0.);
+  return true;
+}
+
+// The cheapest geometry by that estimate.
+bool plan_geometry(const Tc16State &t, const ConvShape &s, Geometry *best) {
+  const int amax = (s.KS - 1) / s.S;
+  bool found = false;
+  auto consider = [&](Geometry g) {
+    for (int d = 1; d <= 8 && d <= t.n_chunks; d *= 2) {
+      g.d = d;
+      Geometry c = g;
+      if (finish_geometry(t, s, &c) && (!found || c.cost < best->cost)) { *best = c; found = true; }
+    }
+  };
+  const long long pixels = (long long)s.N * s.OH * s.OW;
+  for (int npx = 16; npx <= 256; npx += 16) {
+    Geometry g;
+    g.npx = npx;
+    if (s.KS == 1 && s.S == 1 && s.P == 0) {
+      g.mode = kLinear;
+      g.PW = kTW; g.PHI = 1;
+      g.tiles_w = (int)((pixels + npx - 1) / npx);
+      g.box_w = npx; g.reach = npx;
+      consider(g);
+      continue;
+    }
+    // whole padded rows
+    g.mode = kFlat;
+    g.PW = s.OW + amax;
+    g.TH = s.OH;
+    g.PHI = (g.PW - 1 + npx - 1) / g.PW + 1 + amax;
+    g.tiles_w = ((s.OH - 1) * g.PW + s.OW + npx - 1) / npx;
+    g.tiles_n = s.N;
+    g.box_w = g.PW; g.box_h = g.PHI;
+    g.reach = g.PW - 1 + npx + amax * g.PW + amax;
+    consider(g);
+  }
+  if (s.KS == 1 && s.S == 1 && s.P == 0) return found;
+  for (int cuts = (s.OH + 31) / 32, last = 0; cuts <= s.OH; ++cuts) {
+    const int TH = (s.OH + cuts - 1) / cuts;
+    if (TH == last) continue;
+    last = TH;
+    for (int NB = 1; NB <= s.N; ++NB) {
+      if (NB > 1 && (TH != s.OH || (NB - 1) * (TH + amax) + TH > 32)) break;
+      Geometry g;
+      g.mode = kGrid;
+      g.TH = TH; g.NB = NB;
+      g.PW = kTW + amax; g.PHI = TH + amax;
+      const int groups = ((NB - 1) * g.PHI + TH + 1) / 2 * 2;
+      g.npx = 8 * groups;
+      g.tiles_w = (s.OW + kTW - 1) / kTW;
+      g.tiles_h = (s.OH + TH - 1) / TH;
+      g.tiles_n = (s.N + NB - 1) / NB;
+      g.box_w = g.PW; g.box_h = g.PHI; g.box_n = NB;
+      g.reach = (groups - 1 + amax) * g.PW + amax + kTW;
+      consider(g);
+    }
+  }
+  return found;
+}
+
+// The geometry of a shape, planned once (the caller holds the state's mutex).
+const Geometry *geometry_of(Tc16State *t, const ConvShape &s) {
+  if (t->last_geo.mode < 0 || !same_conv(t->last_shape, s)) {
+    t->last_geo = Geometry{};
+    if (!plan_geometry(*t, s, &t->last_geo)) { t->last_geo.mode = -1; return nullptr; }
+    t->last_shape = s;
+  }
+  return &t->last_geo;
+}
+
+template <int NMAX, bool STACK>
+int launch_instance(const CUtensorMap &map_x, const CUtensorMap &map_out, const Tc16Params &p, unsigned grid, size_t smem, cudaStream_t st) {
+  static thread_local bool configured[16] = {false};
+  int dev = 0;
+  TETRIS_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev >= 16 || !configured[dev]) {
+    TETRIS_CUDA_TRY(cudaFuncSetAttribute(conv_tc16_kernel<NMAX, STACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    if (dev < 16) configured[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(Roles<NMAX>::kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)p.d; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = p.d > 1 ? 1 : 0;
+  TETRIS_CUDA_TRY(cudaLaunchKernelEx(&cfg, conv_tc16_kernel<NMAX, STACK>, map_x, map_out, p));
+  return TETRIS_OK;
+}
 
 }  // namespace
 
 void conv_tc16_state_delete(void *state) {
   Tc16State *s = static_cast<Tc16State *>(state);
   if (!s) return;
-  cudaFree(s->d_tiles); cudaFree(s->d_error); cudaFree(s->d_gate); cudaFree(s->d_out_scale);
-  cudaFree(s->d_scratch); cudaFree(s->d_tail_count);
+  cudaFree(s->d_tiles); cudaFree(s->d_error); cudaFree(s->d_out_scale);
   delete s;
 }
 
@@ -847,33 +1087,25 @@ int conv_tc16_prepare(tetris_filter *f, const float *d_dense) {
   if (!s) return TETRIS_OK;
   const int KS = f->kernel_size, taps = KS * KS;
   s->n_chunks = (f->in_channel + KC - 1) / KC;
-  s->bn = f->out_channel <= 64 ? 64 : 128;
-  const int oc_tiles = (f->out_channel + s->bn - 1) / s->bn;
-  const size_t elems = (size_t)taps * s->n_chunks * oc_tiles * s->bn * 64;
+  s->stack = f->out_channel <= 64;
+  s->oc_tiles = (f->out_channel + BM - 1) / BM;
+  const size_t elems = (size_t)taps * s->n_chunks * s->oc_tiles * BM * (s->stack ? 32 : 64);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) s->sms = 0;
-  if (s->sms < 1 || cudaMalloc(&s->d_tiles, elems * sizeof(__half)) != cudaSuccess || cudaMalloc(&s->d_error, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&s->d_gate, 2 * sizeof(unsigned)) != cudaSuccess ||
-      cudaMalloc(&s->d_tail_count, (size_t)s->sms * sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    conv_tc16_state_delete(s);
-    return TETRIS_OK;
-  }
-  cudaMemset(s->d_error, 0, sizeof(int));
-  cudaMemset(s->d_gate, 0, 2 * sizeof(unsigned));
-  cudaMemset(s->d_tail_count, 0, (size_t)s->sms * sizeof(int));
-  // per-channel scales: every output channel's largest |w| lands in [2^12, 2^13)
   float *d_w_scale = nullptr;
-  if (cudaMalloc(&d_w_scale, f->out_channel * sizeof(float)) != cudaSuccess ||
+  if (s->sms < 1 || cudaMalloc(&s->d_tiles, elems * sizeof(__half)) != cudaSuccess || cudaMalloc(&s->d_error, sizeof(int)) != cudaSuccess ||
+      cudaMalloc(&d_w_scale, f->out_channel * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&s->d_out_scale, f->out_channel * sizeof(float)) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(d_w_scale);
     conv_tc16_state_delete(s);
     return TETRIS_OK;
   }
+  cudaMemset(s->d_error, 0, sizeof(int));
+  // per-channel scales: every output channel's largest |w| lands in [2^12, 2^13)
   tc16_scales_kernel<<<f->out_channel, 256>>>(d_dense, f->in_channel * taps, d_w_scale, s->d_out_scale);
   tc16_weight_tiles_kernel<<<(unsigned)std::min<size_t>((elems + 255) / 256, 4096), 256>>>(
-      d_dense, s->d_tiles, f->out_channel, f->in_channel, KS, s->n_chunks, oc_tiles, s->bn, d_w_scale);
+      d_dense, s->d_tiles, f->out_channel, f->in_channel, KS, s->n_chunks, s->oc_tiles, s->stack ? 1 : 0, d_w_scale);
   const cudaError_t err = cudaGetLastError();
   cudaStreamSynchronize(0);  // (d_w_scale is freed next)
   cudaFree(d_w_scale);
@@ -885,216 +1117,110 @@ int conv_tc16_prepare(tetris_filter *f, const float *d_dense) {
   return TETRIS_OK;
 }
 
-// K steps per pipeline group of the kernel instance that serves channel tiles of `bn` and filters
-// of `ks` x `ks`: four for 64-channel tiles, whose MMAs are short (measured on VGG-19 conv1_2 and
-// the 64-channel 3x3 layers of ResNet-50: 3-4 % faster than pairs); 1x1 filters, where a group of
-// four would wait for four patches at a time, and 128-channel tiles stay with pairs.
-static int group_steps(int bn, int ks) { return bn == 64 && ks > 1 ? 4 : 2; }
-
 bool conv_tc16_supported(const tetris_filter *f, const ConvShape &s) {
-  if (!f->tc16_state || !f->tc_state || f->groups != 1) return false;  // (the split-TF32 variant is the out-of-range fallback)
-  if (s.S != 1 || s.N < 1 || s.OH < 1 || s.OW < 1 || (s.IC & 3) != 0) return false;
-  return conv_tc_supported(f, s);
+  if (!f->tc16_state || f->groups != 1) return false;
+  if (s.S < 1 || s.S > 4 || s.N < 1 || s.OH < 1 || s.OW < 1) return false;
+  return (long long)s.N * s.OH * s.OW < (1ll << 31);
+}
+
+// Estimated clocks of a launch (negative: the shape is not covered).
+double conv_tc16_cost(const tetris_filter *f, const ConvShape &s) {
+  if (!conv_tc16_supported(f, s)) return -1.;
+  Tc16State *t = static_cast<Tc16State *>(f->tc16_state);
+  std::lock_guard<std::mutex> lock(t->mutex);
+  const Geometry *g = geometry_of(t, s);
+  return g ? g->cost : -1.;
 }
 
 int launch_conv_tc16(const tetris_filter *f, const float *in, float *out, const ConvShape &s, cudaStream_t st) {
   Tc16State *t = static_cast<Tc16State *>(f->tc16_state);
   if (!conv_tc16_supported(f, s) || (reinterpret_cast<uintptr_t>(in) & 15) != 0) {
-    set_error("split-FP16 tensor-core variant covers stride 1, in_channel a multiple of 4 (at least 8), 16-byte aligned inputs");
+    set_error("split-FP16 tensor-core variant covers strides up to 4, in_channel a multiple of 4 (at least 8), 16-byte aligned inputs");
     return TETRIS_ERR_UNSUPPORTED;
   }
   EncodeFn enc = get_encode();
   if (!enc) { set_error("cuTensorMapEncodeTiled is not available from this driver"); return TETRIS_ERR_UNSUPPORTED; }
-  CUtensorMap map_x;
+  CUtensorMap map_x, map_out;
   Tc16Params p;
-  dim3 grid;
+  unsigned grid = 0;
+  int nmax = 128;
   size_t smem = 0;
-  int bn = 128;
   {
     std::lock_guard<std::mutex> lock(t->mutex);
     Tc16State::Setup *su = nullptr;
-    for (Tc16State::Setup &c : t->setups) {
-      const ConvShape &l = c.shape;
-      if (c.valid && c.in == in && l.relu == s.relu && l.N == s.N && l.H == s.H && l.W == s.W && l.P == s.P && l.S == s.S) { su = &c; break; }
-    }
+    for (Tc16State::Setup &c : t->setups)
+      if (c.valid && c.in == in && c.out == out && same_conv(c.shape, s)) { su = &c; break; }
     if (!su) {
+      const Geometry *g = geometry_of(t, s);
+      if (!g) { set_error("split-FP16 variant: the activation patches of this layer do not fit shared memory"); return TETRIS_ERR_UNSUPPORTED; }
       su = &t->setups[t->next_setup];
       t->next_setup = (t->next_setup + 1) % Tc16State::kSetups;
       su->valid = false;
       Tc16Params &q = su->params;
       q = Tc16Params{};
-      const int KS = s.KS, halo = KS - 1;
-      q.N = s.N; q.OH = s.OH; q.OW = s.OW; q.OC = s.OC; q.P = s.P; q.KS = KS;
-      q.linear = (KS == 1 && s.P == 0) ? 1 : 0;
+      q.N = s.N; q.OH = s.OH; q.OW = s.OW; q.OC = s.OC; q.S = s.S; q.P = s.P; q.KS = s.KS;
+      q.mode = g->mode; q.npx = g->npx; q.PW = g->PW; q.PHI = g->PHI; q.TH = g->TH; q.NB = g->NB;
+      q.box_rows = g->box_w * g->box_h * g->box_n;
+      q.x_stage_bytes = g->x_stage; q.n_x = g->n_x; q.n_w = g->n_w;
+      q.tiles_w = g->tiles_w; q.tiles_h = g->tiles_h; q.tiles_n = g->tiles_n; q.oc_tiles = t->oc_tiles;
+      q.total_tiles = g->tiles_w * g->tiles_h * g->tiles_n * t->oc_tiles;
+      q.by_oc_tiles = fast_div(q.oc_tiles); q.by_tiles_w = fast_div(q.tiles_w); q.by_tiles_h = fast_div(q.tiles_h);
+      q.by_PW = fast_div(q.PW); q.by_PHI = fast_div(q.PHI);
+      q.n_chunks = t->n_chunks; q.d = g->d;
       q.total_pixels = (long long)s.N * s.OH * s.OW;
+      q.out_scale = t->d_out_scale; q.error_flag = t->d_error; q.w_tiles = t->d_tiles;
       cuuint64_t dims[4], strides[3];
-      cuuint32_t box[4], estr[4] = {1, 1, 1, 1};
-      if (q.linear) {
-        q.PW = kTW; q.PHI = kTH; q.TH = kTH; q.NB = 1;
-        q.box_rows = BM;
-        q.tiles_w = (int)((q.total_pixels + BM - 1) / BM); q.tiles_h = 1; q.tiles_n = 1;
+      cuuint32_t box[4], estr[4] = {1, (cuuint32_t)s.S, (cuuint32_t)s.S, 1};
+      if (g->mode == kLinear) {
         dims[0] = (cuuint64_t)s.IC; dims[1] = (cuuint64_t)q.total_pixels; dims[2] = 1; dims[3] = 1;
         strides[0] = (cuuint64_t)s.IC * 4; strides[1] = strides[0] * dims[1]; strides[2] = strides[1];
-        box[0] = KC; box[1] = BM; box[2] = 1; box[3] = 1;
       } else {
-        q.PW = kTW + halo;
-        const bool whole = s.OH <= kTH;                 // the image's rows fit one tile
-        q.TH = whole ? s.OH : kTH;
-        q.PHI = q.TH + halo;
-        q.NB = whole ? std::max(1, std::min(s.N, (kTH + halo) / q.PHI)) : 1;
-        while (q.NB > 1 && (q.NB - 1) * q.PHI + q.TH > kTH) --q.NB;  // every valid group index stays below 16
-        q.box_rows = q.PW * q.PHI * q.NB;
-        q.tiles_w = (s.OW + kTW - 1) / kTW;
-        q.tiles_h = (s.OH + q.TH - 1) / q.TH;
-        q.tiles_n = (s.N + q.NB - 1) / q.NB;
-        // The other geometry: the image laid out with its padded width Wp = W + 2P, a tile = 128
-        // consecutive positions of that layout (8-pixel groups simply follow one another, so a
-        // window is again one descriptor).  Nothing is lost to tile shapes -- only the Wp - OW
-        // positions per row that are no outputs -- at the price of a patch of whole padded rows.
-        // Taken when it needs fewer tiles and the patches still fit beside three weight stages.
-        const int Wp = s.W + 2 * s.P;
-        const int span = (Wp - 1 + BM - 1) / Wp + 1;            // output rows a tile can touch
-        const int nrows = span + halo;
-        const long long tiles_flat = (long long)(((long long)s.OH * Wp + BM - 1) / BM) * s.N;
-        const long long tiles_2d = (long long)q.tiles_w * q.tiles_h * q.tiles_n;
-        const size_t flat_stage = ((size_t)(Wp * nrows + 8) * 128 + 1023) / 1024 * 1024;
-        const size_t room = kSmemBudget - (1024 + kStoreBytes + kNumBars * 8 + 16) - 3 * (size_t)t->bn * 256;
-        // (with room for two patches only -- a pair of K steps may need both -- it has to save 10 % of the tiles)
-        if (Wp <= 256 && nrows <= 256 &&
-            ((3 * flat_stage <= room && tiles_flat * 100 < tiles_2d * 97) || (2 * flat_stage <= room && tiles_flat * 100 < tiles_2d * 90))) {
-          q.flat = 1;
-          q.PW = Wp; q.PHI = nrows; q.TH = s.OH; q.NB = 1;
-          q.box_rows = Wp * nrows;
-          q.tiles_w = (int)(((long long)s.OH * Wp + BM - 1) / BM); q.tiles_h = 1; q.tiles_n = s.N;
-        }
         dims[0] = (cuuint64_t)s.IC; dims[1] = (cuuint64_t)s.W; dims[2] = (cuuint64_t)s.H; dims[3] = (cuuint64_t)s.N;
         strides[0] = (cuuint64_t)s.IC * 4; strides[1] = strides[0] * s.W; strides[2] = strides[1] * s.H;
-        box[0] = KC; box[1] = (cuuint32_t)q.PW; box[2] = (cuuint32_t)q.PHI; box[3] = (cuuint32_t)q.NB;
       }
+      // with element strides a box spans S times the pixels it loads
+      box[0] = KC; box[1] = (cuuint32_t)(g->box_w * s.S); box[2] = (cuuint32_t)(g->box_h * s.S); box[3] = (cuuint32_t)g->box_n;
       const CUresult r = enc(&su->map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(in), dims, strides, box, estr,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
       if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed with code %d", (int)r); return TETRIS_ERR_CUDA; }
-      // a stage holds the patch and whatever the windows of the 16 groups reach beyond it
-      const int reach_rows = q.linear ? BM : q.flat ? q.box_rows + 8 : (kTH + halo) * q.PW + halo + 8;
-      q.x_stage_bytes = (std::max(reach_rows, q.box_rows) * 128 + 1023) / 1024 * 1024;
-      q.n_chunks = t->n_chunks;
-      q.w_tiles = t->d_tiles;
-      q.error_flag = t->d_error;
-      q.gate = t->d_gate;
-      q.out_scale = t->d_out_scale;
-      int dev = 0, sms = 0;
-      TETRIS_CUDA_TRY(cudaGetDevice(&dev));
-      TETRIS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      const long long tiles = (long long)q.tiles_w * q.tiles_h * q.tiles_n * ((s.OC + t->bn - 1) / t->bn);
-      // K range split into d work items per tile when that fills the waves of CTAs better (as in the
-      // split-TF32 variant; cost in K steps: waves x (K steps + ~12 per item) + zeroing the output)
-      const double iters = (double)KS * KS * q.n_chunks;
-      const double zeroing = ((double)s.N * s.OH * s.OW * s.OC * 4 / 6.0e12 + 3e-6) * 1.9e9 / 500.0;
-      int best_d = 1;
-      double best_cost = std::ceil((double)tiles / sms) * (iters + 12.0);
-      q.relu = s.relu;
-      for (int d = 2; d <= 8 && d <= q.n_chunks && !f->deterministic && !s.relu; ++d) {  // (a rectified sum cannot be added up from slices)
-        if (q.n_chunks % d) continue;
-        const double cost = std::ceil((double)tiles * d / sms) * (iters / d + 12.0) + zeroing;
-        if (cost < 0.96 * best_cost) { best_cost = cost; best_d = d; }
+      // the output as boxes of 32 channels x 8 pixels
+      std::memset(&su->map_out, 0, sizeof(su->map_out));
+      q.tma_store = 0;
+      if ((s.OC & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+        cuuint64_t odims[4] = {(cuuint64_t)s.OC, (cuuint64_t)s.OW, (cuuint64_t)s.OH, (cuuint64_t)s.N}, ostrides[3];
+        if (g->mode == kLinear) { odims[1] = (cuuint64_t)q.total_pixels; odims[2] = odims[3] = 1; }
+        ostrides[0] = odims[0] * 4; ostrides[1] = ostrides[0] * odims[1]; ostrides[2] = ostrides[1] * odims[2];
+        const cuuint32_t obox[4] = {32, kTW, 1, 1}, oestr[4] = {1, 1, 1, 1};
+        if (enc(&su->map_out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, out, odims, ostrides, obox, oestr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
+          q.tma_store = 1;
       }
-      q.ksplit = best_d;
-      // Tail split: with T tiles on S CTAs the last wave holds T mod S tiles; when that is a small
-      // remainder, each of those tiles is cut into d K slices (d a divisor of the chunk count, at
-      // most one slice per CTA) that run side by side and are added up through the scratch blocks
-      // -- in slice order, so the result stays bit-reproducible, and with no zeroing of the output.
-      q.tail_tile0 = (int)tiles; q.tail_start = (int)tiles * best_d; q.tail_d = 1;
-      q.scratch = t->d_scratch; q.tail_count = t->d_tail_count;
-      if (best_d == 1 && tiles > sms && sms <= t->sms) {
-        const int full = (int)(tiles / sms) * sms, rest = (int)tiles - full;
-        int d = 0;
-        // (writing the slices out and adding them up costs a tile about as much as 30 K steps:
-        // the split has to save more than that)
-        for (int c = 2; c <= 8 && c <= q.n_chunks; ++c)
-          if (q.n_chunks % c == 0 && rest * c <= sms && iters * (c - 1) >= 32.0 * c) d = c;
-        if (rest > 0 && d >= 2 && !t->d_scratch &&  // (10 MB per filter: only for filters that have such a shape)
-            cudaMalloc(&t->d_scratch, (size_t)t->sms * BM * t->bn * sizeof(float)) != cudaSuccess) {
-          cudaGetLastError();
-          t->d_scratch = nullptr;
-          d = 0;
-        }
-        if (rest > 0 && d >= 2) { q.tail_tile0 = full; q.tail_start = full; q.tail_d = d; q.scratch = t->d_scratch; }
-      }
-      // shared memory: activation ring, weight ring, store staging, barriers
-      const size_t wbytes = (size_t)t->bn * 128 * group_steps(t->bn, KS);  // a weight stage holds a group of K steps
-      const size_t fixed = 1024 + kStoreBytes + kNumBars * 8 + 16;
-      const int chunks_per_item = q.n_chunks / best_d;
-      q.n_w = kWStagesMax;
-      q.n_x = (int)std::min<size_t>(kXStagesMax, (kSmemBudget - fixed - q.n_w * wbytes) / q.x_stage_bytes);
-      while (q.n_x < 3 && q.n_w > 3) {  // (a group of K steps may straddle two patches: at least two stages, better three)
-        --q.n_w;
-        q.n_x = (int)std::min<size_t>(kXStagesMax, (kSmemBudget - fixed - q.n_w * wbytes) / q.x_stage_bytes);
-      }
-      if (q.n_x < 2) { set_error("split-FP16 variant: the activation patches of this layer do not fit shared memory"); return TETRIS_ERR_UNSUPPORTED; }
-      if (KS > 1) q.n_x = std::min(q.n_x, 3);          // a patch feeds KS*KS steps: three stages are ample
-      q.n_x = std::max(2, std::min(q.n_x, std::max(3, 2 * chunks_per_item)));  // (patches are fetched across work items)
-      su->smem = fixed + (size_t)q.n_x * q.x_stage_bytes + (size_t)q.n_w * wbytes;
-      su->grid = dim3((unsigned)std::min<long long>(q.tail_start + (tiles - q.tail_tile0) * q.tail_d, sms));  // persistent: one CTA per SM
+      // persistent CTAs, one per SM; a tile cut into K slices takes a cluster of its own
+      su->grid = (unsigned)(g->d > 1 ? q.total_tiles * g->d : std::min(q.total_tiles, t->sms));
+      su->nmax = g->nmax;
+      su->smem = g->smem;
       su->in = in;
+      su->out = out;
       su->shape = s;
       su->valid = true;
     }
     map_x = su->map_x;
+    map_out = su->map_out;
     p = su->params;
     grid = su->grid;
+    nmax = su->nmax;
     smem = su->smem;
-    bn = t->bn;
   }
   p.out = out;
+  p.relu = s.relu;
   p.withhold_first_load = test_injection(&p.spin_limit);
-#ifdef TETRIS_TC16_PROF
-  static long long *d_prof = nullptr;
-  const bool prof = getenv("TETRIS_TC16_PROF") != nullptr;
-  if (prof) {
-    if (!d_prof) cudaMalloc(&d_prof, 64 * sizeof(long long));
-    cudaMemset(d_prof, 0, 64 * sizeof(long long));
-    p.prof = d_prof;
-  }
-#endif
-  static thread_local bool configured[16] = {false};
-  int dev = 0;
-  TETRIS_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev >= 16 || !configured[dev]) {
-    TETRIS_CUDA_TRY(cudaFuncSetAttribute(conv_tc16_kernel<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
-    TETRIS_CUDA_TRY(cudaFuncSetAttribute(conv_tc16_kernel<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
-    TETRIS_CUDA_TRY(cudaFuncSetAttribute(conv_tc16_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
-    if (dev < 16) configured[dev] = true;
-  }
-  if (p.ksplit > 1)  // the work items add into the output
-    TETRIS_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)s.N * s.OH * s.OW * s.OC * sizeof(float), st));
-  if (bn == 64 && group_steps(64, s.KS) == 4)
-    conv_tc16_kernel<64, 4><<<grid, kThreads, smem, st>>>(map_x, p);
-  else if (bn == 64)
-    conv_tc16_kernel<64, 2><<<grid, kThreads, smem, st>>>(map_x, p);
-  else
-    conv_tc16_kernel<128, 2><<<grid, kThreads, smem, st>>>(map_x, p);
-  TETRIS_CUDA_TRY(cudaGetLastError());
+  const int rc = nmax == 256 ? (t->stack ? launch_instance<256, true>(map_x, map_out, p, grid, smem, st) : launch_instance<256, false>(map_x, map_out, p, grid, smem, st))
+                             : (t->stack ? launch_instance<128, true>(map_x, map_out, p, grid, smem, st) : launch_instance<128, false>(map_x, map_out, p, grid, smem, st));
+  if (rc) return rc;
   count_launch();
   if (p.relu) note_relu_fused();
-#ifdef TETRIS_TC16_PROF
-  if (prof) {
-    long long h[64];
-    cudaDeviceSynchronize();
-    cudaMemcpy(h, d_prof, sizeof(h), cudaMemcpyDeviceToHost);
-    const char *names[6] = {"x loader (xempty)", "w loader (gdone)", "cp (gdone-4, xconv)", "mma (afull, pempty, wfull; mmas, commit)", "convert (xfull)", "sum (gdone)"};
-    const long long tiles_ = (long long)p.tiles_w * p.tiles_h * p.tiles_n * ((s.OC + bn - 1) / bn);
-    const long long items = (p.tail_start + (tiles_ - p.tail_tile0) * p.tail_d + grid.x - 1) / grid.x;
-    const long long steps = (long long)(p.tail_start / grid.x) * s.KS * s.KS * (p.n_chunks / p.ksplit) + (long long)s.KS * s.KS * (p.n_chunks / p.tail_d);
-    fprintf(stderr, "[tc16 prof] grid %u, items/CTA %lld, K steps/CTA %lld, n_x %d n_w %d\n", grid.x, items, steps, p.n_x, p.n_w);
-    for (int r = 0; r < 6; ++r)
-      fprintf(stderr, "[tc16 prof] %-42s total %9lld clk (%5.0f per K step); waits: %lld %lld %lld %lld %lld\n", names[r], h[r * 8],
-              (double)h[r * 8] / (double)steps, h[r * 8 + 1], h[r * 8 + 2], h[r * 8 + 3], h[r * 8 + 4], h[r * 8 + 5]);
-  }
-#endif
-  // The guard: the split-TF32 variant, queued behind; it returns at once unless the largest
-  // activation of this launch lies outside FP16's useful window, in which case it recomputes the layer.
-  return launch_conv_tc_gated(f, in, out, s, st, t->d_gate);
+  return TETRIS_OK;
 }
 
 // 0 = no timeout seen so far, 1 = a bounded wait gave up in some launch (the flag is cleared).
@@ -1103,12 +1229,7 @@ int conv_tc16_check_error(const tetris_filter *f) {
   if (!t) return 0;
   int flag = 0;
   if (cudaMemcpy(&flag, t->d_error, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return 1;
-  if (flag) {
-    // (a launch that gave up may have left the guard's words and the last-wave counters half way)
-    cudaMemset(t->d_error, 0, sizeof(int));
-    cudaMemset(t->d_gate, 0, 2 * sizeof(unsigned));
-    cudaMemset(t->d_tail_count, 0, (size_t)t->sms * sizeof(int));
-  }
+  if (flag) cudaMemset(t->d_error, 0, sizeof(int));
   return flag;
 }
 

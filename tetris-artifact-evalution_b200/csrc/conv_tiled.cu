@@ -439,11 +439,11 @@ int make_plan(const tetris_filter *f, const ConvShape &s, Plan *plan) {
   if (rc) return rc;
   fill_plan(f, s, cands[0], sm_count, plan);
   // The list kernel's wavefront model counts issue slots only and comes out 1.2-1.75x below the
-  // measured time (1.45x on the layers where the two kernels are close); the tensor-core figure
-  // is a measured one.
-  // (the split-FP16 variant runs the same contraction at roughly half the clocks per K step)
-  if (conv_tc16_supported(f, s) && 0.55 * tc_cost(f, s, sm_count) < 1.45 * cands[0].cost) plan->use_tc = 2;
-  else plan->use_tc = conv_tc_supported(f, s) && tc_cost(f, s, sm_count) < 1.45 * cands[0].cost ? 1 : 0;
+  // measured time (1.45x on the layers where the two kernels are close); the tensor-core figures
+  // are measured ones.
+  const double tc16 = conv_tc16_cost(f, s);
+  if (tc16 >= 0. && tc16 < 1.45 * cands[0].cost) plan->use_tc = 2;
+  else plan->use_tc = tc16 < 0. && conv_tc_supported(f, s) && tc_cost(f, s, sm_count) < 1.45 * cands[0].cost ? 1 : 0;
   return TETRIS_OK;
 }
 
@@ -609,7 +609,7 @@ int tune_conv_tiled(const tetris_filter *f, const float *in, float *out, const C
       if (ms < best) { best = ms; best_plan.use_tc = 1; }
     }
   }
-  // ... and the split-FP16 variant (its launch includes the guard kernel queued behind it)
+  // ... and the split-FP16 variant
   if (!rc && conv_tc16_supported(f, s) && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
     rc = launch_conv_tc16(f, in, out, s, st);
     cudaEventRecord(e0, st);

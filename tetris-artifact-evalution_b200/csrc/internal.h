@@ -94,11 +94,10 @@ bool conv_tc_supported(const tetris_filter *f, const ConvShape &s);
 int launch_conv_tc(const tetris_filter *f, const float *in, float *out, const ConvShape &s,
                    cudaStream_t st);
 int conv_tc_check_error(const tetris_filter *f);
-int launch_conv_tc_gated(const tetris_filter *f, const float *in, float *out, const ConvShape &s, cudaStream_t st,
-                         unsigned *gate);
 int conv_tc16_prepare(tetris_filter *f, const float *d_dense);
 void conv_tc16_state_delete(void *state);
 bool conv_tc16_supported(const tetris_filter *f, const ConvShape &s);
+double conv_tc16_cost(const tetris_filter *f, const ConvShape &s);  // estimated clocks of a launch, negative: not covered
 int launch_conv_tc16(const tetris_filter *f, const float *in, float *out, const ConvShape &s, cudaStream_t st);
 int conv_tc16_check_error(const tetris_filter *f);
 int launch_depthwise(const tetris_filter *f, const float *in, float *out, const ConvShape &s,
