@@ -115,3 +115,19 @@ def test_layer_chain_replays_from_a_cuda_graph(tb, torch_cuda, oracle):
     y2 = oracle.host_conv2d(y1, f2w, 1, 1)
     bad, _, _ = oracle.compare(out.cpu().numpy().transpose(0, 3, 1, 2), y2)
     assert bad == 0
+
+
+# channel counts around the tiles' (4 x 1024, 8 x 512, 32 x 128), pixel counts that end inside one,
+# and a tensor that is only 4-byte aligned
+@pytest.mark.parametrize("n,c,h,w", [(2, 4, 33, 32), (1, 1, 40, 40), (2, 8, 23, 23), (1, 9, 16, 16), (2, 32, 8, 16), (1, 33, 43, 3), (3, 64, 7, 7), (2, 36, 17, 31)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_layout_tiles_are_exact(tb, torch_cuda, n, c, h, w, offset):
+    torch = torch_cuda
+    size = n * c * h * w
+    x = torch.rand(size + offset, device="cuda")[offset:]
+    y = torch.full((size + offset,), float("nan"), device="cuda")[offset:]
+    z = torch.full((size + offset,), float("nan"), device="cuda")[offset:]
+    tb.nchw_to_nhwc(x, y, n, c, h, w)
+    assert torch.equal(y.view(n, h, w, c), x.view(n, c, h, w).permute(0, 2, 3, 1).contiguous())
+    tb.nhwc_to_nchw(y, z, n, c, h, w)
+    assert torch.equal(z, x)
