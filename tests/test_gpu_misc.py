@@ -131,3 +131,20 @@ def test_layout_tiles_are_exact(tb, torch_cuda, n, c, h, w, offset):
     assert torch.equal(y.view(n, h, w, c), x.view(n, c, h, w).permute(0, 2, 3, 1).contiguous())
     tb.nhwc_to_nchw(y, z, n, c, h, w)
     assert torch.equal(z, x)
+
+
+@pytest.mark.parametrize("n,c,h,ks,stride,pad", [(2, 64, 20, 3, 1, 1), (1, 32, 7, 3, 1, 1), (2, 32, 15, 3, 2, 1), (2, 24, 19, 3, 1, 1), (1, 20, 12, 3, 2, 1), (1, 7, 9, 5, 1, 2)])
+def test_depthwise_rectifies_at_its_store(tb, torch_cuda, oracle, n, c, h, ks, stride, pad):
+    torch = torch_cuda
+    rng = np.random.default_rng(c + h)
+    filt = rng.normal(0, 0.2, (c, 1, ks, ks)).astype(np.float32)
+    x = (rng.random((n, c, h, h), dtype=np.float32) - 0.4).astype(np.float32)
+    f = tb.SparseFilter(filt, c, c, ks, groups=c)
+    oh = tb.out_extent(h, ks, stride, pad)
+    xin = torch.from_numpy(np.ascontiguousarray(x.transpose(0, 2, 3, 1))).cuda()
+    out = torch.full((n, oh, oh, c), float("nan"), device="cuda")
+    before = tb.launch_count()
+    tb.sparse_conv2d_fused(f, xin, out, n, h, h, stride, pad, relu=True)
+    assert tb.launch_count() - before == 1
+    got = out.cpu().numpy().transpose(0, 3, 1, 2)
+    assert oracle.compare(got, np.maximum(oracle.host_depthwise_conv2d(x, filt, stride, pad), 0))[0] == 0

@@ -23,6 +23,9 @@ namespace {
 // windows, i.e. a block computes a 2-D patch of the image, so that the input rows and columns
 // neighbouring threads share are found in L1 (with a block one window tall the L2 -> SM traffic
 // measured 3.2x the input).
+__device__ __forceinline__ float4 relu4(float4 v) {
+  return make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+}
 struct DwGrid { int cq, wtiles, htiles, qb, aw, ah, qblocks, xblocks, yblocks; };
 
 // 3x3, stride S, four channels per thread, TW output columns x RH output rows per thread.  The
@@ -96,7 +99,7 @@ depthwise3x3_kernel(const float4 *__restrict__ in, float4 *__restrict__ out,
     float4 *o = out + (((size_t)n * s.OH + oh0 + a) * s.OW + ow0) * cq + q;
 #pragma unroll
     for (int j = 0; j < TW; ++j)
-      if (ow0 + j < s.OW) o[(size_t)j * cq] = acc[a][j];
+      if (ow0 + j < s.OW) o[(size_t)j * cq] = s.relu ? relu4(acc[a][j]) : acc[a][j];
   }
 }
 
@@ -119,6 +122,7 @@ struct DwTmaParams {
   int N, C, OH, OW, P;
   int tiles_x, tiles_y, cgs;
   int total;
+  int relu;  // max(y, 0) at the store
 };
 
 __device__ __forceinline__ uint32_t dw_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -220,7 +224,7 @@ depthwise3x3_tma_kernel(const __grid_constant__ CUtensorMap map, const DwTmaPara
 #pragma unroll
     for (int a = 0; a < R; ++a) {
       const int oh = ty * THO + row0 + a;
-      if (ow < p.OW && oh < p.OH) p.out[(((size_t)n * p.OH + oh) * p.OW + ow) * cq + cg * 8 + q] = acc[a];
+      if (ow < p.OW && oh < p.OH) p.out[(((size_t)n * p.OH + oh) * p.OW + ow) * cq + cg * 8 + q] = p.relu ? relu4(acc[a]) : acc[a];
     }
     __syncthreads();  // everybody is done with this stage before it is loaded again
   }
@@ -256,7 +260,7 @@ depthwise_any_kernel(const float *__restrict__ in, float *__restrict__ out,
       acc = fmaf(__ldg(&w[r * s.KS + q]), __ldg(&img[((size_t)ih * s.W + iw) * s.IC]), acc);
     }
   }
-  out[idx] = acc;
+  out[idx] = s.relu ? fmaxf(acc, 0.f) : acc;
 }
 
 typedef CUresult (*DwEncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -316,6 +320,7 @@ int launch_depthwise_tma(const tetris_filter *f, const float *in, float *out, co
   const long long total = (long long)p.tiles_x * p.tiles_y * s.N * p.cgs;
   if (total > 0x7FFFFFFFll / 8) return 1;
   p.total = (int)total;
+  p.relu = s.relu;
   const size_t smem = (size_t)nst * bx * by * 128 + 128;
   static thread_local bool configured[16] = {false};
   if (dev >= 16 || !configured[dev]) {
@@ -348,7 +353,7 @@ int launch_depthwise(const tetris_filter *f, const float *in, float *out, const 
   if (elems <= 0) return TETRIS_OK;
   {
     const int rc = launch_depthwise_tma(f, in, out, s, st);
-    if (rc == 0) { count_launch(); return TETRIS_OK; }
+    if (rc == 0) { count_launch(); note_relu_fused(); return TETRIS_OK; }
     if (rc != 1) return rc;
   }
   const bool vec = s.KS == 3 && (s.S == 1 || s.S == 2) && (s.OC & 3) == 0 &&
@@ -391,6 +396,7 @@ int launch_depthwise(const tetris_filter *f, const float *in, float *out, const 
   }
   TETRIS_CUDA_TRY(cudaGetLastError());
   count_launch();
+  note_relu_fused();
   return TETRIS_OK;
 }
 
