@@ -36,48 +36,6 @@ void set_error(const char *fmt, ...) {
 
 namespace {
 
-// Activation workspace of tetris_conv2d_host, one per device, grown on demand.
-struct Workspace {
-  std::mutex mutex;
-  void *ptr = nullptr;
-  size_t bytes = 0;
-};
-constexpr int kMaxWsDevices = 64;
-Workspace g_workspace[kMaxWsDevices];
-
-// Makes `device` current for the lifetime of the object and restores the previous one.
-struct DeviceGuard {
-  int prev = -1;
-  bool ok = false;
-  explicit DeviceGuard(int device) {
-    if (cudaGetDevice(&prev) != cudaSuccess) return;
-    ok = cudaSetDevice(device) == cudaSuccess;
-  }
-  ~DeviceGuard() {
-    if (prev >= 0) cudaSetDevice(prev);
-  }
-};
-
-int make_shape(const tetris_filter *f, int batch, int h, int w, int stride, int padding,
-               ConvShape *s) {
-  if (!f) { set_error("filter handle is NULL"); return TETRIS_ERR_INVALID; }
-  if (batch < 0 || h < 1 || w < 1 || stride < 1 || padding < 0) {
-    set_error("bad conv shape: batch=%d h=%d w=%d stride=%d padding=%d", batch, h, w, stride, padding);
-    return TETRIS_ERR_INVALID;
-  }
-  s->N = batch; s->H = h; s->W = w; s->IC = f->in_channel; s->OC = f->out_channel;
-  s->KS = f->kernel_size; s->S = stride; s->P = padding;
-  // output extent as in Tetris/spconv2d.cc:339-340
-  s->OH = (h + 2 * padding - f->kernel_size) / stride + 1;
-  s->OW = (w + 2 * padding - f->kernel_size) / stride + 1;
-  if (h + 2 * padding < f->kernel_size || w + 2 * padding < f->kernel_size) {
-    set_error("image %dx%d (+pad %d) smaller than the %dx%d kernel", h, w, padding,
-              f->kernel_size, f->kernel_size);
-    return TETRIS_ERR_INVALID;
-  }
-  return TETRIS_OK;
-}
-
 thread_local bool tl_relu_fused = false;
 
 int dispatch_kernel(const tetris_filter *f, const float *in, float *out, const ConvShape &s,
@@ -119,6 +77,26 @@ int dispatch_kernel(const tetris_filter *f, const float *in, float *out, const C
 }
 
 }  // namespace
+
+int make_shape(const tetris_filter *f, int batch, int h, int w, int stride, int padding,
+               ConvShape *s) {
+  if (!f) { set_error("filter handle is NULL"); return TETRIS_ERR_INVALID; }
+  if (batch < 0 || h < 1 || w < 1 || stride < 1 || padding < 0) {
+    set_error("bad conv shape: batch=%d h=%d w=%d stride=%d padding=%d", batch, h, w, stride, padding);
+    return TETRIS_ERR_INVALID;
+  }
+  s->N = batch; s->H = h; s->W = w; s->IC = f->in_channel; s->OC = f->out_channel;
+  s->KS = f->kernel_size; s->S = stride; s->P = padding;
+  // output extent as in Tetris/spconv2d.cc:339-340
+  s->OH = (h + 2 * padding - f->kernel_size) / stride + 1;
+  s->OW = (w + 2 * padding - f->kernel_size) / stride + 1;
+  if (h + 2 * padding < f->kernel_size || w + 2 * padding < f->kernel_size) {
+    set_error("image %dx%d (+pad %d) smaller than the %dx%d kernel", h, w, padding,
+              f->kernel_size, f->kernel_size);
+    return TETRIS_ERR_INVALID;
+  }
+  return TETRIS_OK;
+}
 
 void note_relu_fused() { tl_relu_fused = true; }
 
@@ -201,17 +179,20 @@ int tetris_filter_create_ex(const float *filter_oihw, int in_channel, int out_ch
   int32_t *d_scratch = nullptr;
   int rc = TETRIS_OK;
   auto fail = [&](int code) {
-    cudaFree(d_dense); cudaFree(d_scratch);
     f->d_dense = nullptr;
+    cudaDeviceSynchronize();
+    device_free(d_dense); device_free(d_scratch);
     tetris_filter_destroy(f);
     return code;
   };
-  if (cudaMalloc(&d_dense, dense_bytes) != cudaSuccess) {
+  auto alloc = [&](void **p, size_t bytes, const char *what) {
+    if (device_alloc(p, bytes) == cudaSuccess) return true;
     cudaGetLastError();
-    set_error("cudaMalloc of %zu bytes for the dense filter failed", dense_bytes);
-    return fail(TETRIS_ERR_NOMEM);
-  }
-  if (cudaMemcpy(d_dense, filter_oihw, dense_bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+    set_error("allocation of %zu bytes of device memory for %s failed", bytes, what);
+    return false;
+  };
+  if (!alloc((void **)&d_dense, dense_bytes, "the dense filter")) return fail(TETRIS_ERR_NOMEM);
+  if (copy_to_device(d_dense, filter_oihw, dense_bytes, 0) != cudaSuccess) {
     set_error("copy of the dense filter to the device failed");
     return fail(TETRIS_ERR_CUDA);
   }
@@ -222,94 +203,67 @@ int tetris_filter_create_ex(const float *filter_oihw, int in_channel, int out_ch
     int64_t nnz = 0;
     for (size_t i = 0; i < dense_bytes / sizeof(float); ++i) nnz += filter_oihw[i] != 0.f;
     f->nnz = nnz;
+    if (cudaStreamSynchronize(0) != cudaSuccess) {
+      set_error("copy of the dense filter to the device failed: %s", cudaGetErrorString(cudaGetLastError()));
+      return fail(TETRIS_ERR_CUDA);
+    }
     *out = f;
     return TETRIS_OK;
   }
 
-  // List pieces are staged in shared memory by the tiled kernel, so their length is bounded:
-  // when the stage size is left to the engine, halve it until the longest piece is short enough.
+  // Both forms are counted and scanned, then the host reads their totals and longest pieces once.
+  // List pieces are staged in shared memory by the tiled kernel, so their length is bounded: when
+  // the stage size is left to the engine, it is halved (and the pieces counted again) until the
+  // longest piece is short enough.
   constexpr int kPieceUnitsTarget = 640;
+  struct Meta { int32_t list_total, list_longest, prog_total, prog_longest; unsigned long long nnz; } meta;
   const int B = (out_channel + K - 1) / K;
   int T = 0, P = 0;
-  std::vector<int32_t> h_offsets;
-  auto alloc_offsets = [&](int32_t **d_offsets) {
-    cudaFree(d_scratch); cudaFree(*d_offsets);
-    d_scratch = nullptr; *d_offsets = nullptr;
-    return cudaMalloc(&d_scratch, compress_scratch_bytes(P)) == cudaSuccess &&
-           cudaMalloc(d_offsets, (size_t)(P + 1) * sizeof(int32_t)) == cudaSuccess;
-  };
-  auto fetch_offsets = [&](const int32_t *d_offsets, int *longest) {
-    h_offsets.resize(P + 1);
-    if (cudaMemcpy(h_offsets.data(), d_offsets, (size_t)(P + 1) * sizeof(int32_t),
-                   cudaMemcpyDeviceToHost) != cudaSuccess)
-      return false;
-    *longest = 0;
-    for (int i = 0; i < P; ++i) *longest = std::max(*longest, h_offsets[i + 1] - h_offsets[i]);
-    return true;
-  };
-  // ---- LIST form (tiled kernel) ----
   for (;;) {
     T = (in_channel + TIC - 1) / TIC;
     P = B * T;
-    if (!alloc_offsets(&f->d_list_offsets)) {
-      cudaGetLastError();
-      set_error("cudaMalloc of compressor scratch failed");
+    device_free(d_scratch); device_free(f->d_list_offsets); device_free(f->d_prog_offsets);
+    d_scratch = f->d_list_offsets = f->d_prog_offsets = nullptr;
+    const size_t lens_bytes = ((size_t)P * sizeof(int32_t) + 15) / 16 * 16;
+    if (!alloc((void **)&d_scratch, 2 * lens_bytes + sizeof(Meta), "the compressor") ||
+        !alloc((void **)&f->d_list_offsets, (size_t)(P + 1) * sizeof(int32_t), "piece offsets") ||
+        !alloc((void **)&f->d_prog_offsets, (size_t)(P + 1) * sizeof(int32_t), "piece offsets"))
       return fail(TETRIS_ERR_NOMEM);
-    }
-    if ((rc = list_count(d_dense, in_channel, out_channel, kernel_size, K, TIC, B, T, d_scratch, 0)) ||
-        (rc = compress_scan(d_scratch, f->d_list_offsets, P, 0)))
+    int32_t *list_lens = d_scratch, *prog_lens = d_scratch + lens_bytes / sizeof(int32_t);
+    Meta *d_meta = reinterpret_cast<Meta *>(d_scratch + 2 * lens_bytes / sizeof(int32_t));
+    if ((rc = list_count(d_dense, in_channel, out_channel, kernel_size, K, TIC, B, T, list_lens, 0)) ||
+        (rc = compress_count(d_dense, in_channel, out_channel, kernel_size, K, TIC, B, T, prog_lens, &d_meta->nnz, 0)) ||
+        (rc = compress_scan(list_lens, f->d_list_offsets, P, &d_meta->list_total, 0)) ||
+        (rc = compress_scan(prog_lens, f->d_prog_offsets, P, &d_meta->prog_total, 0)))
       return fail(rc);
-    if (!fetch_offsets(f->d_list_offsets, &f->max_list_units)) {
+    if (cudaMemcpy(&meta, d_meta, sizeof(meta), cudaMemcpyDeviceToHost) != cudaSuccess) {
       set_error("compressor count/scan failed: %s", cudaGetErrorString(cudaGetLastError()));
       return fail(TETRIS_ERR_CUDA);
     }
-    if (!auto_tic || f->max_list_units <= kPieceUnitsTarget || TIC <= 4) break;
+    if (!auto_tic || meta.list_longest <= kPieceUnitsTarget || TIC <= 4) break;
     TIC /= 2;
   }
   f->tile_ic = TIC;
   f->n_oc_blocks = B; f->n_stages = T;
-  f->n_list_units = (int64_t)h_offsets[P] + 2;
-  if (cudaMalloc(&f->d_lists, (size_t)f->n_list_units * sizeof(uint64_t)) != cudaSuccess) {
-    cudaGetLastError();
-    set_error("cudaMalloc of %lld list units failed", (long long)f->n_list_units);
+  f->max_list_units = meta.list_longest; f->max_prog_ops = meta.prog_longest;
+  f->nnz = (int64_t)meta.nnz;
+  f->n_list_units = (int64_t)meta.list_total + 2;
+  f->n_ops = (int64_t)meta.prog_total + kTailPadOps;
+  if (!alloc((void **)&f->d_lists, (size_t)f->n_list_units * sizeof(uint64_t), "the weight lists") ||
+      !alloc((void **)&f->d_ops, (size_t)f->n_ops * sizeof(uint64_t), "the weight programs"))
     return fail(TETRIS_ERR_NOMEM);
-  }
   if ((rc = list_fill(d_dense, in_channel, out_channel, kernel_size, K, TIC, B, T,
-                      f->d_list_offsets, f->d_lists, f->n_list_units, 0)))
+                      f->d_list_offsets, f->d_lists, f->n_list_units, 0)) ||
+      (rc = compress_fill(d_dense, in_channel, out_channel, kernel_size, K, TIC, B, T,
+                          f->d_prog_offsets, f->d_ops, f->n_ops, 0)) ||
+      (rc = tensor_prepare(f, d_dense)))
     return fail(rc);
-  // ---- PROGRAM form (generic kernel) ----
-  if (!alloc_offsets(&f->d_prog_offsets)) {
-    cudaGetLastError();
-    set_error("cudaMalloc of compressor scratch failed");
-    return fail(TETRIS_ERR_NOMEM);
-  }
-  if ((rc = compress_count(d_dense, in_channel, out_channel, kernel_size, K, TIC, B, T, d_scratch, 0)) ||
-      (rc = compress_scan(d_scratch, f->d_prog_offsets, P, 0)))
-    return fail(rc);
-  unsigned long long nnz = 0;
-  if (!fetch_offsets(f->d_prog_offsets, &f->max_prog_ops) ||
-      cudaMemcpy(&nnz, compress_nnz_ptr(d_scratch, P), sizeof(nnz), cudaMemcpyDeviceToHost) != cudaSuccess) {
-    set_error("compressor count/scan failed: %s", cudaGetErrorString(cudaGetLastError()));
-    return fail(TETRIS_ERR_CUDA);
-  }
-  const int32_t total = h_offsets[P];
-  f->nnz = (int64_t)nnz;
-  f->n_ops = (int64_t)total + kTailPadOps;
-  if (cudaMalloc(&f->d_ops, (size_t)f->n_ops * sizeof(uint64_t)) != cudaSuccess) {
-    cudaGetLastError();
-    set_error("cudaMalloc of %lld program records failed", (long long)f->n_ops);
-    return fail(TETRIS_ERR_NOMEM);
-  }
-  if ((rc = compress_fill(d_dense, in_channel, out_channel, kernel_size, K, TIC, B, T,
-                          f->d_prog_offsets, f->d_ops, f->n_ops, 0)))
-    return fail(rc);
-  if ((rc = conv_tc_prepare(f, d_dense)) || (rc = conv_tc16_prepare(f, d_dense))) return fail(rc);
-  if (cudaDeviceSynchronize() != cudaSuccess) {
+  if (cudaStreamSynchronize(0) != cudaSuccess) {
     set_error("compressor fill failed: %s", cudaGetErrorString(cudaGetLastError()));
     return fail(TETRIS_ERR_CUDA);
   }
-  cudaFree(d_dense);
-  cudaFree(d_scratch);
+  device_free(d_dense);
+  device_free(d_scratch);
   *out = f;
   return TETRIS_OK;
 }
@@ -317,14 +271,15 @@ int tetris_filter_create_ex(const float *filter_oihw, int in_channel, int out_ch
 void tetris_filter_destroy(tetris_filter_t *f) {
   if (!f) return;
   DeviceGuard guard(f->device);
-  cudaFree(f->d_ops);
-  cudaFree(f->d_prog_offsets);
-  cudaFree(f->d_lists);
-  cudaFree(f->d_list_offsets);
+  cudaDeviceSynchronize();  // launches on any stream may still read the filter
+  device_free(f->d_ops);
+  device_free(f->d_prog_offsets);
+  device_free(f->d_lists);
+  device_free(f->d_list_offsets);
   tiled_plan_cache_delete(f->plan_cache);
   conv_tc_state_delete(f->tc_state);
   conv_tc16_state_delete(f->tc16_state);
-  cudaFree(f->d_dense);
+  device_free(f->d_dense);
   delete f;
 }
 
@@ -352,7 +307,7 @@ int tetris_filter_download(const tetris_filter_t *f, uint64_t *ops, size_t ops_c
   DeviceGuard guard(f->device);
   if (ops) {
     if (ops_capacity < (size_t)f->n_ops) { set_error("ops buffer too small"); return TETRIS_ERR_INVALID; }
-    TETRIS_CUDA_TRY(cudaMemcpy(ops, f->d_ops, (size_t)f->n_ops * sizeof(uint64_t), cudaMemcpyDeviceToHost));
+    TETRIS_CUDA_TRY(copy_to_host(ops, f->d_ops, (size_t)f->n_ops * sizeof(uint64_t), 0));
   }
   if (prog_offsets) {
     const size_t n = (size_t)f->n_oc_blocks * f->n_stages + 1;
@@ -369,7 +324,7 @@ int tetris_filter_download_lists(const tetris_filter_t *f, uint64_t *units, size
   DeviceGuard guard(f->device);
   if (units) {
     if (units_capacity < (size_t)f->n_list_units) { set_error("units buffer too small"); return TETRIS_ERR_INVALID; }
-    TETRIS_CUDA_TRY(cudaMemcpy(units, f->d_lists, (size_t)f->n_list_units * sizeof(uint64_t), cudaMemcpyDeviceToHost));
+    TETRIS_CUDA_TRY(copy_to_host(units, f->d_lists, (size_t)f->n_list_units * sizeof(uint64_t), 0));
   }
   if (list_offsets) {
     const size_t n = (size_t)f->n_oc_blocks * f->n_stages + 1;
@@ -503,157 +458,6 @@ int tetris_nchw_to_nhwc(const float *d_src, float *d_dst, int N, int C, int H, i
 int tetris_nhwc_to_nchw(const float *d_src, float *d_dst, int N, int C, int H, int W, void *stream) {
   if (!d_src || !d_dst || N < 0 || C < 1 || H < 1 || W < 1) { set_error("bad layout arguments"); return TETRIS_ERR_INVALID; }
   return launch_nhwc_to_nchw(d_src, d_dst, N, C, H, W, (cudaStream_t)stream);
-}
-
-int tetris_conv2d_host(const tetris_filter_t *f, const float *h_input_nchw,
-                       float *h_output_nchw, int batch_size, int img_h, int img_w, int stride,
-                       int padding, void *stream) {
-  ConvShape s;
-  int rc = make_shape(f, batch_size, img_h, img_w, stride, padding, &s);
-  if (rc) return rc;
-  if (batch_size == 0) return TETRIS_OK;
-  if (!h_input_nchw || !h_output_nchw) { set_error("input or output pointer is NULL"); return TETRIS_ERR_INVALID; }
-  DeviceGuard guard(f->device);
-  if (!guard.ok) { set_error("cudaSetDevice(%d) failed", f->device); return TETRIS_ERR_CUDA; }
-  cudaStream_t st = (cudaStream_t)stream;
-  const size_t in_elems = (size_t)s.N * s.IC * s.H * s.W, out_elems = (size_t)s.N * s.OC * s.OH * s.OW;
-  // One buffer: [input NCHW | input NHWC | output NHWC | output NCHW].  It comes from a
-  // grow-only per-device workspace that is kept between calls (tetris_release_workspace frees
-  // it); a call that finds the workspace in use by another thread allocates its own.
-  const size_t need = (2 * in_elems + 2 * out_elems) * sizeof(float);
-  Workspace *ws = f->device < kMaxWsDevices ? &g_workspace[f->device] : nullptr;
-  const bool cached = ws && ws->mutex.try_lock();
-  float *d = nullptr;
-  if (cached) {
-    if (ws->bytes < need) {
-      cudaFree(ws->ptr);
-      ws->ptr = nullptr; ws->bytes = 0;
-      if (cudaMalloc(&ws->ptr, need) == cudaSuccess) ws->bytes = need;
-    }
-    d = static_cast<float *>(ws->ptr);
-  } else if (cudaMalloc(&d, need) != cudaSuccess) {
-    d = nullptr;
-  }
-  if (!d) {
-    cudaGetLastError();
-    if (cached) ws->mutex.unlock();
-    set_error("cudaMalloc of %zu bytes of activations failed", need);
-    return TETRIS_ERR_NOMEM;
-  }
-  float *d_in_nchw = d, *d_in_nhwc = d + in_elems, *d_out_nhwc = d + 2 * in_elems,
-        *d_out_nchw = d + 2 * in_elems + out_elems;
-  auto done = [&](int code) {
-    if (cached) ws->mutex.unlock(); else cudaFree(d);
-    return code;
-  };
-  if (cudaMemcpyAsync(d_in_nchw, h_input_nchw, in_elems * sizeof(float), cudaMemcpyHostToDevice, st) != cudaSuccess) {
-    set_error("host-to-device copy failed: %s", cudaGetErrorString(cudaGetLastError()));
-    return done(TETRIS_ERR_CUDA);
-  }
-  if ((rc = launch_nchw_to_nhwc(d_in_nchw, d_in_nhwc, s.N, s.IC, s.H, s.W, st))) return done(rc);
-  if ((rc = dispatch(f, d_in_nhwc, d_out_nhwc, s, st, TETRIS_VARIANT_AUTO))) return done(rc);
-  if ((rc = launch_nhwc_to_nchw(d_out_nhwc, d_out_nchw, s.N, s.OC, s.OH, s.OW, st))) return done(rc);
-  if (cudaMemcpyAsync(h_output_nchw, d_out_nchw, out_elems * sizeof(float), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess) {
-    set_error("convolution or device-to-host copy failed: %s", cudaGetErrorString(cudaGetLastError()));
-    return done(TETRIS_ERR_CUDA);
-  }
-  return done(TETRIS_OK);
-}
-
-// ---- pipelined host-pointer path: `slot` selects one of kSlots (stream, workspace) pairs per
-//      device, so the upload of one call overlaps the download of the previous one ----
-namespace {
-constexpr int kSlots = 4;
-struct HostSlot {
-  std::mutex mutex;
-  cudaStream_t stream = nullptr;
-  void *ptr = nullptr;
-  size_t bytes = 0;
-};
-HostSlot g_slots[kMaxWsDevices][kSlots];
-}  // namespace
-
-int tetris_conv2d_host_async(const tetris_filter_t *f, const float *h_input_nchw,
-                             float *h_output_nchw, int batch_size, int img_h, int img_w, int stride,
-                             int padding, int slot) {
-  ConvShape s;
-  int rc = make_shape(f, batch_size, img_h, img_w, stride, padding, &s);
-  if (rc) return rc;
-  if (slot < 0 || slot >= kSlots || f->device >= kMaxWsDevices) {
-    set_error("slot %d outside [0, %d)", slot, kSlots);
-    return TETRIS_ERR_INVALID;
-  }
-  if (batch_size == 0) return TETRIS_OK;
-  if (!h_input_nchw || !h_output_nchw) { set_error("input or output pointer is NULL"); return TETRIS_ERR_INVALID; }
-  DeviceGuard guard(f->device);
-  if (!guard.ok) { set_error("cudaSetDevice(%d) failed", f->device); return TETRIS_ERR_CUDA; }
-  HostSlot &hs = g_slots[f->device][slot];
-  std::lock_guard<std::mutex> lock(hs.mutex);
-  if (!hs.stream) TETRIS_CUDA_TRY(cudaStreamCreateWithFlags(&hs.stream, cudaStreamNonBlocking));
-  const size_t in_elems = (size_t)s.N * s.IC * s.H * s.W, out_elems = (size_t)s.N * s.OC * s.OH * s.OW;
-  const size_t need = (2 * in_elems + 2 * out_elems) * sizeof(float);
-  if (hs.bytes < need) {
-    // the slot's earlier work may still read the old buffer
-    TETRIS_CUDA_TRY(cudaStreamSynchronize(hs.stream));
-    cudaFree(hs.ptr);
-    hs.ptr = nullptr; hs.bytes = 0;
-    if (cudaMalloc(&hs.ptr, need) != cudaSuccess) {
-      cudaGetLastError();
-      set_error("cudaMalloc of %zu bytes of activations failed", need);
-      return TETRIS_ERR_NOMEM;
-    }
-    hs.bytes = need;
-  }
-  float *d = static_cast<float *>(hs.ptr);
-  float *d_in_nchw = d, *d_in_nhwc = d + in_elems, *d_out_nhwc = d + 2 * in_elems,
-        *d_out_nchw = d + 2 * in_elems + out_elems;
-  cudaStream_t st = hs.stream;
-  TETRIS_CUDA_TRY(cudaMemcpyAsync(d_in_nchw, h_input_nchw, in_elems * sizeof(float), cudaMemcpyHostToDevice, st));
-  if ((rc = launch_nchw_to_nhwc(d_in_nchw, d_in_nhwc, s.N, s.IC, s.H, s.W, st))) return rc;
-  if ((rc = dispatch(f, d_in_nhwc, d_out_nhwc, s, st, TETRIS_VARIANT_AUTO))) return rc;
-  if ((rc = launch_nhwc_to_nchw(d_out_nhwc, d_out_nchw, s.N, s.OC, s.OH, s.OW, st))) return rc;
-  TETRIS_CUDA_TRY(cudaMemcpyAsync(h_output_nchw, d_out_nchw, out_elems * sizeof(float), cudaMemcpyDeviceToHost, st));
-  return TETRIS_OK;
-}
-
-int tetris_host_sync(int device, int slot) {
-  if (device < 0 || device >= kMaxWsDevices || slot >= kSlots) { set_error("bad device/slot"); return TETRIS_ERR_INVALID; }
-  DeviceGuard guard(device);
-  for (int i = 0; i < kSlots; ++i) {
-    if (slot >= 0 && i != slot) continue;
-    HostSlot &hs = g_slots[device][i];
-    std::lock_guard<std::mutex> lock(hs.mutex);
-    if (hs.stream && cudaStreamSynchronize(hs.stream) != cudaSuccess) {
-      set_error("pipelined convolution failed: %s", cudaGetErrorString(cudaGetLastError()));
-      return TETRIS_ERR_CUDA;
-    }
-  }
-  return TETRIS_OK;
-}
-
-void tetris_release_workspace(void) {
-  int prev = -1;
-  cudaGetDevice(&prev);
-  for (int dev = 0; dev < kMaxWsDevices; ++dev) {
-    Workspace &ws = g_workspace[dev];
-    std::lock_guard<std::mutex> lock(ws.mutex);
-    if (!ws.ptr) continue;
-    if (cudaSetDevice(dev) == cudaSuccess) cudaFree(ws.ptr);
-    ws.ptr = nullptr;
-    ws.bytes = 0;
-  }
-  for (int dev = 0; dev < kMaxWsDevices; ++dev)
-    for (int i = 0; i < kSlots; ++i) {
-      HostSlot &hs = g_slots[dev][i];
-      std::lock_guard<std::mutex> lock(hs.mutex);
-      if (!hs.stream && !hs.ptr) continue;
-      if (cudaSetDevice(dev) != cudaSuccess) continue;
-      if (hs.stream) { cudaStreamSynchronize(hs.stream); cudaStreamDestroy(hs.stream); }
-      cudaFree(hs.ptr);
-      hs.stream = nullptr; hs.ptr = nullptr; hs.bytes = 0;
-    }
-  if (prev >= 0) cudaSetDevice(prev);
 }
 
 int tetris_batch_slice(int batch_size, int world, int rank, int *begin, int *count) {

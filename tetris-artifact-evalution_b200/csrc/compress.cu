@@ -66,18 +66,27 @@ count_kernel(const float *__restrict__ filt, int IC, int OC, int KS, int K, int 
   }
 }
 
-// Exclusive scan of n ints by one block; offsets[n] = total.
+// Exclusive scan of n ints by one block, eight per thread; offsets[n] = total.  meta, if not null:
+// {total, largest}.
 __global__ void __launch_bounds__(1024)
-scan_kernel(const int32_t *__restrict__ lens, int32_t *__restrict__ offsets, int n) {
-  __shared__ int warp_sums[32];
+scan_kernel(const int32_t *__restrict__ lens, int32_t *__restrict__ offsets, int n, int32_t *__restrict__ meta) {
+  constexpr int kEach = 8;
+  __shared__ int warp_sums[32], warp_max[32];
   __shared__ int carry;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int longest = 0;
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
-  for (int base = 0; base < n; base += 1024) {
-    const int i = base + threadIdx.x;
-    const int v = i < n ? lens[i] : 0;
-    int x = v;
+  for (int base = 0; base < n; base += 1024 * kEach) {
+    const int i0 = base + threadIdx.x * kEach;
+    int v[kEach], sum = 0;
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+      v[j] = i0 + j < n ? lens[i0 + j] : 0;
+      sum += v[j];
+      longest = max(longest, v[j]);
+    }
+    int x = sum;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, d);
@@ -95,13 +104,26 @@ scan_kernel(const int32_t *__restrict__ lens, int32_t *__restrict__ offsets, int
       warp_sums[lane] = w;
     }
     __syncthreads();
-    const int before = carry + (warp > 0 ? warp_sums[warp - 1] : 0) + x - v;
-    if (i < n) offsets[i] = before;
+    int before = carry + (warp > 0 ? warp_sums[warp - 1] : 0) + x - sum;
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+      if (i0 + j < n) offsets[i0 + j] = before;
+      before += v[j];
+    }
     __syncthreads();
-    if (threadIdx.x == 1023) carry = before + v;
+    if (threadIdx.x == 1023) carry = before;
     __syncthreads();
   }
-  if (threadIdx.x == 0) offsets[n] = carry;
+  for (int d = 16; d; d >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, d));
+  if (lane == 0) warp_max[warp] = longest;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    offsets[n] = carry;
+    if (meta) {
+      for (int i = 1; i < 32; ++i) longest = max(longest, warp_max[i]);
+      meta[0] = carry; meta[1] = longest;
+    }
+  }
 }
 
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
@@ -233,36 +255,20 @@ int list_fill(const float *d_filter, int IC, int OC, int KS, int K, int TIC, int
   return TETRIS_OK;
 }
 
-size_t compress_scratch_bytes(int n_programs) {
-  // program lengths, then one 64-bit nonzero counter (8-byte aligned)
-  return ((size_t)n_programs * sizeof(int32_t) + 7) / 8 * 8 + sizeof(unsigned long long);
-}
-
-static unsigned long long *nnz_slot(int32_t *d_scratch, int n_programs) {
-  return reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(d_scratch) +
-                                                ((size_t)n_programs * sizeof(int32_t) + 7) / 8 * 8);
-}
-
-// lens -> d_scratch[0..n), nnz -> the counter behind them; offsets -> d_offsets[0..n].
 int compress_count(const float *d_filter, int IC, int OC, int KS, int K, int TIC, int B, int T,
-                   int32_t *d_scratch, cudaStream_t st) {
+                   int32_t *d_lens, unsigned long long *d_nnz, cudaStream_t st) {
   const int P = B * T;
-  unsigned long long *d_nnz = nnz_slot(d_scratch, P);
   TETRIS_CUDA_TRY(cudaMemsetAsync(d_nnz, 0, sizeof(unsigned long long), st));
   count_kernel<<<(P + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, 0, st>>>(
-      d_filter, IC, OC, KS, K, TIC, B, T, d_scratch, d_nnz);
+      d_filter, IC, OC, KS, K, TIC, B, T, d_lens, d_nnz);
   TETRIS_CUDA_TRY(cudaGetLastError());
   return TETRIS_OK;
 }
 
-int compress_scan(const int32_t *d_scratch, int32_t *d_offsets, int n_programs, cudaStream_t st) {
-  scan_kernel<<<1, 1024, 0, st>>>(d_scratch, d_offsets, n_programs);
+int compress_scan(const int32_t *d_lens, int32_t *d_offsets, int n, int32_t *meta, cudaStream_t st) {
+  scan_kernel<<<1, 1024, 0, st>>>(d_lens, d_offsets, n, meta);
   TETRIS_CUDA_TRY(cudaGetLastError());
   return TETRIS_OK;
-}
-
-const unsigned long long *compress_nnz_ptr(const int32_t *d_scratch, int n_programs) {
-  return nnz_slot(const_cast<int32_t *>(d_scratch), n_programs);
 }
 
 int compress_fill(const float *d_filter, int IC, int OC, int KS, int K, int TIC, int B, int T,

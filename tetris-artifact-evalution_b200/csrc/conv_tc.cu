@@ -117,7 +117,7 @@ struct TcParams {
   int ksplit;                  // work items per tile: each takes n_chunks / ksplit chunks and adds its result in
   int relu;                    // max(y, 0) at the store (never together with a split K range)
   int *error_flag;
-  const float *w_tiles;        // weight tile images, see tc_weight_tiles_kernel
+  const float *w_tiles;        // weight tile images, see weights.cu and tc_folded_tiles_kernel
   int tma_store;               // the summing warps hand their staged blocks to TMA stores (see the epilogue)
   unsigned spin_limit;         // polls after which a barrier wait gives up (0: kSpinLimit)
   int withhold_first_load;     // failure-detection test only: every CTA leaves out its first activation load
@@ -734,32 +734,18 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
 }
 
-// Dense OIHW -> the images the weight loader copies: for every (32-channel chunk, tap, channel
-// tile) a block {w_hi, w_lo} of BN rows x 128 bytes each, rows = output channels, already in the
-// 128-byte-swizzled order the tensor core reads (16-byte chunk j of row r sits at chunk
-// j ^ (r & 7)), so that one contiguous bulk copy fills a stage.  Channels past IC or OC are zero.
-__global__ void tc_weight_tiles_kernel(const float *__restrict__ filt, float *__restrict__ tiles,
-                                       int OC, int IC, int KS, int n_chunks, int oc_tiles, int BN, int folded) {
-  const long long total = (long long)(folded ? 1 : KS * KS) * n_chunks * oc_tiles * 2 * BN * KC;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int col = (int)(i % KC);
-    const int row = (int)((i / KC) % BN);
-    const int half = (int)((i / ((long long)KC * BN)) % 2);
-    long long tile = i / ((long long)2 * KC * BN);
-    const int oct = (int)(tile % oc_tiles); tile /= oc_tiles;
-    const int k = (((col >> 2) ^ (row & 7)) << 2) | (col & 3);
-    const int oc = oct * BN + row;
-    float w = 0.f;
-    if (folded) {  // K index = (filter row, filter column, channel), cut into chunks of 32
-      const int kk = (int)tile * KC + k;
-      const int tap = kk / IC, ic = kk - tap * IC;
-      if (tap < KS * KS && oc < OC) w = filt[((size_t)oc * IC + ic) * KS * KS + tap];
-    } else {
-      const int tap = (int)(tile % (KS * KS));  // K steps run chunk-major, tap-minor
-      const int chunk = (int)(tile / (KS * KS));
-      const int ic = chunk * KC + k;
-      if (ic < IC && oc < OC) w = filt[((size_t)oc * IC + ic) * KS * KS + tap];
-    }
+// Folded stems: K index = (filter row, filter column, channel), cut into chunks of 32; for every
+// (chunk, channel tile) a block {w_hi, w_lo} of BN rows x 128 bytes each, rows = output channels, in
+// the 128-byte-swizzled order the tensor core reads (16-byte piece j of row r at piece j ^ (r & 7)).
+__global__ void tc_folded_tiles_kernel(const float *__restrict__ filt, float *__restrict__ tiles,
+                                       int OC, int IC, int KS, int n_chunks, int oc_tiles, int BN) {
+  const int total = n_chunks * oc_tiles * 2 * BN * KC;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int col = i % KC, row = (i / KC) % BN, half = (i / (KC * BN)) % 2, tile = i / (2 * KC * BN);
+    const int oct = tile % oc_tiles, chunk = tile / oc_tiles;
+    const int kk = chunk * KC + ((((col >> 2) ^ (row & 7)) << 2) | (col & 3));
+    const int oc = oct * BN + row, tap = kk / IC, ic = kk - tap * IC;
+    const float w = tap < KS * KS && oc < OC ? filt[((size_t)oc * IC + ic) * KS * KS + tap] : 0.f;
     const float h = __uint_as_float(round_tf32(w));
     tiles[i] = half ? __uint_as_float(round_tf32(w - h)) : h;
   }
@@ -793,7 +779,7 @@ int encode_map(CUtensorMap *map, void *ptr, int rank, const cuuint64_t *dims, co
 
 struct TcState {
   float *d_tiles = nullptr;  // weight tile images
-  int *d_error = nullptr;
+  int *d_error = nullptr;      // (behind the tiles)
   int n_chunks = 0, bn = 128;  // K chunks per tap; channel tile (fixed by the filter: 64 up to 64 channels)
   bool folded = false;         // <= 4 input channels: taps and channels folded into one K axis
   // Launch set-ups (tensor map of the input, tile plan, grid), one per (input pointer, conv
@@ -819,14 +805,14 @@ struct TcState {
 void conv_tc_state_delete(void *state) {
   TcState *s = static_cast<TcState *>(state);
   if (!s) return;
-  cudaFree(s->d_tiles); cudaFree(s->d_error);
+  device_free(s->d_tiles);
   delete s;
 }
 
-// Builds the dense split weights and their tensor maps (called from filter creation, d_dense is
-// the OIHW filter on the device).  Failure here is not fatal for the filter: the variant is then
-// reported as unsupported.
-int conv_tc_prepare(tetris_filter *f, const float *d_dense) {
+// Makes room for the split weight images (called from filter creation and from the file loader;
+// d_dense is the OIHW filter on the device) and builds a folded stem's.  Failure here is not fatal
+// for the filter: the variant is then reported as unsupported.
+int conv_tc_prepare(tetris_filter *f, const float *d_dense, WeightImages *w) {
   const bool folded = f->in_channel <= 4;
   if (f->groups != 1 || (!folded && (f->in_channel & 3) != 0)) return TETRIS_OK;  // not covered: leave tc_state null
   TcState *s = new (std::nothrow) TcState();
@@ -837,17 +823,23 @@ int conv_tc_prepare(tetris_filter *f, const float *d_dense) {
   s->bn = f->out_channel <= 64 ? 64 : 128;
   const int oc_tiles = (f->out_channel + s->bn - 1) / s->bn;
   const size_t elems = (size_t)(folded ? 1 : taps) * s->n_chunks * oc_tiles * 2 * s->bn * KC;
-  if (cudaMalloc(&s->d_tiles, elems * 4) != cudaSuccess || cudaMalloc(&s->d_error, sizeof(int)) != cudaSuccess) {
+  if (device_alloc((void **)&s->d_tiles, elems * 4 + sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     conv_tc_state_delete(s);
     return TETRIS_OK;
   }
-  cudaMemset(s->d_error, 0, sizeof(int));
-  tc_weight_tiles_kernel<<<(unsigned)std::min<size_t>((elems + 255) / 256, 4096), 256>>>(
-      d_dense, s->d_tiles, f->out_channel, f->in_channel, KS, s->n_chunks, oc_tiles, s->bn, folded ? 1 : 0);
-  if (cudaGetLastError() != cudaSuccess) {
-    conv_tc_state_delete(s);
-    return TETRIS_OK;
+  s->d_error = reinterpret_cast<int *>(s->d_tiles + elems);
+  cudaMemsetAsync(s->d_error, 0, sizeof(int), 0);
+  if (folded) {
+    tc_folded_tiles_kernel<<<(unsigned)std::min<size_t>((elems + 255) / 256, 4096), 256>>>(
+        d_dense, s->d_tiles, f->out_channel, f->in_channel, KS, s->n_chunks, oc_tiles, s->bn);
+    if (cudaGetLastError() != cudaSuccess) {
+      conv_tc_state_delete(s);
+      return TETRIS_OK;
+    }
+  } else {
+    w->tc = s->d_tiles;
+    w->bn = s->bn;
   }
   f->tc_state = s;
   return TETRIS_OK;

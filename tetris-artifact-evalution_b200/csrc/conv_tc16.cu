@@ -852,34 +852,6 @@ __global__ void tc16_scales_kernel(const float *__restrict__ w, int per_oc, floa
   }
 }
 
-// Dense OIHW -> the images the weight loader copies, one per (channel tile, 32-channel chunk, tap),
-// in the swizzled order the tensor core reads.  Plain: 128 rows of 128 bytes, row = output channel
-// = {w_hi[32], w_lo[32]} FP16 of w * scale[oc], 16-byte piece j of row r at piece j ^ (r & 7).
-// Stacked (at most 64 channels): 128 rows of 64 bytes, rows 0..63 w_hi and 64..127 w_lo of channel
-// r & 63, piece j at piece j ^ ((r >> 1) & 3).  Channels past IC or OC are zero.
-__global__ void tc16_weight_tiles_kernel(const float *__restrict__ filt, __half *__restrict__ tiles,
-                                         int OC, int IC, int KS, int n_chunks, int oc_tiles, int stack, const float *__restrict__ scale) {
-  const int cols = stack ? 32 : 64;
-  const long long total = (long long)KS * KS * n_chunks * oc_tiles * BM * cols;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int col = (int)(i % cols);               // FP16 position inside the stored row
-    const int row = (int)((i / cols) % BM);
-    long long tile = i / ((long long)cols * BM);
-    const int tap = (int)(tile % (KS * KS));
-    tile /= KS * KS;
-    const int chunk = (int)(tile % n_chunks);
-    const int oct = (int)(tile / n_chunks);
-    const int piece = (col >> 3) ^ (stack ? (row >> 1) & 3 : row & 7);  // logical 16-byte piece stored at this position
-    const int k = ((piece & 3) << 3) | (col & 7);  // channel inside the chunk
-    const bool is_lo = stack ? row >= 64 : piece >= 4;
-    const int oc = stack ? row & 63 : oct * BM + row, ic = chunk * KC + k;
-    float w = 0.f;
-    if (ic < IC && oc < OC) w = filt[((size_t)oc * IC + ic) * KS * KS + tap] * scale[oc];
-    const __half h = __float2half_rn(w);
-    tiles[i] = is_lo ? __float2half_rn(w - __half2float(h)) : h;
-  }
-}
-
 typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                              const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1074,14 +1046,14 @@ int launch_instance(const CUtensorMap &map_x, const CUtensorMap &map_out, const 
 void conv_tc16_state_delete(void *state) {
   Tc16State *s = static_cast<Tc16State *>(state);
   if (!s) return;
-  cudaFree(s->d_tiles); cudaFree(s->d_error); cudaFree(s->d_out_scale);
+  device_free(s->d_tiles);
   delete s;
 }
 
-// Builds the split FP16 weight images (called from filter creation and from the file loader;
-// d_dense is the OIHW filter on the device).  Failure here is not fatal for the filter: the
-// variant is then reported as unsupported.
-int conv_tc16_prepare(tetris_filter *f, const float *d_dense) {
+// Makes room for the split FP16 weight images and works out the scales (called from filter creation
+// and from the file loader; d_dense is the OIHW filter on the device).  Failure here is not fatal
+// for the filter: the variant is then reported as unsupported.
+int conv_tc16_prepare(tetris_filter *f, const float *d_dense, WeightImages *w) {
   if (f->groups != 1 || (f->in_channel & 3) != 0 || f->in_channel < 8 || f->kernel_size > 7) return TETRIS_OK;
   Tc16State *s = new (std::nothrow) Tc16State();
   if (!s) return TETRIS_OK;
@@ -1089,30 +1061,28 @@ int conv_tc16_prepare(tetris_filter *f, const float *d_dense) {
   s->n_chunks = (f->in_channel + KC - 1) / KC;
   s->stack = f->out_channel <= 64;
   s->oc_tiles = (f->out_channel + BM - 1) / BM;
-  const size_t elems = (size_t)taps * s->n_chunks * s->oc_tiles * BM * (s->stack ? 32 : 64);
+  const size_t tile_bytes = (size_t)taps * s->n_chunks * s->oc_tiles * BM * (s->stack ? 64 : 128);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) s->sms = 0;
-  float *d_w_scale = nullptr;
-  if (s->sms < 1 || cudaMalloc(&s->d_tiles, elems * sizeof(__half)) != cudaSuccess || cudaMalloc(&s->d_error, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&d_w_scale, f->out_channel * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&s->d_out_scale, f->out_channel * sizeof(float)) != cudaSuccess) {
+  // one buffer: images, scales of the outputs and of the weights, error flag
+  if (s->sms < 1 || device_alloc((void **)&s->d_tiles, tile_bytes + 2 * f->out_channel * sizeof(float) + sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(d_w_scale);
     conv_tc16_state_delete(s);
     return TETRIS_OK;
   }
-  cudaMemset(s->d_error, 0, sizeof(int));
+  s->d_out_scale = reinterpret_cast<float *>(reinterpret_cast<char *>(s->d_tiles) + tile_bytes);
+  float *d_w_scale = s->d_out_scale + f->out_channel;
+  s->d_error = reinterpret_cast<int *>(d_w_scale + f->out_channel);
+  cudaMemsetAsync(s->d_error, 0, sizeof(int), 0);
   // per-channel scales: every output channel's largest |w| lands in [2^12, 2^13)
   tc16_scales_kernel<<<f->out_channel, 256>>>(d_dense, f->in_channel * taps, d_w_scale, s->d_out_scale);
-  tc16_weight_tiles_kernel<<<(unsigned)std::min<size_t>((elems + 255) / 256, 4096), 256>>>(
-      d_dense, s->d_tiles, f->out_channel, f->in_channel, KS, s->n_chunks, s->oc_tiles, s->stack ? 1 : 0, d_w_scale);
-  const cudaError_t err = cudaGetLastError();
-  cudaStreamSynchronize(0);  // (d_w_scale is freed next)
-  cudaFree(d_w_scale);
-  if (err != cudaSuccess) {
+  if (cudaGetLastError() != cudaSuccess) {
     conv_tc16_state_delete(s);
     return TETRIS_OK;
   }
+  w->tc16 = s->d_tiles;
+  w->stack = s->stack ? 1 : 0;
+  w->scale = d_w_scale;
   f->tc16_state = s;
   return TETRIS_OK;
 }

@@ -50,14 +50,35 @@ struct ConvShape {
   int relu = 0;  // fused epilogue: max(y, 0) at the store (tetris_conv2d_launch_fused)
 };
 
-// compress.cu: dense filter on the device -> program stream.  `d_scratch` holds
-// n_programs + 1 ints (program lengths, then their exclusive scan) and one 64-bit
-// nonzero counter after them.
-size_t compress_scratch_bytes(int n_programs);
+// Makes `device` current for the lifetime of the object and restores the previous one.
+struct DeviceGuard {
+  int prev = -1;
+  bool ok = false;
+  explicit DeviceGuard(int device) {
+    if (cudaGetDevice(&prev) != cudaSuccess) return;
+    ok = cudaSetDevice(device) == cudaSuccess;
+  }
+  ~DeviceGuard() {
+    if (prev >= 0) cudaSetDevice(prev);
+  }
+};
+
+// api.cu: checks the arguments of a conv call and fills in the shape
+int make_shape(const tetris_filter *f, int batch, int h, int w, int stride, int padding, ConvShape *s);
+
+// memory.cu: device memory of the filters, copies with ordinary host memory
+cudaError_t device_alloc(void **p, size_t bytes);
+void device_free(void *p);
+cudaError_t copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t st);
+cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st);
+void release_memory();
+
+// compress.cu: dense filter on the device -> program stream.  The count kernel writes the length of
+// every program and adds the nonzeros to *d_nnz.
 int compress_count(const float *d_filter, int IC, int OC, int KS, int K, int TIC, int B, int T,
-                   int32_t *d_scratch, cudaStream_t st);
-int compress_scan(const int32_t *d_scratch, int32_t *d_offsets, int n_programs, cudaStream_t st);
-const unsigned long long *compress_nnz_ptr(const int32_t *d_scratch, int n_programs);
+                   int32_t *d_lens, unsigned long long *d_nnz, cudaStream_t st);
+// Exclusive scan of n lengths into n + 1 offsets; `meta` (may be null) receives {total, longest}.
+int compress_scan(const int32_t *d_lens, int32_t *d_offsets, int n, int32_t *meta, cudaStream_t st);
 int compress_fill(const float *d_filter, int IC, int OC, int KS, int K, int TIC, int B, int T,
                   const int32_t *d_offsets, uint64_t *d_ops, int64_t n_ops, cudaStream_t st);
 
@@ -88,13 +109,23 @@ void count_launch();
 // out every CTA's first activation load, with the poll limit their barrier waits then use.
 int test_injection(unsigned *spin_limit);
 void tiled_plan_cache_delete(void *cache);
-int conv_tc_prepare(tetris_filter *f, const float *d_dense);
+// weights.cu: the tensor-core kernels' weight images of a filter, where they cover it
+struct WeightImages {
+  float *tc = nullptr;            // split TF32
+  int bn = 128;                   // ... channels of its tiles
+  void *tc16 = nullptr;           // split FP16
+  int stack = 0;                  // ... w_hi and w_lo stacked (at most 64 output channels)
+  const float *scale = nullptr;   // ... per output channel
+};
+int tensor_prepare(tetris_filter *f, const float *d_dense);
+// the variants' shares of it: buffers, scales, folded stems; what is left to build goes into `w`
+int conv_tc_prepare(tetris_filter *f, const float *d_dense, WeightImages *w);
 void conv_tc_state_delete(void *state);
 bool conv_tc_supported(const tetris_filter *f, const ConvShape &s);
 int launch_conv_tc(const tetris_filter *f, const float *in, float *out, const ConvShape &s,
                    cudaStream_t st);
 int conv_tc_check_error(const tetris_filter *f);
-int conv_tc16_prepare(tetris_filter *f, const float *d_dense);
+int conv_tc16_prepare(tetris_filter *f, const float *d_dense, WeightImages *w);
 void conv_tc16_state_delete(void *state);
 bool conv_tc16_supported(const tetris_filter *f, const ConvShape &s);
 double conv_tc16_cost(const tetris_filter *f, const ConvShape &s);  // estimated clocks of a launch, negative: not covered

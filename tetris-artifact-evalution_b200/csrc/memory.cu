@@ -1,0 +1,323 @@
+// Device memory of the filters and copies between the device and ordinary host memory.
+//
+// Filters take their device memory from one stream-ordered pool per device: a cudaMalloc costs
+// 10-100 us and a cudaFree waits for the device, and a filter has a dozen buffers (512 x 512 x 3 x 3:
+// 5 ms to create, most of it in the allocator).  Up to 256 MB of freed memory stay with the pool;
+// tetris_release_workspace gives them back.
+//
+// Ordinary (pageable) host memory.  A copy between it and the device runs through the driver's own
+// bounce buffer on the calling thread, at the speed of one core's memcpy (15 GB/s on a host whose
+// link carries 55): 210 us for 3.2 MB each way, against 58 us of DMA.  Here a few threads move chunks
+// between the caller's array and a page-locked ring while the copy engine moves the chunks before
+// them, so that the link sets the pace.  Page-locked arrays are copied from and to directly.
+#include <string.h>
+
+#include <algorithm>
+#include <atomic>
+#include <condition_variable>
+#include <mutex>
+#include <new>
+#include <thread>
+#include <vector>
+
+#include "internal.h"
+
+namespace tetris {
+namespace {
+
+constexpr int kMaxDevices = 64;
+constexpr uint64_t kKeptBytes = (uint64_t)256 << 20;
+
+struct DevicePool {
+  std::mutex mutex;
+  cudaMemPool_t pool = nullptr;
+};
+DevicePool g_pools[kMaxDevices];
+
+// ---- chunked copies through page-locked memory -------------------------------------------------
+constexpr int kRing = 32;                          // chunks in flight per direction
+constexpr size_t kMaxChunk = (size_t)512 << 10, kMinChunk = (size_t)64 << 10;
+constexpr size_t kStagedBytes = (size_t)256 << 10;  // smaller copies are left to the driver
+
+struct Job {
+  char *user;                     // the caller's array
+  char *ring;                     // page-locked chunks
+  size_t bytes, chunk;
+  int n;                          // chunks
+  bool to_ring;
+  std::atomic<int> next{0};       // first chunk nobody has taken
+  std::atomic<int> ready{0};      // chunks below this may be taken
+  std::atomic<unsigned char> *done;
+  std::atomic<int> users{0};      // threads that hold a pointer to this job
+
+  // Takes and moves one chunk; false if none may be taken now.
+  bool work() {
+    int i = next.load(std::memory_order_relaxed);
+    do {
+      if (i >= n || i >= ready.load(std::memory_order_acquire)) return false;
+    } while (!next.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
+    char *u = user + (size_t)i * chunk, *r = ring + (size_t)(i % kRing) * kMaxChunk;
+    const size_t len = std::min(chunk, bytes - (size_t)i * chunk);
+    if (to_ring) memcpy(r, u, len); else memcpy(u, r, len);
+    done[i].store(1, std::memory_order_release);
+    return true;
+  }
+};
+
+inline void relax() {
+#if defined(__x86_64__)
+  __builtin_ia32_pause();
+#endif
+}
+
+// One per device, made at the first staged copy and never destroyed (its threads may outlive static
+// destructors); release() gives the threads and the memory back.
+class Stager {
+ public:
+  std::mutex in_use;              // one staged copy at a time; others go through the driver
+
+  bool open() {
+    if (ring_in_) return true;
+    if (cudaHostAlloc((void **)&ring_in_, 2 * kRing * kMaxChunk, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      ring_in_ = nullptr;
+      return false;
+    }
+    ring_out_ = ring_in_ + kRing * kMaxChunk;
+    for (int i = 0; i < kRing; ++i)
+      if (cudaEventCreateWithFlags(&events_[i], cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        release();
+        return false;
+      }
+    if (cudaEventCreateWithFlags(&uploaded_, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); release(); return false; }
+    // four cores move as much as the link carries; the caller is one more
+    const int n = (int)std::min(4u, std::max(1u, std::thread::hardware_concurrency() / 3));
+    stop_ = false;
+    try {
+      for (int i = 0; i < n; ++i) threads_.emplace_back([this] { serve(); });
+    } catch (...) {  // (the caller then moves the chunks alone)
+    }
+    return true;
+  }
+
+  void release() {
+    { std::lock_guard<std::mutex> lock(mutex_); stop_ = true; }
+    wake_.notify_all();
+    for (std::thread &t : threads_) t.join();
+    threads_.clear();
+    if (uploaded_) { cudaEventSynchronize(uploaded_); cudaEventDestroy(uploaded_); uploaded_ = nullptr; }
+    for (cudaEvent_t &e : events_) { if (e) cudaEventDestroy(e); e = nullptr; }
+    cudaFreeHost(ring_in_);
+    ring_in_ = ring_out_ = nullptr;
+  }
+
+  // The caller's array -> device; when this returns the array may be reused, the last copies out of
+  // the ring may still be under way on `st`.
+  cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    cudaEventSynchronize(uploaded_);  // (the last upload has left the ring)
+    Job job;
+    prepare(&job, static_cast<char *>(const_cast<void *>(src)), ring_in_, bytes, true);
+    job.ready.store(std::min(job.n, kRing), std::memory_order_release);
+    post(&job);
+    cudaError_t err = cudaSuccess;
+    for (int sent = 0, back = 0; sent < job.n && err == cudaSuccess;) {
+      if (job.done[sent].load(std::memory_order_acquire)) {
+        const size_t at = (size_t)sent * job.chunk;
+        err = cudaMemcpyAsync(static_cast<char *>(dst) + at, job.ring + (size_t)(sent % kRing) * kMaxChunk,
+                              std::min(job.chunk, bytes - at), cudaMemcpyHostToDevice, st);
+        if (err == cudaSuccess && job.n > kRing) err = cudaEventRecord(events_[sent % kRing], st);
+        ++sent;
+      } else if (back < sent && back + kRing < job.n && cudaEventQuery(events_[back % kRing]) == cudaSuccess) {
+        job.ready.store(std::min(job.n, ++back + kRing), std::memory_order_release);  // that chunk of the ring is free again
+      } else if (!job.work()) {
+        relax();
+      }
+    }
+    finish(&job);
+    const cudaError_t marked = cudaEventRecord(uploaded_, st);
+    return err == cudaSuccess ? marked : err;
+  }
+
+  // Device -> the caller's array, behind what `st` holds; complete when this returns.
+  cudaError_t download(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    Job job;
+    prepare(&job, static_cast<char *>(dst), ring_out_, bytes, false);
+    cudaError_t err = cudaSuccess;
+    int sent = 0, landed = 0;
+    auto send = [&]() {
+      const size_t at = (size_t)sent * job.chunk;
+      err = cudaMemcpyAsync(job.ring + (size_t)(sent % kRing) * kMaxChunk, static_cast<const char *>(src) + at,
+                            std::min(job.chunk, bytes - at), cudaMemcpyDeviceToHost, st);
+      if (err == cudaSuccess) err = cudaEventRecord(events_[sent % kRing], st);
+      ++sent;
+    };
+    while (sent < std::min(job.n, kRing) && err == cudaSuccess) send();
+    post(&job);
+    for (int moved = 0; moved < job.n && err == cudaSuccess;) {
+      if (job.done[moved].load(std::memory_order_acquire)) {
+        if (sent < job.n && sent - moved <= kRing) send();  // (chunk `moved` of the ring is free again)
+        ++moved;
+      } else if (landed < sent) {
+        const cudaError_t q = cudaEventQuery(events_[landed % kRing]);
+        if (q == cudaSuccess) job.ready.store(++landed, std::memory_order_release);
+        else if (q != cudaErrorNotReady) err = q;
+        else if (!job.work()) relax();
+      } else if (!job.work()) {
+        relax();
+      }
+    }
+    finish(&job);
+    if (err != cudaSuccess) cudaStreamSynchronize(st);  // (copies into the ring may be under way)
+    return err;
+  }
+
+ private:
+  void prepare(Job *job, char *user, char *ring, size_t bytes, bool to_ring) {
+    job->user = user; job->ring = ring; job->bytes = bytes; job->to_ring = to_ring;
+    // eight chunks or more, so that the first copy starts early and the last one is short
+    job->chunk = std::min(kMaxChunk, std::max(kMinChunk, (bytes / 8 + 4095) / 4096 * 4096));
+    job->n = (int)((bytes + job->chunk - 1) / job->chunk);
+    flags_ = std::vector<std::atomic<unsigned char>>(job->n);
+    job->done = flags_.data();
+  }
+  void post(Job *job) {
+    { std::lock_guard<std::mutex> lock(mutex_); job_ = job; }
+    wake_.notify_all();
+  }
+  void finish(Job *job) {  // nobody takes another chunk, and nobody is left inside the job
+    job->next.store(job->n, std::memory_order_relaxed);
+    { std::lock_guard<std::mutex> lock(mutex_); job_ = nullptr; }
+    while (job->users.load(std::memory_order_acquire)) relax();
+  }
+  void serve() {
+    std::unique_lock<std::mutex> lock(mutex_);
+    for (;;) {
+      wake_.wait(lock, [this] { return stop_ || (job_ && job_->next.load(std::memory_order_relaxed) < job_->n); });
+      if (stop_) return;
+      Job *job = job_;
+      job->users.fetch_add(1, std::memory_order_relaxed);
+      lock.unlock();
+      for (int idle = 0; job->next.load(std::memory_order_relaxed) < job->n;) {
+        if (job->work()) { idle = 0; continue; }
+        if (++idle > 2000) std::this_thread::yield(); else relax();  // (waiting for the device)
+      }
+      job->users.fetch_sub(1, std::memory_order_release);
+      lock.lock();
+    }
+  }
+
+  std::mutex mutex_;
+  std::condition_variable wake_;
+  Job *job_ = nullptr;
+  bool stop_ = false;
+  std::vector<std::thread> threads_;
+  std::vector<std::atomic<unsigned char>> flags_;
+  char *ring_in_ = nullptr, *ring_out_ = nullptr;
+  cudaEvent_t events_[kRing] = {}, uploaded_ = nullptr;
+};
+
+std::mutex g_stagers_mutex;
+Stager *g_stagers[kMaxDevices];
+
+Stager *stager_of(int device) {
+  if (device >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> lock(g_stagers_mutex);
+  if (!g_stagers[device]) g_stagers[device] = new (std::nothrow) Stager();
+  return g_stagers[device];
+}
+
+bool pageable(const void *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return true; }
+  return a.type == cudaMemoryTypeUnregistered;
+}
+
+// Whether a copy of `bytes` with this host array goes through the ring; the stager then is in use.
+Stager *take_stager(const void *host, size_t bytes) {
+  int dev = 0;
+  if (bytes < kStagedBytes || !pageable(host) || cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  Stager *s = stager_of(dev);
+  if (!s || !s->in_use.try_lock()) return nullptr;
+  if (s->open()) return s;
+  s->in_use.unlock();
+  return nullptr;
+}
+
+}  // namespace
+
+// `bytes` from the pool of the current device, ready on every stream.
+cudaError_t device_alloc(void **p, size_t bytes) {
+  *p = nullptr;
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  if (dev >= kMaxDevices) return cudaMalloc(p, bytes);
+  DevicePool &dp = g_pools[dev];
+  {
+    std::lock_guard<std::mutex> lock(dp.mutex);
+    if (!dp.pool) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      if ((err = cudaMemPoolCreate(&dp.pool, &props)) != cudaSuccess) { dp.pool = nullptr; return err; }
+      uint64_t keep = kKeptBytes;
+      cudaMemPoolSetAttribute(dp.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+  }
+  // (allocated, used and freed in the order of the default stream; other streams see a filter only
+  // once its creation has been waited for)
+  return cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), dp.pool, 0);
+}
+
+// Nothing on the device may still use `p` (tetris_filter_destroy waits for the device).
+void device_free(void *p) {
+  if (p) cudaFreeAsync(p, 0);
+}
+
+// Host -> device in the order of `st`; `src` may be reused when this returns (unless it is
+// page-locked: then once `st` has passed).
+cudaError_t copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+  Stager *s = take_stager(src, bytes);
+  if (!s) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  const cudaError_t err = s->upload(dst, src, bytes, st);
+  s->in_use.unlock();
+  return err;
+}
+
+// Device -> host behind what `st` holds; complete when this returns.
+cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+  Stager *s = take_stager(dst, bytes);
+  if (s) {
+    const cudaError_t err = s->download(dst, src, bytes, st);
+    s->in_use.unlock();
+    return err;
+  }
+  const cudaError_t err = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+  return err == cudaSuccess ? cudaStreamSynchronize(st) : err;
+}
+
+// Gives back the rings, their threads and what the pools keep.
+void release_memory() {
+  int prev = -1;
+  cudaGetDevice(&prev);
+  {
+    std::lock_guard<std::mutex> lock(g_stagers_mutex);
+    for (int dev = 0; dev < kMaxDevices; ++dev) {
+      if (!g_stagers[dev]) continue;
+      std::lock_guard<std::mutex> use(g_stagers[dev]->in_use);
+      if (cudaSetDevice(dev) == cudaSuccess) g_stagers[dev]->release();
+    }
+  }
+  for (int dev = 0; dev < kMaxDevices; ++dev) {
+    std::lock_guard<std::mutex> lock(g_pools[dev].mutex);
+    if (g_pools[dev].pool && cudaSetDevice(dev) == cudaSuccess) {
+      cudaDeviceSynchronize();
+      cudaMemPoolTrimTo(g_pools[dev].pool, 0);
+    }
+  }
+  if (prev >= 0) cudaSetDevice(prev);
+}
+
+}  // namespace tetris

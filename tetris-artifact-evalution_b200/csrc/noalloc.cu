@@ -99,5 +99,5 @@ extern "C" int tetris_list_offsets_noalloc(const float *d_filter_oihw, int in_ch
   if ((rc = list_count(d_filter_oihw, in_channel, out_channel, kernel_size, oc_block, tile_ic, B, T,
                        d_counts, st)))
     return rc;
-  return compress_scan(d_counts, d_list_offsets, (int)pieces, st);
+  return compress_scan(d_counts, d_list_offsets, (int)pieces, nullptr, st);
 }

@@ -172,7 +172,7 @@ int tetris_filter_save(const tetris_filter_t *f, const char *path) {
   unsigned char *w = payload.data();
   cudaError_t err = cudaSuccess;
   auto pull = [&](const void *src, size_t n) {
-    if (n && err == cudaSuccess) err = cudaMemcpy(w, src, n, cudaMemcpyDeviceToHost);
+    if (n && err == cudaSuccess) err = copy_to_host(w, src, n, 0);
     w += n;
   };
   pull(f->d_list_offsets, ob); pull(f->d_prog_offsets, ob); pull(f->d_lists, lb); pull(f->d_ops, pb); pull(f->d_dense, db);
@@ -231,15 +231,15 @@ int tetris_filter_load(const char *path, int device, tetris_filter_t **out) {
   const unsigned char *r = payload.data();
   float *d_dense = nullptr;
   auto fail = [&](int code) {
-    cudaFree(d_dense);
+    device_free(d_dense);
     tetris_filter_destroy(f);
     cudaSetDevice(prev);
     return code;
   };
   cudaError_t err = cudaSuccess;
   auto push = [&](void **dst, size_t n) {
-    if (n && err == cudaSuccess) err = cudaMalloc(dst, n);
-    if (n && err == cudaSuccess) err = cudaMemcpy(*dst, r, n, cudaMemcpyHostToDevice);
+    if (n && err == cudaSuccess) err = device_alloc(dst, n);
+    if (n && err == cudaSuccess) err = copy_to_device(*dst, r, n, 0);
     r += n;
   };
   push((void **)&f->d_list_offsets, ob); push((void **)&f->d_prog_offsets, ob);
@@ -252,23 +252,27 @@ int tetris_filter_load(const char *path, int device, tetris_filter_t **out) {
   if (f->groups == 1) {
     // the tensor-core tile images: back to dense on the device, then as at creation
     const size_t dense_bytes = (size_t)f->out_channel * f->in_channel * f->kernel_size * f->kernel_size * sizeof(float);
-    if (cudaMalloc(&d_dense, dense_bytes) != cudaSuccess) {
+    if (device_alloc((void **)&d_dense, dense_bytes) != cudaSuccess) {
       cudaGetLastError();
-      set_error("cudaMalloc of %zu bytes for the dense filter failed", dense_bytes);
+      set_error("allocation of %zu bytes for the dense filter failed", dense_bytes);
       return fail(TETRIS_ERR_NOMEM);
     }
-    cudaMemset(d_dense, 0, dense_bytes);
+    cudaMemsetAsync(d_dense, 0, dense_bytes, 0);
     const int P = f->n_oc_blocks * f->n_stages;
     lists_to_dense_kernel<<<(P + 7) / 8, 256>>>(f->d_lists, f->d_list_offsets, d_dense, f->in_channel, f->out_channel,
                                                  f->kernel_size, f->oc_block, f->tile_ic, f->n_oc_blocks, f->n_stages);
-    if ((rc = conv_tc_prepare(f, d_dense)) || (rc = conv_tc16_prepare(f, d_dense))) return fail(rc);
+    if ((rc = tensor_prepare(f, d_dense))) return fail(rc);
     if (cudaDeviceSynchronize() != cudaSuccess) {
       set_error("rebuilding the tensor-core tile images failed: %s", cudaGetErrorString(cudaGetLastError()));
       return fail(TETRIS_ERR_CUDA);
     }
-    cudaFree(d_dense);
+    device_free(d_dense);
     d_dense = nullptr;
     if (tb) tiled_plans_import(f, reinterpret_cast<const int32_t *>(r), h.n_tuned);
+  }
+  if (cudaDeviceSynchronize() != cudaSuccess) {
+    set_error("upload of the compressed filter failed: %s", cudaGetErrorString(cudaGetLastError()));
+    return fail(TETRIS_ERR_CUDA);
   }
   cudaSetDevice(prev);
   *out = f;
