@@ -16,7 +16,9 @@ namespace tetris {
 namespace {
 
 // y = max(y, 0) in place (for kernels whose store does not rectify itself)
-__global__ void __launch_bounds__(256) relu_kernel(float *__restrict__ y, size_t n4, size_t n) {
+__global__ void __launch_bounds__(256) relu_kernel(float *y, size_t n4, size_t n) {
+  grid_release();
+  y = grid_wait(y);
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n4) {
     float4 v = reinterpret_cast<float4 *>(y)[i];
@@ -29,8 +31,17 @@ __global__ void __launch_bounds__(256) relu_kernel(float *__restrict__ y, size_t
 
 // 2x2 max-pooling, stride 2, NHWC; odd trailing rows / columns are dropped (floor), as the
 // networks' own pooling layers do.
+// T: float4 where the channel count allows it (C then counts quads; a thread per channel spent
+// more on its three 64-bit divisions than on its four loads), else float.
+__device__ __forceinline__ float max2(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ float4 max2(const float4 &a, const float4 &b) {
+  return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w));
+}
+template <typename T>
 __global__ void __launch_bounds__(256)
-pool2x2_kernel(const float *__restrict__ in, float *__restrict__ out, int N, int H, int W, int C) {
+pool2x2_kernel(const T *in, T *__restrict__ out, int N, int H, int W, int C) {
+  grid_release();
+  in = grid_wait(in);
   const int OH = H / 2, OW = W / 2;
   const size_t total = (size_t)N * OH * OW * C;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -40,9 +51,9 @@ pool2x2_kernel(const float *__restrict__ in, float *__restrict__ out, int N, int
   const int ow = (int)(r % OW); r /= OW;
   const int oh = (int)(r % OH);
   const int n = (int)(r / OH);
-  const float *p = in + (((size_t)n * H + 2 * oh) * W + 2 * ow) * C + c;
+  const T *p = in + (((size_t)n * H + 2 * oh) * W + 2 * ow) * C + c;
   const size_t row = (size_t)W * C;
-  out[i] = fmaxf(fmaxf(p[0], p[C]), fmaxf(p[row], p[row + C]));
+  out[i] = max2(max2(p[0], p[C]), max2(p[row], p[row + C]));
 }
 
 }  // namespace
@@ -52,8 +63,7 @@ int launch_relu_inplace(float *y, size_t n, cudaStream_t st) {
   const bool vec = (reinterpret_cast<uintptr_t>(y) & 15) == 0;
   const size_t n4 = vec ? n / 4 : 0;
   const size_t threads = n4 ? n4 : 1;
-  relu_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(y, n4, n);
-  TETRIS_CUDA_TRY(cudaGetLastError());
+  TETRIS_CUDA_TRY(launch_overlapped(relu_kernel, dim3((unsigned)((threads + 255) / 256)), 256, 0, st, 1, y, n4, n));
   return TETRIS_OK;
 }
 
@@ -189,9 +199,14 @@ int tetris_chain_run(tetris_chain_t *c, const float *d_input_nhwc, void *stream)
     if (rc) return rc;
     x = c->conv_out[i];
     if (c->pool_out[i]) {
-      const size_t total = (size_t)s.N * (s.OH / 2) * (s.OW / 2) * s.OC;
-      pool2x2_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(x, c->pool_out[i], s.N, s.OH, s.OW, s.OC);
-      TETRIS_CUDA_TRY(cudaGetLastError());
+      const bool vec = (s.OC & 3) == 0;  // (the chain's own buffers are aligned)
+      const size_t total = (size_t)s.N * (s.OH / 2) * (s.OW / 2) * s.OC / (vec ? 4 : 1);
+      const dim3 blocks((unsigned)((total + 255) / 256));
+      if (vec)
+        TETRIS_CUDA_TRY(launch_overlapped(pool2x2_kernel<float4>, blocks, 256, 0, st, 1, reinterpret_cast<const float4 *>(x),
+                                          reinterpret_cast<float4 *>(c->pool_out[i]), s.N, s.OH, s.OW, s.OC / 4));
+      else
+        TETRIS_CUDA_TRY(launch_overlapped(pool2x2_kernel<float>, blocks, 256, 0, st, 1, x, c->pool_out[i], s.N, s.OH, s.OW, s.OC));
       x = c->pool_out[i];
     }
   }

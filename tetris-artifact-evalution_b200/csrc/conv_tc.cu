@@ -258,6 +258,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  if (tid == 0) grid_release();
+  if (warp != 2) grid_wait();  // (warp 2 sends for weights first)
 
   // Persistent CTA: tiles blockIdx.x, blockIdx.x + gridDim.x, ...; the channel tile is the
   // fastest index, so CTAs that run side by side read the same activation patch.
@@ -344,6 +346,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         decode(t, w0, h0, n0, oc0, chunk0);
         for (int it = 0; it < iters; ++it, ++g) {
           const int s = g % p.w_stages;
+          if (g == p.w_stages) grid_wait();  // (the bounded waits below must not run while earlier launches do)
           if (g >= p.w_stages && !(ok = wait_group(group_of(g - p.w_stages)))) break;
           // K step `it` of channel tile oc0 / BN: one contiguous {w_hi, w_lo} image
           const float *src = p.w_tiles + ((size_t)(chunk0 * taps + it) * oc_tiles + oc0 / BN) * (2 * BN * KC);
@@ -502,7 +505,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
               const uint32_t fr = (k * rcp_row) >> 16, rem = k - fr * (uint32_t)fold_row;
               const int ih = f_ih0 + (int)fr, iw = f_iw0 + (int)((rem * rcp_ic) >> 16);
               const bool inside = f_live && (int)k < fold_k && ih >= 0 && ih < p.H && iw >= 0 && iw < p.W;
-              hi[c] = inside ? __float_as_uint(__ldg(f_img + ((long long)ih * p.W + f_iw0) * p.IC + (int)rem)) : 0u;
+              hi[c] = inside ? __float_as_uint(f_img[((long long)ih * p.W + f_iw0) * p.IC + (int)rem]) : 0u;
             }
           } else {
           if (p.per_tap || seen_u != u) {  // a patch is waited for once, at the first tap this warp reads
@@ -983,10 +986,9 @@ int launch_conv_tc(const tetris_filter *f, const float *in, float *out, const Co
   if (p.ksplit > 1)  // the work items add into the output
     TETRIS_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)s.N * s.OH * s.OW * s.OC * sizeof(float), st));
   if (bn == 64)
-    conv_tc_kernel<64><<<grid, kThreads, smem, st>>>(map_x, map_out, p);
+    TETRIS_CUDA_TRY(launch_overlapped(conv_tc_kernel<64>, grid, kThreads, smem, st, 1, map_x, map_out, p));
   else
-    conv_tc_kernel<128><<<grid, kThreads, smem, st>>>(map_x, map_out, p);
-  TETRIS_CUDA_TRY(cudaGetLastError());
+    TETRIS_CUDA_TRY(launch_overlapped(conv_tc_kernel<128>, grid, kThreads, smem, st, 1, map_x, map_out, p));
   count_launch();
   if (p.relu) note_relu_fused();
   return TETRIS_OK;

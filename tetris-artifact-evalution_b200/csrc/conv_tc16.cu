@@ -279,6 +279,8 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  if (tid == 0) grid_release();  // (this CTA has its tensor memory: nothing it waits for can be held by the next launch)
+  if (warp != 0) grid_wait();    // (warp 0 sends for weights first)
 
   // Work items: tile blockIdx.x / d, + gridDim.x / d, ... (d > 1: exactly one).  The channel tile
   // is the fastest index, so CTAs that run side by side read the same activation patch.
@@ -343,6 +345,37 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         const __half *wsrc = p.w_tiles + (size_t)(wt - quot(wt, p.by_oc_tiles) * p.oc_tiles) * p.n_chunks * taps * (kWBytes / 2);
         uint32_t idle = 0;
         const uint32_t limit = (uint32_t)abort_flag[1];
+        auto load_weights = [&]() {  // the next K step's image
+          mbar_expect_tx(bar_wfull(sw), (uint32_t)kWBytes);
+          bulk_load(smem_u32(wbase + (size_t)sw * kWBytes), wsrc + ((size_t)wc * taps + wr * p.KS + wq) * (kWBytes / 2), (uint32_t)kWBytes, bar_wfull(sw));
+          ++w_loads;
+          if (++sw == p.n_w) { sw = 0; pw ^= 1u; }
+          if ((wq += p.S) >= p.KS) {
+            if ((wr += p.S) >= p.KS) {
+              if (++wpq == phases) {
+                wpq = 0;
+                if (++wpr == phases) {
+                  wpr = 0;
+                  if (++wc == chunk1) {
+                    wc = chunk0;
+                    if (++wb == bands) {
+                      wb = 0;
+                      wt += tile_step;
+                      w_left = wt < p.total_tiles;
+                      wsrc = p.w_tiles + (size_t)(wt - quot(wt, p.by_oc_tiles) * p.oc_tiles) * p.n_chunks * taps * (kWBytes / 2);
+                    }
+                  }
+                }
+              }
+              wr = wpr;
+            }
+            wq = wpq;
+          }
+        };
+        if (first && w_loads == 0) {  // the ring is empty: filled while the launch before this one drains
+          while (w_left && w_loads < p.n_w) load_weights();
+          grid_wait();
+        }
         while (x_left || w_left) {
           bool moved = false;
           if (x_left && mbar_test(bar_xempty(sx), px ^ 1u)) {
@@ -376,31 +409,7 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           }
           if (w_left && mbar_test(bar_wempty(sw), pw ^ 1u)) {
             moved = true;
-            mbar_expect_tx(bar_wfull(sw), (uint32_t)kWBytes);
-            bulk_load(smem_u32(wbase + (size_t)sw * kWBytes), wsrc + ((size_t)wc * taps + wr * p.KS + wq) * (kWBytes / 2), (uint32_t)kWBytes, bar_wfull(sw));
-            ++w_loads;
-            if (++sw == p.n_w) { sw = 0; pw ^= 1u; }
-            if ((wq += p.S) >= p.KS) {
-              if ((wr += p.S) >= p.KS) {
-                if (++wpq == phases) {
-                  wpq = 0;
-                  if (++wpr == phases) {
-                    wpr = 0;
-                    if (++wc == chunk1) {
-                      wc = chunk0;
-                      if (++wb == bands) {
-                        wb = 0;
-                        wt += tile_step;
-                        w_left = wt < p.total_tiles;
-                        wsrc = p.w_tiles + (size_t)(wt - quot(wt, p.by_oc_tiles) * p.oc_tiles) * p.n_chunks * taps * (kWBytes / 2);
-                      }
-                    }
-                  }
-                }
-                wr = wpr;
-              }
-              wq = wpq;
-            }
+            load_weights();
           }
           if (moved) { idle = 0; continue; }
           if ((++idle & 31) == 0) {
@@ -568,7 +577,6 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       float *give = reinterpret_cast<float *>(exch) + kSumWarps * 1024 + me * 1024;  // stacked tiles
       const float *take = reinterpret_cast<const float *>(exch) + kSumWarps * 1024 + (me ^ 2) * 1024;
       int nblk = 0;
-      const bool vec = (p.OC & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;  // 16-byte stores
       const float unscale = banded ? pow2f(4 - band_exp(0)) : 1.f;
       for (int t = tile0; t < p.total_tiles; t += tile_step) {
         int oc0, w0, h0, n0;
@@ -931,7 +939,9 @@ bool finish_geometry(const Tc16State &t, const ConvShape &s, Geometry *g) {
     if (g->n_w < kWStagesMax && fits(g->n_x, g->n_w + 1)) { ++g->n_w; grew = true; }
     if (g->n_x < x_want && fits(g->n_x + 1, g->n_w)) { ++g->n_x; grew = true; }
   }
-  g->smem = fixed + (size_t)g->n_x * g->x_stage + g->n_w * wb;
+  // (more than half of an SM's: the CTAs of a launch that is placed while another one drains must
+  // not be doubled up on the SMs that are free first)
+  g->smem = std::max(fixed + (size_t)g->n_x * g->x_stage + g->n_w * wb, (size_t)116 * 1024);
   if (g->d > 1 && (size_t)g->npx * BM * 4 > (size_t)g->n_x * g->x_stage + g->n_w * wb) return false;  // (the sums of a slice)
   // clocks per K step: the MMAs themselves, the shared-memory pipe (MMA operands, weight copy,
   // patch landing, read and written by the conversion), the conversion, the issuing warp
@@ -1028,16 +1038,7 @@ int launch_instance(const CUtensorMap &map_x, const CUtensorMap &map_out, const 
     TETRIS_CUDA_TRY(cudaFuncSetAttribute(conv_tc16_kernel<NMAX, STACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
     if (dev < 16) configured[dev] = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(Roles<NMAX>::kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)p.d; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = p.d > 1 ? 1 : 0;
-  TETRIS_CUDA_TRY(cudaLaunchKernelEx(&cfg, conv_tc16_kernel<NMAX, STACK>, map_x, map_out, p));
+  TETRIS_CUDA_TRY(launch_overlapped(conv_tc16_kernel<NMAX, STACK>, dim3(grid), Roles<NMAX>::kThreads, smem, st, (unsigned)p.d, map_x, map_out, p));
   return TETRIS_OK;
 }
 

@@ -184,6 +184,8 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) conv_tiled_kernel(const Tile
     sts_u1(smem0 + p.stage_bytes + p.TIC * p.ICP + i, 0u);
   }
 
+  grid_release();
+  grid_wait();
   issue_stage(0, 0);
 #pragma unroll 1
   for (int t = 0; t < p.T; ++t) {
@@ -461,8 +463,7 @@ int launch_instance(const Plan &plan, const float *in, float *out, cudaStream_t 
   TiledParams p = plan.p;
   p.in = in;
   p.out = out;
-  kern<<<plan.grid, WARPS * 32, plan.smem_bytes, st>>>(p);
-  TETRIS_CUDA_TRY(cudaGetLastError());
+  TETRIS_CUDA_TRY(launch_overlapped(kern, plan.grid, WARPS * 32, plan.smem_bytes, st, 1, p));
   count_launch();
   return TETRIS_OK;
 }

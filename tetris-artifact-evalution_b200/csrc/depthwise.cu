@@ -33,7 +33,7 @@ struct DwGrid { int cq, wtiles, htiles, qb, aw, ah, qblocks, xblocks, yblocks; }
 // whose three taps cover it, so an input value is loaded once per thread, not once per output row.
 template <int S, int TW, int RH>
 __global__ void __launch_bounds__(256)
-depthwise3x3_kernel(const float4 *__restrict__ in, float4 *__restrict__ out,
+depthwise3x3_kernel(const float4 *in, float4 *__restrict__ out,
                     const float *__restrict__ filt, ConvShape s, DwGrid g) {
   const int cq = g.cq;
   const int ql = threadIdx.x & (g.qb - 1), pos = threadIdx.x / g.qb;
@@ -62,7 +62,8 @@ depthwise3x3_kernel(const float4 *__restrict__ in, float4 *__restrict__ out,
   constexpr int NCOL = (TW - 1) * S + 3;  // input columns this thread touches per row
   constexpr int NROW = (RH - 1) * S + 3;  // input rows of its window
   const int iw0 = ow0 * S - s.P, ih0 = oh0 * S - s.P;
-  const float4 *img = in + (size_t)n * s.H * s.W * cq + q;
+  grid_release();
+  const float4 *img = grid_wait(in) + (size_t)n * s.H * s.W * cq + q;
   // Taps are added in (r, s) order per output, the order of the CPU loop nest
   // (Tetris/tensor_utils.cc:152-153): window row i serves output row a with filter row r = i - a*S,
   // and i ascends.
@@ -74,7 +75,7 @@ depthwise3x3_kernel(const float4 *__restrict__ in, float4 *__restrict__ out,
 #pragma unroll
     for (int c = 0; c < NCOL; ++c) {
       const int iw = iw0 + c;
-      x[c] = (iw >= 0 && iw < s.W) ? __ldg(&img[((size_t)ih * s.W + iw) * cq])
+      x[c] = (iw >= 0 && iw < s.W) ? img[((size_t)ih * s.W + iw) * cq]
                                    : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
@@ -114,6 +115,7 @@ depthwise3x3_kernel(const float4 *__restrict__ in, float4 *__restrict__ out,
 // three 16-byte loads per input row, each input row feeding up to three output rows.  Taps are
 // added in (r, s) order per output, as above.
 constexpr uint32_t kDwSpinLimit = 1u << 22;
+constexpr size_t kDwMinSmem = (size_t)77 * 1024;
 __device__ int g_dw_error;  // a bounded wait of the pipeline gave up (read and cleared by tetris_filter_check)
 
 struct DwTmaParams {
@@ -160,6 +162,8 @@ depthwise3x3_tma_kernel(const __grid_constant__ CUtensorMap map, const DwTmaPara
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  grid_release();
+  grid_wait();
   const int per_cg = p.tiles_x * p.tiles_y * p.N;
   auto issue = [&](int t, int s) {
     const int cg = t / per_cg;
@@ -321,19 +325,19 @@ int launch_depthwise_tma(const tetris_filter *f, const float *in, float *out, co
   if (total > 0x7FFFFFFFll / 8) return 1;
   p.total = (int)total;
   p.relu = s.relu;
-  const size_t smem = (size_t)nst * bx * by * 128 + 128;
+  // (at least a third of an SM's: a launch that is placed while another one drains must not put
+  // more than two CTAs on the SMs that are free first)
+  const size_t smem = std::max((size_t)nst * bx * by * 128 + 128, kDwMinSmem);
   static thread_local bool configured[16] = {false};
   if (dev >= 16 || !configured[dev]) {
     TETRIS_CUDA_TRY(cudaFuncSetAttribute(depthwise3x3_tma_kernel<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 18 * 10 * 128 + 128));
-    TETRIS_CUDA_TRY(cudaFuncSetAttribute(depthwise3x3_tma_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 10 * 10 * 128 + 128));
+    TETRIS_CUDA_TRY(cudaFuncSetAttribute(depthwise3x3_tma_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwMinSmem));
     TETRIS_CUDA_TRY(cudaFuncSetAttribute(depthwise3x3_tma_kernel<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 17 * 17 * 128 + 128));
     if (dev < 16) configured[dev] = true;
   }
   const unsigned grid = (unsigned)std::min<long long>(total, 2ll * sms);
-  if (s.S == 1 && two == 16) depthwise3x3_tma_kernel<1, 16><<<grid, 256, smem, st>>>(e->map, p);
-  else if (s.S == 1) depthwise3x3_tma_kernel<1, 8><<<grid, 256, smem, st>>>(e->map, p);
-  else depthwise3x3_tma_kernel<2, 8><<<grid, 256, smem, st>>>(e->map, p);
-  TETRIS_CUDA_TRY(cudaGetLastError());
+  auto kernel = s.S == 2 ? depthwise3x3_tma_kernel<2, 8> : two == 16 ? depthwise3x3_tma_kernel<1, 16> : depthwise3x3_tma_kernel<1, 8>;
+  TETRIS_CUDA_TRY(launch_overlapped(kernel, dim3(grid), 256, smem, st, 1, e->map, p));
   return 0;
 }
 
@@ -383,14 +387,9 @@ int launch_depthwise(const tetris_filter *f, const float *in, float *out, const 
     g.xblocks = (wtiles + g.aw - 1) / g.aw;
     g.yblocks = (htiles + g.ah - 1) / g.ah;
     const unsigned blocks = (unsigned)((long long)g.qblocks * g.xblocks * g.yblocks * s.N);
-    if (s.S == 1 && RH == 2)
-      depthwise3x3_kernel<1, TW, 2><<<blocks, 256, 0, st>>>(in4, out4, f->d_dense, s, g);
-    else if (s.S == 1)
-      depthwise3x3_kernel<1, TW, 1><<<blocks, 256, 0, st>>>(in4, out4, f->d_dense, s, g);
-    else if (RH == 2)
-      depthwise3x3_kernel<2, TW, 2><<<blocks, 256, 0, st>>>(in4, out4, f->d_dense, s, g);
-    else
-      depthwise3x3_kernel<2, TW, 1><<<blocks, 256, 0, st>>>(in4, out4, f->d_dense, s, g);
+    auto kernel = s.S == 1 ? (RH == 2 ? depthwise3x3_kernel<1, TW, 2> : depthwise3x3_kernel<1, TW, 1>)
+                           : (RH == 2 ? depthwise3x3_kernel<2, TW, 2> : depthwise3x3_kernel<2, TW, 1>);
+    TETRIS_CUDA_TRY(launch_overlapped(kernel, dim3(blocks), 256, 0, st, 1, in4, out4, f->d_dense, s, g));
   } else {
     depthwise_any_kernel<<<(unsigned)((elems + 255) / 256), 256, 0, st>>>(in, out, f->d_dense, s);
   }

@@ -45,6 +45,42 @@ void set_error(const char *fmt, ...);
     }                                                                                      \
   } while (0)
 
+// Overlapped launches.  A kernel that follows another on its stream may be set up -- its blocks
+// placed, barriers and tensor memory made ready, weights on their way -- while the one before it
+// drains: launch_overlapped marks the launch as such, grid_release in a running kernel lets the next
+// one start being placed, and grid_wait returns once everything before it on the stream is complete
+// and visible.  EVERY kernel launched this way calls grid_wait before it touches activations (reads
+// or writes them), in at least one thread of every block on whose data all stores of that block depend:
+// completion then passes on from launch to launch, and a kernel launched in the ordinary way, a
+// copy or an event still sees all work before it.  What is read ahead of it is what no launch on a
+// stream writes: a filter's images, complete when its creation returned.
+// Activations are not read through the non-coherent path (__ldg) in these kernels: they may change
+// while the kernel is resident.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// (the pointer passes through the wait, so that no load through it is moved ahead)
+template <typename T> __device__ __forceinline__ T *grid_wait(T *p) {
+  asm volatile("griddepcontrol.wait;" : "+l"(p) :: "memory");
+  return p;
+}
+// Blocks of a persistent kernel call it once they hold what they need to finish (tensor memory).
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, unsigned cluster, const A &...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 struct ConvShape {
   int N, H, W, IC, OC, KS, S, P, OH, OW;
   int relu = 0;  // fused epilogue: max(y, 0) at the store (tetris_conv2d_launch_fused)

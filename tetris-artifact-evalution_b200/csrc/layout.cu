@@ -32,10 +32,12 @@ __device__ __forceinline__ Tile tile_of(unsigned b, unsigned ctiles, unsigned pt
 // [C][P] -> [P][C] per image.  VEC: 32-channel tiles, C a multiple of 4 and dst 16-byte aligned.
 template <int TC, bool VEC>
 __global__ void __launch_bounds__(kThreads)
-to_channels_last_kernel(const float *__restrict__ src, float *__restrict__ dst, int C, int P, unsigned ctiles, unsigned ptiles) {
+to_channels_last_kernel(const float *src, float *__restrict__ dst, int C, int P, unsigned ctiles, unsigned ptiles) {
   constexpr int TP = Shape<TC>::TP, kPitch = Shape<TC>::pitch;
   __shared__ float tile[TC * kPitch];
   const Tile t = tile_of<TC>(blockIdx.x, ctiles, ptiles, C, P);
+  grid_release();
+  src = grid_wait(src);
   float v[kElems / kThreads];
 #pragma unroll
   for (int i = 0; i < kElems / kThreads; ++i) {
@@ -72,10 +74,12 @@ to_channels_last_kernel(const float *__restrict__ src, float *__restrict__ dst, 
 // [P][C] -> [C][P] per image.  VEC: 32-channel tiles, C a multiple of 4 and src 16-byte aligned.
 template <int TC, bool VEC>
 __global__ void __launch_bounds__(kThreads)
-to_channels_first_kernel(const float *__restrict__ src, float *__restrict__ dst, int C, int P, unsigned ctiles, unsigned ptiles) {
+to_channels_first_kernel(const float *src, float *__restrict__ dst, int C, int P, unsigned ctiles, unsigned ptiles) {
   constexpr int TP = Shape<TC>::TP, kPitch = Shape<TC>::pitch;
   __shared__ float tile[TC * kPitch];
   const Tile t = tile_of<TC>(blockIdx.x, ctiles, ptiles, C, P);
+  grid_release();
+  src = grid_wait(src);
   if (VEC) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = 4 * (lane & 7);
     float4 v[4];
@@ -123,9 +127,8 @@ int launch_tiles(const float *src, float *dst, int N, int C, long long P, bool t
     return TETRIS_ERR_UNSUPPORTED;
   }
   const unsigned b = (unsigned)blocks, ct = (unsigned)ctiles, pt = (unsigned)ptiles;
-  if (to_last) to_channels_last_kernel<TC, VEC><<<b, kThreads, 0, st>>>(src, dst, C, (int)P, ct, pt);
-  else to_channels_first_kernel<TC, VEC><<<b, kThreads, 0, st>>>(src, dst, C, (int)P, ct, pt);
-  TETRIS_CUDA_TRY(cudaGetLastError());
+  TETRIS_CUDA_TRY(launch_overlapped(to_last ? to_channels_last_kernel<TC, VEC> : to_channels_first_kernel<TC, VEC>, dim3(b), kThreads, 0, st, 1,
+                                    src, dst, C, (int)P, ct, pt));
   return TETRIS_OK;
 }
 
