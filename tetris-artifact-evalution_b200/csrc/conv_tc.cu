@@ -59,8 +59,16 @@
 // map's element strides) in a 4-deep ring of 16 KiB stages.
 //
 // With at most 4 input channels (the stems of the networks) taps and channels are folded into
-// one K axis, K = KS*KS*IC in chunks of 32, and the converter warps gather the activations from
-// global memory themselves (TMA needs 16-byte strides; an NHWC pixel of 3 floats has 12).
+// one K axis, K = KS*KS*IC in chunks of 32.  Where an image row is a multiple of 16 bytes the image
+// is a tensor {W * IC, H, N} to TMA, a patch is the rows under a tile (its start rounded down to 16
+// bytes), one load per work item, and the converters pick each pixel's K values from it.  Within a
+// filter row the (column, channel) pairs of a pixel are contiguous, so value k of every lane lies at
+// one and the same offset from its pixel: no index arithmetic or bounds check per lane.  Other images
+// (a width of 225 floats, an input off the 16-byte grid) are gathered from global memory by the
+// converters: 5000 clocks per K step, half of it address arithmetic and half of it the L1 pipe (a
+// load of 32 pixels touches 6 to 12 lines).  (A warp that copied the rows with cp.async instead was
+// slower than that gather: 130 us against 79 on 224x224x3 -> 64, batch 16, 6000 clocks of its own
+// instructions per tile.)
 //
 // No cluster launch: every load is issued by one CTA for itself.  Covers strides 1-8, IC <= 4 or
 // IC % 4 == 0.
@@ -108,8 +116,10 @@ struct TcParams {
   int PW, PH;                  // the tile with its halo: PW = TW + KS - 1, PH = TH + KS - 1
   int per_tap, S;              // per_tap: one strided box per K step instead of a patch per chunk (stride > 1)
   int w_stages;                // weight stages in use: 5, or 4 with the fifth as store staging block
-  int folded;                  // <= 4 input channels: K = (filter row, filter column, channel) folded into
-                               // 32-wide chunks, activations gathered from global memory by the converters
+  int folded;                  // <= 4 input channels: K = (filter row, filter column, channel) folded into 32-wide
+                               // chunks.  1: gathered from global memory by the converters; 2: patches of image
+                               // rows by TMA; then PW is the pitch of a patch row in floats, PH its rows
+  int x_ring;                  // patch stages in use: 2, or 4 of half the size (folded 2, where they suffice)
   const float *in;             // activations (folded mode only)
   int H, W, IC;                // input extent (folded mode only)
   int tiles_w, tiles_h, tiles_n;
@@ -165,6 +175,11 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
 // The same for a whole converged warp, with one answer for all lanes.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag, int lane) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+__device__ __forceinline__ uint32_t lds_u32(const float *p) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
+  return v;
 }
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2, int c3) {
   asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
@@ -297,8 +312,22 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     if (lane == 0) {
       int u = 0;  // loads of this CTA, across tiles
       bool ok = true;
-      if (p.folded) {
+      if (p.folded == 1) {
         // the converters gather the activations themselves
+      } else if (p.folded) {
+        // the image rows under a work item's tile
+        const uint32_t x_box_bytes = (uint32_t)(p.PW * p.PH * p.NB * 4), stage_bytes = (uint32_t)(kXBytes / p.x_ring);
+        for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++u) {
+          int w0, h0, n0, oc0, chunk0;
+          decode(t, w0, h0, n0, oc0, chunk0);
+          const int s = u & (p.x_ring - 1);
+          if (!(ok = mbar_wait(bar_xempty(s), ((u / p.x_ring) & 1) ^ 1, abort_flag))) break;
+          if (u == 0 && p.withhold_first_load) continue;  // (test: this patch never arrives, its readers give up)
+          mbar_expect_tx(bar_xfull(s), x_box_bytes);
+          tma_load_4d(smem_u32(xbase) + (uint32_t)s * stage_bytes, &map_x, bar_xfull(s), ((w0 * p.S - p.P) * p.IC) & ~3, h0 * p.S - p.P, n0, 0);
+        }
+        if (!ok || *abort_flag)
+          for (int v = max(u - p.x_ring, p.withhold_first_load ? 1 : 0); v < u; ++v) mbar_drain(bar_xfull(v & (p.x_ring - 1)), (uint32_t)(v / p.x_ring) & 1u);
       } else if (!p.per_tap) {
         // One patch per 32-channel chunk: the tile plus its halo, shared by all taps.
         const uint32_t x_box_bytes = (uint32_t)(p.PW * p.PH * p.NB * KC * 4);
@@ -466,16 +495,26 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     bool ok = true;
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
       int tap = 0, r = 0, q = 0;
-      // folded mode: input position of this thread's pixel for filter tap (0, 0)
+      // folded mode: this thread's pixel -- its input position for filter tap (0, 0), or its place in the patch
       int f_ih0 = 0, f_iw0 = 0, f_chunk0 = 0;
       const float *f_img = nullptr;
       bool f_live = false;
-      if (p.folded) {
+      if (p.folded) f_chunk0 = cur[0] * item_chunks;
+      if (p.folded == 1) {
         const int n = cur[4] * p.NB + pn, oh = cur[3] * p.TH + ph, ow = cur[2] * p.TW + pw;
-        f_chunk0 = cur[0] * item_chunks;
         f_live = live && n < p.N && oh < p.OH && ow < p.OW;
         f_ih0 = oh * p.S - p.P; f_iw0 = ow * p.S - p.P;
         f_img = p.in + (size_t)(f_live ? n : 0) * p.H * p.W * p.IC;
+      } else if (p.folded) {
+        const int s = u & (p.x_ring - 1);
+        f_img = reinterpret_cast<const float *>(xbase + s * (kXBytes / p.x_ring));
+        // (the patch starts at a multiple of four floats: up to three lie before the tile's first)
+        if (live) f_img += (pn * p.PH + ph * p.S) * p.PW + pw * p.S * p.IC + ((cur[2] * p.TW * p.S - p.P) * p.IC & 3);  // (rows past the tile read somewhere in it)
+        // Every warp waits for every patch, also one whose K steps are all the other set's: it releases
+        // them all, and must not release this stage's next patch before this one is.
+        if (!(ok = mbar_wait_warp(bar_xfull(s), (u / p.x_ring) & 1, abort_flag, lane))) break;
+      }
+      if (p.folded) {
         int carry = 0;
 #pragma unroll
         for (int d = 0; d < 4; ++d) {
@@ -488,24 +527,34 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       for (int it = 0; it < iters; ++it, ++g) {
         const int sa = g % kAStages;
         // activation stage, its phase, and whether this K step is the last to read it
-        const int sx = p.per_tap ? g % kXStages : u & 1;
-        const uint32_t xphase = (uint32_t)(p.per_tap ? g / kXStages : u >> 1) & 1u;
-        const bool last_of_chunk = tap == taps - 1;
+        const int sx = p.per_tap ? g % kXStages : u & (p.x_ring - 1);
+        const uint32_t xphase = (uint32_t)(p.per_tap ? g / kXStages : u >> 1) & 1u;  // (folded items have waited already)
+        const bool last_of_chunk = p.folded == 2 ? it == iters - 1 : tap == taps - 1;  // (folded: a patch serves the whole item)
         if ((g & 1) == set) {
           // Read and split this tap's rows first: everything up to the tensor-memory store can
           // be done while the operand stage is still in use.
           uint32_t hi[32], lo[32];
           if (p.folded) {
-            // K index k = (filter row, filter column, channel): within a filter row the
-            // (column, channel) pairs are contiguous in the NHWC input, so element k of this
-            // pixel is img[(ih0 + row) * W * IC + iw0 * IC + rem] where it exists.
+            // K index k = (filter row, filter column, channel)
+            const int k0 = (f_chunk0 + it) * KC;
+            if (p.folded == 2) {  // k, and with it the offset, is the same for all lanes
+              const int fr = (int)(((uint32_t)k0 * rcp_row) >> 16);
+              int rem = k0 - fr * fold_row, off = fr * p.PW + rem;
 #pragma unroll
-            for (int c = 0; c < 32; ++c) {
-              const uint32_t k = (uint32_t)((f_chunk0 + it) * KC + c);
-              const uint32_t fr = (k * rcp_row) >> 16, rem = k - fr * (uint32_t)fold_row;
-              const int ih = f_ih0 + (int)fr, iw = f_iw0 + (int)((rem * rcp_ic) >> 16);
-              const bool inside = f_live && (int)k < fold_k && ih >= 0 && ih < p.H && iw >= 0 && iw < p.W;
-              hi[c] = inside ? __float_as_uint(f_img[((long long)ih * p.W + f_iw0) * p.IC + (int)rem]) : 0u;
+              for (int c = 0; c < 32; ++c) {
+                hi[c] = k0 + c < fold_k ? lds_u32(f_img + off) : 0u;
+                ++off;
+                if (++rem == fold_row) { rem = 0; off += p.PW - fold_row; }
+              }
+            } else {
+#pragma unroll
+              for (int c = 0; c < 32; ++c) {
+                const uint32_t k = (uint32_t)(k0 + c);
+                const uint32_t fr = (k * rcp_row) >> 16, rem = k - fr * (uint32_t)fold_row;
+                const int ih = f_ih0 + (int)fr, iw = f_iw0 + (int)((rem * rcp_ic) >> 16);
+                const bool inside = f_live && (int)k < fold_k && ih >= 0 && ih < p.H && iw >= 0 && iw < p.W;
+                hi[c] = inside ? __float_as_uint(f_img[((long long)ih * p.W + f_iw0) * p.IC + (int)rem]) : 0u;
+              }
             }
           } else {
           if (p.per_tap || seen_u != u) {  // a patch is waited for once, at the first tap this warp reads
@@ -551,7 +600,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         // waits, produced wrong results on the 56x56 and 112x112 layers.)
         if (last_of_chunk) {
           __syncwarp();
-          if (lane == 0 && !p.per_tap && !p.folded) mbar_arrive(bar_xempty(sx));
+          if (lane == 0 && !p.per_tap && p.folded != 1) mbar_arrive(bar_xempty(sx));
           ++u;
           tap = 0; r = 0; q = 0;
         } else {
@@ -770,11 +819,11 @@ EncodeFn get_encode() {
 }
 
 int encode_map(CUtensorMap *map, void *ptr, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
-               const cuuint32_t *box, const cuuint32_t *estr) {
+               const cuuint32_t *box, const cuuint32_t *estr, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   EncodeFn enc = get_encode();
   if (!enc) { set_error("cuTensorMapEncodeTiled is not available from this driver"); return TETRIS_ERR_UNSUPPORTED; }
   const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, ptr, dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed with code %d", (int)r); return TETRIS_ERR_CUDA; }
   return TETRIS_OK;
@@ -878,36 +927,59 @@ int launch_conv_tc(const tetris_filter *f, const float *in, float *out, const Co
       // pixels of a tile: TW x TH x NB rows, at most 128, as full as possible, and -- at stride
       // 1, where all taps read one patch -- such that the tile with its halo fits a stage
       // (1x1 filters have no halo to share either, and the per-K-step ring is four deep)
-      const bool per_tap = s.S > 1 || s.KS == 1 || t->folded;
+      // folded stems by TMA patches: image rows of a multiple of 16 bytes (and dimensions TMA takes)
+      const bool patches = t->folded && (reinterpret_cast<uintptr_t>(in) & 15) == 0 && (s.W * s.IC & 3) == 0;
+      const bool per_tap = t->folded ? !patches : s.S > 1 || s.KS == 1;
       const int halo = per_tap ? 0 : s.KS - 1;
+      // folded stems: floats of a patch row (at least the three that the start may be rounded down by;
+      // a pitch that continues the lanes' bank sequence in the tile's next row) and bytes of a patch
+      auto fold_pitch = [&](int TW) {
+        const int need = (((TW - 1) * s.S + s.KS) * s.IC + 3 + 3) / 4 * 4;
+        for (int q = need; q < need + 32; q += 4)
+          if (((q - TW * s.IC) & 31) == 0) return q;
+        return need;
+      };
+      auto fits = [&](int TW, int TH, int NB) {
+        if (patches) {
+          const int pitch = fold_pitch(TW), rows = (TH - 1) * s.S + s.KS;
+          return pitch <= 256 && rows <= 256 && pitch * rows * NB * 4 <= kPatchBytes;
+        }
+        return (TW + halo) * (TH + halo) * NB <= kPatchRows;
+      };
       int best_tw = 0, best_th = 1, best_nb = 1;
       double best = -1.0;
       bool best_boxy = false;
       for (int TW = 1; TW <= std::min(s.OW, 128); ++TW) {
         int TH = std::min(s.OH, 128 / TW);
-        while (TH > 1 && (TW + halo) * (TH + halo) > kPatchRows) --TH;
-        if (TH < 1 || (TW + halo) * (TH + halo) > kPatchRows || (!t->folded && (TW * s.S > 256 || TH * s.S > 256))) continue;
+        while (TH > 1 && !fits(TW, TH, 1)) --TH;
+        if (TH < 1 || !fits(TW, TH, 1) || (!t->folded && (TW * s.S > 256 || TH * s.S > 256))) continue;
         int NB = (TH == s.OH && TW == s.OW) ? std::min(s.N, 128 / (TW * TH)) : 1;
-        while (NB > 1 && (TW + halo) * (TH + halo) * NB > kPatchRows) --NB;
+        while (NB > 1 && !fits(TW, TH, NB)) --NB;
         const double tiles = (double)((s.OW + TW - 1) / TW) * ((s.OH + TH - 1) / TH) * ((s.N + NB - 1) / NB);
         const double eff = (double)s.N * s.OH * s.OW / (tiles * 128.0);
         // (among equally full tiles, one whose rows fill a warp's 32 lanes: see tma_store below)
         // (a tile shorter than 128 rows qualifies when it spans the image's height: the rows past
         // its end then lie below the image and the store drops them)
         const bool boxy = NB == 1 && 32 % TW == 0 && (TW * TH == 128 || TH == s.OH);
-        if (eff > best + 1e-9 || (eff > best - 1e-9 && boxy && !best_boxy)) { best = eff; best_tw = TW; best_th = TH; best_nb = NB; best_boxy = boxy; }
+        if (eff > best + 1e-9 || (eff > best - 1e-9 && boxy && (!best_boxy || (patches && TW <= 16)))) { best = std::max(best, eff); best_tw = TW; best_th = TH; best_nb = NB; best_boxy = boxy; }
       }
       if (best_tw == 0) {
         set_error("tensor-core variant: no tile of this layer fits an activation stage");
         return TETRIS_ERR_UNSUPPORTED;
       }
-      const int PW = best_tw + halo, PH = best_th + halo;
+      const int PW = patches ? fold_pitch(best_tw) : best_tw + halo, PH = patches ? (best_th - 1) * s.S + s.KS : best_th + halo;
       const cuuint64_t dims[4] = {(cuuint64_t)s.IC, (cuuint64_t)s.W, (cuuint64_t)s.H, (cuuint64_t)s.N};
       const cuuint64_t strides[3] = {(cuuint64_t)s.IC * 4, (cuuint64_t)s.IC * 4 * s.W, (cuuint64_t)s.IC * 4 * s.W * s.H};
       // with element strides the box spans S times the pixels it loads
       const cuuint32_t box[4] = {KC, (cuuint32_t)(PW * s.S), (cuuint32_t)(PH * s.S), (cuuint32_t)best_nb};
       const cuuint32_t estr[4] = {1, (cuuint32_t)s.S, (cuuint32_t)s.S, 1};
-      if (!t->folded) {  // (folded mode reads the activations with plain loads)
+      if (patches) {  // the images as rows of W * IC floats
+        const cuuint64_t row = (cuuint64_t)s.W * s.IC, fdims[4] = {row, (cuuint64_t)s.H, (cuuint64_t)s.N, 1};
+        const cuuint64_t fstrides[3] = {row * 4, row * 4 * s.H, row * 4 * s.H * s.N};
+        const cuuint32_t fbox[4] = {(cuuint32_t)PW, (cuuint32_t)PH, (cuuint32_t)best_nb, 1}, fone[4] = {1, 1, 1, 1};
+        const int rc = encode_map(&su->map_x, const_cast<float *>(in), 4, fdims, fstrides, fbox, fone, CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (rc) return rc;
+      } else if (!t->folded) {  // (the converters' gather uses plain loads)
         const int rc = encode_map(&su->map_x, const_cast<float *>(in), 4, dims, strides, box, estr);
         if (rc) return rc;
       }
@@ -915,8 +987,9 @@ int launch_conv_tc(const tetris_filter *f, const float *in, float *out, const Co
       q.N = s.N; q.OH = s.OH; q.OW = s.OW; q.OC = s.OC; q.P = s.P; q.KS = s.KS;
       q.TW = best_tw; q.TH = best_th; q.NB = best_nb;
       q.PW = PW; q.PH = PH;
+      q.x_ring = patches && PW * PH * best_nb * 4 <= kPatchBytes / 2 ? 4 : 2;
       q.per_tap = per_tap ? 1 : 0; q.S = s.S;
-      q.folded = t->folded ? 1 : 0; q.in = in; q.H = s.H; q.W = s.W; q.IC = s.IC;
+      q.folded = patches ? 2 : t->folded ? 1 : 0; q.in = in; q.H = s.H; q.W = s.W; q.IC = s.IC;
       q.tiles_w = (s.OW + best_tw - 1) / best_tw;
       q.tiles_h = (s.OH + best_th - 1) / best_th;
       q.tiles_n = (s.N + best_nb - 1) / best_nb;
