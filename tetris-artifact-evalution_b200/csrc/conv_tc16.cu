@@ -217,12 +217,16 @@ __device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
-__device__ __forceinline__ float4 ld_cluster4(uint32_t addr, uint32_t rank) {
-  float4 v;
-  asm volatile("{\n.reg .b32 r;\nmapa.shared::cluster.u32 r, %4, %5;\nld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [r];\n}"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
-  return v;
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {  // `addr` of this CTA in CTA `rank` of the cluster
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
 }
+__device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+// Pixels of a tile that one CTA of a cluster of `d` adds up and stores: whole blocks of 16.
+__host__ __device__ constexpr int share_pixels(int npx, int d) { return ((npx >> 4) + d - 1) / d * 16; }
 
 // NMAX: most pixels of a tile.  A summing warp keeps NMAX / 2 running sums per thread, which sets
 // the register count: 12 warps (2 of them converters) for 256 pixels, 16 warps (6 converters) for
@@ -331,6 +335,8 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   // activation.  If the largest one lies outside FP16's window a last, banded pass follows.
   bool first = true, banded = false;
   int emax = 0;                       // exponent of the largest activation (banded pass)
+  uint32_t total_at = 0;              // d > 1: a summing warp's columns of its sums
+  float total_scale = 1.f;
   for (;;) {
     const int bands = banded ? kBands : 1;
     auto band_exp = [&](int b) { return banded ? min(127, 14 - emax + kBandBits * b) : 4; };  // scale of band b: 2^that
@@ -663,17 +669,8 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         ++sp;
         const int oc = oc0 + ocl;
         if (p.d > 1) {
-          // a slice of a tile: its sums into this CTA's shared memory (the rings are idle: every MMA
-          // of the only item has completed), one row of 128 accumulator lanes per pixel
-          float *rows = reinterpret_cast<float *>(xbase) + quarter * 32 + lane;
-#pragma unroll 1
-          for (int c0 = 0; c0 < ncols; c0 += 16) {
-            uint32_t v[16];
-            tmem_ld16(ttotal + c0, v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) rows[(j0 + c0 + j) * BM] = __uint_as_float(v[j]) * unscale;
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (a further pass loads over it)
+          total_at = ttotal;  // a slice of a tile: its sums stay in tensor memory until the cluster meets
+          total_scale = unscale;
         } else {
           // Store: a thread holds one channel of many pixels, an 8-pixel group of a warp is a box of
           // 32 channels x 8 pixels of the output.  16 pixels at a time go into a staging block (one
@@ -779,56 +776,69 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (tid == 0) atomicExch(p.error_flag, 1);
   }
   if (p.d > 1) {
-    // The slices of a tile meet: CTA `rank` adds up its share of the pixels over the cluster, in
-    // slice order, and stores them (a warp takes one pixel's 32 channels at a time).
+    // The slices of a tile meet.  Each CTA owns a share of the tile's pixels; once every ring of the
+    // cluster is idle, the summing warps write their sums of a pixel into its owner's shared memory (one
+    // row of 128 accumulator lanes per slice and pixel), and the owner adds the rows up in slice order and
+    // stores the result.  The code is small on purpose: it runs once, at the rate of its instruction
+    // fetches.  (Sums fetched from the other CTAs, four pixels per warp unrolled, and a barrier behind
+    // the stores took 6000 to 14000 clocks whatever the amount of data.)
+    const int per = share_pixels(p.npx, p.d);
     cluster_sync_all();
-    const int per = (p.npx + p.d - 1) / p.d, ja = rank * per, jb = min(p.npx, ja + per);
+    if (warp >= kFirstSum && !*abort_flag) {
+      const int me = warp - kFirstSum, quarter = me & 3, half = me >> 2;
+      const int hc = ((p.npx >> 4) + 1) / 2 * 16, j0 = half * hc, ncols = half ? p.npx - hc : hc;
+      const uint32_t row = smem_u32(xbase) + (uint32_t)(quarter * 32 + lane) * 4u;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+      for (int c0 = 0; c0 < ncols; c0 += 16) {
+        const int owner = (j0 + c0) / per;
+        const uint32_t dst = cluster_addr(row + (uint32_t)((rank * per + j0 + c0 - owner * per) * BM) * 4u, (uint32_t)owner);
+        uint32_t v[16];
+        tmem_ld16(total_at + c0, v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) st_cluster(dst + (uint32_t)(j * BM) * 4u, __uint_as_float(v[j]) * total_scale);
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    __syncwarp();
+    cluster_sync_all();  // (all rows have arrived; nothing reaches into another CTA after this)
     int oc0, w0, h0, n0;
     decode(tile0, oc0, w0, h0, n0);
-    // A lane adds up four channels of a pixel, 16 bytes per slice; four pixels in flight.
-    constexpr int kPix = STACK ? 2 : 1;                // pixels of a warp's row of loads
-    const int sub = STACK ? lane >> 4 : 0, oc = oc0 + 4 * (STACK ? lane & 15 : lane);
-    const uint32_t rows = smem_u32(xbase) + (uint32_t)(STACK ? lane & 15 : lane) * 16u;
+    constexpr int kPix = STACK ? 2 : 1;                // pixels of a warp at a time; a lane adds up four channels
+    const int l4 = 4 * (STACK ? lane & 15 : lane), oc = oc0 + l4;
     const bool vec = (p.OC & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
-    for (int j = ja + warp * 4 * kPix + sub; j < jb; j += kThreads / 32 * 4 * kPix) {
-      float4 y[4];
+    float sc[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) y[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < 4; ++i) sc[i] = oc + i < p.OC ? __ldg(p.out_scale + oc + i) : 0.f;
+    const float4 *rows = reinterpret_cast<const float4 *>(xbase) + (l4 >> 2);
+    const int jend = *abort_flag ? 0 : min(per, p.npx - rank * per);
+#pragma unroll 1
+    for (int j = warp * kPix + (STACK ? lane >> 4 : 0); j < jend; j += kThreads / 32 * kPix) {
+      float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 2
       for (int s = 0; s < p.d; ++s) {
-        float4 u[4], l[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t a = rows + (uint32_t)(min(j + e * kPix, jb - 1) * BM) * 4u;
-          u[e] = ld_cluster4(a, (uint32_t)s);
-          if (STACK) l[e] = ld_cluster4(a + 256u, (uint32_t)s);
+        float4 u = rows[(s * per + j) * (BM / 4)];
+        if (STACK) {
+          const float4 l = rows[(s * per + j) * (BM / 4) + 16];
+          u.x += l.x; u.y += l.y; u.z += l.z; u.w += l.w;
         }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (STACK) { u[e].x += l[e].x; u[e].y += l[e].y; u[e].z += l[e].z; u[e].w += l[e].w; }
-          y[e].x += u[e].x; y[e].y += u[e].y; y[e].z += u[e].z; y[e].w += u[e].w;
-        }
+        y.x += u.x; y.y += u.y; y.z += u.z; y.w += u.w;
       }
+      const int pix = pixel_of(rank * per + j, w0, h0, n0);
+      if (pix < 0 || oc >= p.OC) continue;
+      float v[4] = {y.x * sc[0], y.y * sc[1], y.z * sc[2], y.w * sc[3]};
+      if (p.relu) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int pix = j + e * kPix < jb && !*abort_flag ? pixel_of(j + e * kPix, w0, h0, n0) : -1;
-        if (pix < 0 || oc >= p.OC) continue;
-        float v[4] = {y[e].x, y[e].y, y[e].z, y[e].w};
+        for (int i = 0; i < 4; ++i) v[i] = fmaxf(v[i], 0.f);
+      }
+      float *o = p.out + (size_t)pix * p.OC + oc;
+      if (vec) *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+      else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          v[i] *= oc + i < p.OC ? __ldg(p.out_scale + oc + i) : 0.f;
-          if (p.relu) v[i] = fmaxf(v[i], 0.f);
-        }
-        float *o = p.out + (size_t)pix * p.OC + oc;
-        if (vec) *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
-        else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (oc + i < p.OC) o[i] = v[i];
-        }
+        for (int i = 0; i < 4; ++i)
+          if (oc + i < p.OC) o[i] = v[i];
       }
     }
-    cluster_sync_all();  // (nobody leaves while its shared memory is being read)
   }
   __syncthreads();
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
@@ -942,7 +952,7 @@ bool finish_geometry(const Tc16State &t, const ConvShape &s, Geometry *g) {
   // (more than half of an SM's: the CTAs of a launch that is placed while another one drains must
   // not be doubled up on the SMs that are free first)
   g->smem = std::max(fixed + (size_t)g->n_x * g->x_stage + g->n_w * wb, (size_t)116 * 1024);
-  if (g->d > 1 && (size_t)g->npx * BM * 4 > (size_t)g->n_x * g->x_stage + g->n_w * wb) return false;  // (the sums of a slice)
+  if (g->d > 1 && (size_t)g->d * share_pixels(g->npx, g->d) * BM * 4 > (size_t)g->n_x * g->x_stage + g->n_w * wb) return false;  // (the sums of a slice)
   // clocks per K step: the MMAs themselves, the shared-memory pipe (MMA operands, weight copy,
   // patch landing, read and written by the conversion), the conversion, the issuing warp
   const int nm = t.stack ? 4 : 6, conv = g->nmax == 256 ? 2 : 6;
