@@ -892,7 +892,8 @@ struct Geometry {
   int box_w = 1, box_h = 1, box_n = 1, reach = 0;  // patch load; furthest row a window touches
   int d = 1, nmax = 128, n_x = 2, n_w = 3, x_stage = 0;
   size_t smem = 0;
-  double cost = 0.;  // estimated clocks
+  double cost = 0.;  // estimated clocks, to compare with the list kernel's model
+  double rank = 0.;  // estimated clocks, to compare geometries
 };
 
 struct Tc16State {
@@ -968,6 +969,19 @@ bool finish_geometry(const Tc16State &t, const ConvShape &s, Geometry *g) {
   const double waves = std::ceil(tiles * g->d / slots);
   const double item = std::max(k_steps * step, 12. * g->npx) + 400.;
   g->cost = waves * item + 5000. + 10. * g->npx + 0.3 * box_rows * 10. + (g->d > 1 ? 2500. + 8. * g->npx + (waves - 1.) * 5000. : 0.);
+  // The geometries among themselves.  Measured on 26 layers, batch 1 to 16: loads reach an SM at about 30
+  // bytes per clock, weights (which many CTAs ask for at once) slower than patches -- 1x1 96 pixels
+  // 920 to 1160 clocks per K step (28 KB), 3x3 96 pixels 640 (18 KB), 176 pixels 1450 (38 KB); a K step
+  // of the smallest tiles takes 450; 6000 clocks pass before the first MMA; an epilogue takes 2000 clocks
+  // (32 pixels) to 4400 (176); a cluster meets in 3400 (16 pixels), 5300 (96), 7000 (112), 13000 (224).
+  // Without the load term small tiles in many CTAs looked cheap: 1x1 1024->1024 at 7x7 batch 1 took 128
+  // CTAs of 16 pixels, 11.8 us; 64 of 64 pixels take 9.6; 256->64 at 56x56 batch 16 128 pixels, 22.0,
+  // against 176, 19.8; 3x3 64->64 at 56x56 batch 1 10.1 against 9.2.
+  const double loads = wb / 24. + 128. * box_rows / steps / 40.;
+  const double slow = std::max(std::max(step, 450.), loads);
+  const double meet = g->d > 1 ? 2000. + 45. * g->npx : 1000. + 22. * g->npx;
+  g->rank = waves * (std::max(k_steps * slow, 12. * g->npx) + 400.) + 6000. + 3. * box_rows + meet +
+            (g->d > 1 ? (waves - 1.) * (6000. + meet) : 0.);
   return true;
 }
 
@@ -979,7 +993,7 @@ bool plan_geometry(const Tc16State &t, const ConvShape &s, Geometry *best) {
     for (int d = 1; d <= 8 && d <= t.n_chunks; d *= 2) {
       g.d = d;
       Geometry c = g;
-      if (finish_geometry(t, s, &c) && (!found || c.cost < best->cost)) { *best = c; found = true; }
+      if (finish_geometry(t, s, &c) && (!found || c.rank < best->rank)) { *best = c; found = true; }
     }
   };
   const long long pixels = (long long)s.N * s.OH * s.OW;
