@@ -106,6 +106,7 @@ struct Tc16Params {
   int x_stage_bytes, n_x, n_w;
   int tiles_w, tiles_h, tiles_n, oc_tiles, total_tiles;
   FastDiv by_oc_tiles, by_tiles_w, by_tiles_h, by_PW, by_PHI;
+  int super;                   // K steps per partial sum (a power of two)
   int n_chunks;
   int d;                       // CTAs of a cluster = slices of a tile's K range
   int relu;                    // max(y, 0) at the store
@@ -293,7 +294,7 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   const int chunk0 = p.n_chunks * rank / p.d, chunk1 = p.n_chunks * (rank + 1) / p.d;
   const int taps = p.KS * p.KS;
   const int iters = taps * (chunk1 - chunk0);       // K steps of an item (per band)
-  const int supers = (iters + kSuper - 1) / kSuper;
+  const int supers = (iters + p.super - 1) / p.super;
   const int phases = min(p.S, p.KS);                // input phases per axis that a tap falls into
   auto decode = [&](int t, int &oc0, int &w0, int &h0, int &n0) {
     int u = quot(t, p.by_oc_tiles);
@@ -443,14 +444,14 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       };
       int k = 0;                  // K step of the band
       auto step = [&](uint32_t xd, bool patch_end) {
-        const bool fresh = (k & (kSuper - 1)) == 0;
+        const bool fresh = (k & (p.super - 1)) == 0;
         if (fresh) wait(bar_pempty(sp & 1), ((sp >> 1) & 1) ^ 1);  // first step of a partial sum: its accumulator has been drained
         wait(bar_wfull(sw), pw);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem_d = tmem_base + (uint32_t)((sp & 1) * NMAX);
         const uint32_t wd = (uint32_t)dw0 + (uint32_t)(sw * (kWBytes >> 4));
         ++k;
-        const bool super_end = k == iters || (k & (kSuper - 1)) == 0;
+        const bool super_end = k == iters || (k & (p.super - 1)) == 0;
         if (elect_one()) {
           // K slices of 16 channels are 32 bytes = 2 in the address field; x_lo (w_lo) lies 64 bytes after x_hi (w_hi)
           if (STACK) {
@@ -1162,6 +1163,9 @@ int launch_conv_tc16(const tetris_filter *f, const float *in, float *out, const 
       q.by_oc_tiles = fast_div(q.oc_tiles); q.by_tiles_w = fast_div(q.tiles_w); q.by_tiles_h = fast_div(q.tiles_h);
       q.by_PW = fast_div(q.PW); q.by_PHI = fast_div(q.PHI);
       q.n_chunks = t->n_chunks; q.d = g->d;
+      // (strided layers keep the shorter chain of the split-TF32 kernel that ran them before: relative
+      // error 3.4e-7 against 4.9e-7 on 128->256 at 52x52)
+      q.super = s.S > 1 ? kSuper / 2 : kSuper;
       q.total_pixels = (long long)s.N * s.OH * s.OW;
       q.out_scale = t->d_out_scale; q.error_flag = t->d_error; q.w_tiles = t->d_tiles;
       cuuint64_t dims[4], strides[3];
