@@ -97,3 +97,21 @@ def test_activations_outside_the_window(tb, torch_cuda, oracle, case):
     assert oracle.compare(got[far], want[far])[0] == 0
     f.close()
     g.close()
+
+
+@pytest.mark.parametrize("case", [(1, 512, 14, 14, 128, 1, 1, 0), (1, 100, 7, 7, 64, 3, 1, 1), (1, 512, 7, 7, 256, 3, 1, 1),  # cut over clusters
+                                  (16, 32, 40, 40, 72, 3, 1, 1), (16, 32, 56, 56, 48, 3, 1, 1)],                          # whole tiles, plain and stacked
+                         ids=lambda c: "n%d_ic%d_%dx%d_oc%d_k%d_s%d_p%d" % c)
+@pytest.mark.parametrize("xe,we", [(112, 0), (126, -20), (-100, -20), (-60, -60), (-110, 40)])
+def test_scales_at_the_ends_of_fp32(tb, torch_cuda, oracle, case, xe, we):
+    """Activations x 2^xe, weights x 2^we: the results are normal FP32 numbers (or just below them), so they
+    have to be those of the unscaled layer times 2^(xe + we), to the bar of the path.  On the way the
+    kernel's sums, at the scale of its FP16 operands, lie up to 2^150 away from them.  (The smallest results,
+    about 2^-122, are rounded to multiples of 2^-149: 2e-8 of the layer's own scale.)"""
+    filt, x = _layer(case, 5)
+    want = oracle.host_conv2d(x, filt, case[6], case[7], threads=True)
+    f = tb.SparseFilter(np.ldexp(filt, we), case[1], case[4], case[5])
+    got = _run(tb, torch_cuda, f, np.ldexp(x, xe), case[6], case[7], False)
+    assert np.isfinite(got).all()
+    assert oracle.compare(np.ldexp(got.astype(np.float64), -xe - we).astype(np.float32), want)[0] == 0
+    f.close()

@@ -337,7 +337,7 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   bool first = true, banded = false;
   int emax = 0;                       // exponent of the largest activation (banded pass)
   uint32_t total_at = 0;              // d > 1: a summing warp's columns of its sums
-  float total_scale = 1.f;
+  float total_scale = 1.f;            // d > 1: what takes a summing lane's sums to the output's scale
   for (;;) {
     const int bands = banded ? kBands : 1;
     auto band_exp = [&](int b) { return banded ? min(127, 14 - emax + kBandBits * b) : 4; };  // scale of band b: 2^that
@@ -668,16 +668,37 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           ttotal = partial();
         }
         ++sp;
+        // The sums leave by one multiplication by 2^-sh[oc] / 16 times the banded pass's own factor, exact
+        // as powers of two.  Each factor alone can take a sum (up to 2^30) out of FP32's range though the
+        // result is inside it (|x| of 2^112 and weights of 0.05), and where both are tiny so can their
+        // product: there the sums take the banded pass's factor first, where they lie.
         const int oc = oc0 + ocl;
+        const float channel_scale = oc < p.OC ? p.out_scale[oc] : 0.f;
+        float sc = channel_scale * unscale;
+        if (banded) {
+          const bool apart = channel_scale != 0.f && !(sc >= 1.17549435e-38f && sc <= 3.402823466e38f);
+          if (__any_sync(0xffffffffu, apart)) {
+            const float f = apart ? unscale : 1.f;
+#pragma unroll 1
+            for (int c0 = 0; c0 < ncols; c0 += 16) {
+              uint32_t v[16];
+              tmem_ld16(ttotal + c0, v);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * f);
+              tmem_st16(ttotal + c0, v);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            if (apart) sc = channel_scale;
+          }
+        }
         if (p.d > 1) {
           total_at = ttotal;  // a slice of a tile: its sums stay in tensor memory until the cluster meets
-          total_scale = unscale;
+          total_scale = sc;
         } else {
           // Store: a thread holds one channel of many pixels, an 8-pixel group of a warp is a box of
           // 32 channels x 8 pixels of the output.  16 pixels at a time go into a staging block (one
           // conflict-free 4-byte store per value), which TMA stores carry on from there while the
           // warp stages the next block.
-          const float sc = oc < p.OC ? p.out_scale[oc] * unscale : 0.f;
           const int ocw = oc - lane;  // first channel of the warp
           auto put16 = [&](int c0, const float (&v)[16]) {  // pixels c0 .. c0 + 15 of this warp
             float *blk = blocks + (nblk & 1) * 512;
@@ -778,9 +799,9 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   }
   if (p.d > 1) {
     // The slices of a tile meet.  Each CTA owns a share of the tile's pixels; once every ring of the
-    // cluster is idle, the summing warps write their sums of a pixel into its owner's shared memory (one
-    // row of 128 accumulator lanes per slice and pixel), and the owner adds the rows up in slice order and
-    // stores the result.  The code is small on purpose: it runs once, at the rate of its instruction
+    // cluster is idle, the summing warps write their sums of a pixel, at the output's scale, into its owner's
+    // shared memory (one row of 128 accumulator lanes per slice and pixel), and the owner adds the rows up in
+    // slice order and stores the result.  The code is small on purpose: it runs once, at the rate of its instruction
     // fetches.  (Sums fetched from the other CTAs, four pixels per warp unrolled, and a barrier behind
     // the stores took 6000 to 14000 clocks whatever the amount of data.)
     const int per = share_pixels(p.npx, p.d);
@@ -808,9 +829,6 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     constexpr int kPix = STACK ? 2 : 1;                // pixels of a warp at a time; a lane adds up four channels
     const int l4 = 4 * (STACK ? lane & 15 : lane), oc = oc0 + l4;
     const bool vec = (p.OC & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
-    float sc[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) sc[i] = oc + i < p.OC ? __ldg(p.out_scale + oc + i) : 0.f;
     const float4 *rows = reinterpret_cast<const float4 *>(xbase) + (l4 >> 2);
     const int jend = *abort_flag ? 0 : min(per, p.npx - rank * per);
 #pragma unroll 1
@@ -827,7 +845,7 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       }
       const int pix = pixel_of(rank * per + j, w0, h0, n0);
       if (pix < 0 || oc >= p.OC) continue;
-      float v[4] = {y.x * sc[0], y.y * sc[1], y.z * sc[2], y.w * sc[3]};
+      float v[4] = {y.x, y.y, y.z, y.w};
       if (p.relu) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] = fmaxf(v[i], 0.f);
