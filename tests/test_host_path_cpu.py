@@ -1,0 +1,31 @@
+"""CPU: the host-array path (host_path.cu, memory.cu) against a model of the CUDA runtime, in a process of its own
+(tests/host_path_harness.cc): what it does between threads and when a call of the runtime fails."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "tetris-artifact-evalution_b200", "csrc")
+
+
+@pytest.fixture(scope="module")
+def harness(tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    if not os.path.exists(os.path.join(include, "cuda_runtime.h")):
+        pytest.skip("no CUDA headers")
+    exe = str(tmp_path_factory.mktemp("harness") / "harness")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-g", "-pthread", "-I", include, "-x", "c++", os.path.join(CSRC, "memory.cu"),
+                    os.path.join(CSRC, "host_path.cu"), os.path.join(ROOT, "tests", "host_path_harness.cc"), "-o", exe], check=True)
+    return exe
+
+
+def _run(harness, scenario):
+    res = subprocess.run([harness, scenario], capture_output=True, text=True, timeout=60)
+    assert res.returncode == 0, res.stderr
+
+
+def test_release_waits_for_a_call_that_uses_the_copy_streams(harness):
+    _run(harness, "release_race")

@@ -30,7 +30,7 @@ struct HostSlot {
   void *ptr = nullptr;
   size_t bytes = 0;
 };
-struct CopyStreams {
+struct CopyStreams {  // made under this mutex and one slot's, destroyed under those of all slots
   std::mutex mutex;
   cudaStream_t up = nullptr, down = nullptr;
 };
@@ -116,7 +116,9 @@ int tetris_conv2d_host_async(const tetris_filter_t *f, const float *h_input_nchw
   if (!h_input_nchw || !h_output_nchw) { set_error("input or output pointer is NULL"); return TETRIS_ERR_INVALID; }
   DeviceGuard guard(f->device);
   if (!guard.ok) { set_error("cudaSetDevice(%d) failed", f->device); return TETRIS_ERR_CUDA; }
-  cudaStream_t up, down;
+  HostSlot &hs = g_slots[f->device][slot];
+  std::lock_guard<std::mutex> lock(hs.mutex);
+  cudaStream_t up, down;  // (live while a slot's mutex is held)
   {
     CopyStreams &cs = g_copy[f->device];
     std::lock_guard<std::mutex> lock(cs.mutex);
@@ -124,8 +126,6 @@ int tetris_conv2d_host_async(const tetris_filter_t *f, const float *h_input_nchw
     if (!cs.down) TETRIS_CUDA_TRY(cudaStreamCreateWithFlags(&cs.down, cudaStreamNonBlocking));
     up = cs.up; down = cs.down;
   }
-  HostSlot &hs = g_slots[f->device][slot];
-  std::lock_guard<std::mutex> lock(hs.mutex);
   if (!hs.stream) TETRIS_CUDA_TRY(cudaStreamCreateWithFlags(&hs.stream, cudaStreamNonBlocking));
   for (cudaEvent_t *e : {&hs.arrived, &hs.computed, &hs.left})
     if (!*e) TETRIS_CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
@@ -191,9 +191,10 @@ void tetris_release_workspace(void) {
     ws.bytes = 0;
   }
   for (int dev = 0; dev < kMaxDevices; ++dev) {
+    std::unique_lock<std::mutex> slots[kSlots];  // (a call that holds its slot's may be using the copy streams)
+    for (int i = 0; i < kSlots; ++i) slots[i] = std::unique_lock<std::mutex>(g_slots[dev][i].mutex);
     for (int i = 0; i < kSlots; ++i) {
       HostSlot &hs = g_slots[dev][i];
-      std::lock_guard<std::mutex> lock(hs.mutex);
       if (!hs.stream && !hs.ptr) continue;
       if (cudaSetDevice(dev) != cudaSuccess) continue;
       if (hs.left) cudaEventSynchronize(hs.left);
