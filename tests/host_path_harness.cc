@@ -162,9 +162,39 @@ static int release_race() {
   return rc || g_faults ? 1 : 0;
 }
 
+// An event reports an error of the device: the call returns it, whichever way the data goes, and the next
+// call is served.  The first array is larger than the ring, the chunks that went round it are watched by events.
+static int device_error(bool upload) {
+  tetris_filter f = make_filter(16);
+  const int h = 700;
+  const auto x = ramp((size_t)16 * h * h);
+  std::vector<float> y(x.size(), -1.f);
+  if (tetris_conv2d_host(&f, x.data(), y.data(), 1, h, h, 1, 0, nullptr) || y != x || g_ring_copies == 0) return 1;
+  const int before = g_queries;
+  const int fail_at = upload ? 5 : 40;
+  g_query = [&](cudaEvent_t) { return g_queries - before >= fail_at ? cudaErrorIllegalAddress : cudaSuccess; };
+  if (tetris_conv2d_host(&f, x.data(), y.data(), 1, h, h, 1, 0, nullptr) != TETRIS_ERR_CUDA) return 1;
+  g_query = nullptr;
+  y.assign(y.size(), -1.f);
+  return tetris_conv2d_host(&f, x.data(), y.data(), 1, h, h, 1, 0, nullptr) || y != x || g_faults;
+}
+
+// The upload before this one ended in an error: so does this call
+static int upload_mark_error() {
+  tetris_filter f = make_filter(16);
+  const auto x = ramp((size_t)16 * 128 * 128);
+  std::vector<float> y(x.size());
+  if (tetris_conv2d_host(&f, x.data(), y.data(), 1, 128, 128, 1, 0, nullptr) || y != x) return 1;
+  g_event_sync = [](cudaEvent_t) { return cudaErrorIllegalAddress; };
+  return tetris_conv2d_host(&f, x.data(), y.data(), 1, 128, 128, 1, 0, nullptr) != TETRIS_ERR_CUDA;
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "release_race") return release_race();
+  if (what == "upload_error") return device_error(true);
+  if (what == "download_error") return device_error(false);
+  if (what == "upload_mark_error") return upload_mark_error();
   fprintf(stderr, "unknown scenario\n");
   return 2;
 }

@@ -115,12 +115,12 @@ class Stager {
   // The caller's array -> device; when this returns the array may be reused, the last copies out of
   // the ring may still be under way on `st`.
   cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st) {
-    cudaEventSynchronize(uploaded_);  // (the last upload has left the ring)
+    cudaError_t err = cudaEventSynchronize(uploaded_);  // (the last upload has left the ring)
+    if (err != cudaSuccess) return err;
     Job job;
     prepare(&job, static_cast<char *>(const_cast<void *>(src)), ring_in_, bytes, true);
     job.ready.store(std::min(job.n, kRing), std::memory_order_release);
     post(&job);
-    cudaError_t err = cudaSuccess;
     for (int sent = 0, back = 0; sent < job.n && err == cudaSuccess;) {
       if (job.done[sent].load(std::memory_order_acquire)) {
         const size_t at = (size_t)sent * job.chunk;
@@ -128,15 +128,20 @@ class Stager {
                               std::min(job.chunk, bytes - at), cudaMemcpyHostToDevice, st);
         if (err == cudaSuccess && job.n > kRing) err = cudaEventRecord(events_[sent % kRing], st);
         ++sent;
-      } else if (back < sent && back + kRing < job.n && cudaEventQuery(events_[back % kRing]) == cudaSuccess) {
-        job.ready.store(std::min(job.n, ++back + kRing), std::memory_order_release);  // that chunk of the ring is free again
+      } else if (back < sent && back + kRing < job.n) {
+        const cudaError_t q = cudaEventQuery(events_[back % kRing]);
+        if (q == cudaSuccess) job.ready.store(std::min(job.n, ++back + kRing), std::memory_order_release);  // that chunk of the ring is free again
+        else if (q != cudaErrorNotReady) err = q;
+        else if (!job.work()) relax();
       } else if (!job.work()) {
         relax();
       }
     }
     finish(&job);
     const cudaError_t marked = cudaEventRecord(uploaded_, st);
-    return err == cudaSuccess ? marked : err;
+    if (err == cudaSuccess) return marked;
+    cudaStreamSynchronize(st);  // (copies out of the ring may be under way)
+    return err;
   }
 
   // Device -> the caller's array, behind what `st` holds; complete when this returns.
