@@ -12,6 +12,7 @@
 #include <condition_variable>
 #include <functional>
 #include <mutex>
+#include <new>
 #include <set>
 #include <string>
 #include <thread>
@@ -29,6 +30,15 @@ static std::function<cudaError_t(cudaEvent_t)> g_event_sync;     // answers cuda
 static std::function<void(cudaStream_t)> g_on_wait, g_on_sync;   // called before these are answered
 static const char *g_ring = nullptr;
 static size_t g_ring_bytes = 0;
+
+static std::atomic<bool> g_no_memory{false};  // operator new fails
+void *operator new(size_t n) {
+  void *p = g_no_memory ? nullptr : malloc(n ? n : 1);
+  if (!p) throw std::bad_alloc();
+  return p;
+}
+void operator delete(void *p) noexcept { free(p); }
+void operator delete(void *p, size_t) noexcept { free(p); }
 
 static void use_stream(cudaStream_t s) {
   std::lock_guard<std::mutex> lock(g_model);
@@ -189,12 +199,27 @@ static int upload_mark_error() {
   return tetris_conv2d_host(&f, x.data(), y.data(), 1, 128, 128, 1, 0, nullptr) != TETRIS_ERR_CUDA;
 }
 
+// A staged copy, once the ring is there, takes no memory: nothing to throw through the C entry
+static int no_memory() {
+  tetris_filter f = make_filter(16);
+  const int h = 700;
+  const auto x = ramp((size_t)16 * h * h);
+  std::vector<float> y(x.size());
+  if (tetris_conv2d_host(&f, x.data(), y.data(), 1, h, h, 1, 0, nullptr) || y != x) return 1;
+  y.assign(y.size(), -1.f);
+  g_no_memory = true;
+  const int rc = tetris_conv2d_host(&f, x.data(), y.data(), 1, h, h, 1, 0, nullptr);
+  g_no_memory = false;
+  return rc || y != x;
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "release_race") return release_race();
   if (what == "upload_error") return device_error(true);
   if (what == "download_error") return device_error(false);
   if (what == "upload_mark_error") return upload_mark_error();
+  if (what == "no_memory") return no_memory();
   fprintf(stderr, "unknown scenario\n");
   return 2;
 }

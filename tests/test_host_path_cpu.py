@@ -34,3 +34,7 @@ def test_release_waits_for_a_call_that_uses_the_copy_streams(harness):
 @pytest.mark.parametrize("scenario", ["upload_error", "download_error", "upload_mark_error"])
 def test_an_error_of_the_device_ends_a_staged_copy(harness, scenario):
     _run(harness, scenario)
+
+
+def test_staged_copies_take_no_memory(harness):
+    _run(harness, "no_memory")

@@ -47,7 +47,8 @@ struct Job {
   bool to_ring;
   std::atomic<int> next{0};       // first chunk nobody has taken
   std::atomic<int> ready{0};      // chunks below this may be taken
-  std::atomic<unsigned char> *done;
+  // chunk i has been moved: flag i % kRing, taken back by the caller before chunk i + kRing is ready
+  std::atomic<unsigned char> done[kRing] = {};
   std::atomic<int> users{0};      // threads that hold a pointer to this job
 
   // Takes and moves one chunk; false if none may be taken now.
@@ -59,7 +60,12 @@ struct Job {
     char *u = user + (size_t)i * chunk, *r = ring + (size_t)(i % kRing) * kMaxChunk;
     const size_t len = std::min(chunk, bytes - (size_t)i * chunk);
     if (to_ring) memcpy(r, u, len); else memcpy(u, r, len);
-    done[i].store(1, std::memory_order_release);
+    done[i % kRing].store(1, std::memory_order_release);
+    return true;
+  }
+  bool take_done(int i) {
+    if (!done[i % kRing].load(std::memory_order_acquire)) return false;
+    done[i % kRing].store(0, std::memory_order_relaxed);
     return true;
   }
 };
@@ -122,7 +128,7 @@ class Stager {
     job.ready.store(std::min(job.n, kRing), std::memory_order_release);
     post(&job);
     for (int sent = 0, back = 0; sent < job.n && err == cudaSuccess;) {
-      if (job.done[sent].load(std::memory_order_acquire)) {
+      if (job.take_done(sent)) {
         const size_t at = (size_t)sent * job.chunk;
         err = cudaMemcpyAsync(static_cast<char *>(dst) + at, job.ring + (size_t)(sent % kRing) * kMaxChunk,
                               std::min(job.chunk, bytes - at), cudaMemcpyHostToDevice, st);
@@ -160,7 +166,7 @@ class Stager {
     while (sent < std::min(job.n, kRing) && err == cudaSuccess) send();
     post(&job);
     for (int moved = 0; moved < job.n && err == cudaSuccess;) {
-      if (job.done[moved].load(std::memory_order_acquire)) {
+      if (job.take_done(moved)) {
         if (sent < job.n && sent - moved <= kRing) send();  // (chunk `moved` of the ring is free again)
         ++moved;
       } else if (landed < sent) {
@@ -183,8 +189,6 @@ class Stager {
     // eight chunks or more, so that the first copy starts early and the last one is short
     job->chunk = std::min(kMaxChunk, std::max(kMinChunk, (bytes / 8 + 4095) / 4096 * 4096));
     job->n = (int)((bytes + job->chunk - 1) / job->chunk);
-    flags_ = std::vector<std::atomic<unsigned char>>(job->n);
-    job->done = flags_.data();
   }
   void post(Job *job) {
     { std::lock_guard<std::mutex> lock(mutex_); job_ = job; }
@@ -217,7 +221,6 @@ class Stager {
   Job *job_ = nullptr;
   bool stop_ = false;
   std::vector<std::thread> threads_;
-  std::vector<std::atomic<unsigned char>> flags_;
   char *ring_in_ = nullptr, *ring_out_ = nullptr;
   cudaEvent_t events_[kRing] = {}, uploaded_ = nullptr;
 };
