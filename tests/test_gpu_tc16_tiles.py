@@ -115,3 +115,36 @@ def test_scales_at_the_ends_of_fp32(tb, torch_cuda, oracle, case, xe, we):
     assert np.isfinite(got).all()
     assert oracle.compare(np.ldexp(got.astype(np.float64), -xe - we).astype(np.float32), want)[0] == 0
     f.close()
+
+
+# (n, ic, h, w, oc, ks, stride, pad) and the K steps of 32 channels that a partial sum may hold
+PARTIALS = [
+    ((16, 256, 14, 14, 1024, 1, 1, 0), 4),   # 1x1
+    ((2, 128, 20, 20, 128, 3, 1, 1), 4),     # larger filter, few tiles
+    ((2, 64, 57, 57, 96, 3, 2, 1), 4),       # strided
+    ((2, 512, 20, 20, 256, 1, 1, 0), 2),     # 1x1, few tiles: what a slice of the K range would hold
+    ((2, 512, 40, 40, 256, 1, 2, 0), 2),
+    ((2, 256, 10, 10, 1024, 1, 1, 0), 1),
+]
+
+
+@pytest.mark.parametrize("case,steps", PARTIALS, ids=lambda c: "n%d_ic%d_%dx%d_oc%d_k%d_s%d_p%d" % c if isinstance(c, tuple) else str(c))
+def test_error_against_64_bits(tb, torch_cuda, case, steps):
+    """The tensor core truncates its adds, so the error of a partial sum grows with its MMAs, six per K step.
+    An add loses half a unit in the last place on average, 0.72 * 2^-24 of the sum it leaves (the mean over a
+    binade), and the sums of a partial are half its final one on average: 0.36 * 2^-24 per MMA.  To that come the
+    roundings to nearest of the operands' halves and of the adds outside, a few 2^-25.  Relative, 2-norm."""
+    torch = torch_cuda
+    n, ic, h, w, oc, ks, stride, pad = case
+    rng = np.random.default_rng(5)
+    filt = rng.normal(0, 0.05, (oc, ic, ks, ks)).astype(np.float32)
+    filt[rng.random(filt.shape) < 0.8] = 0
+    x = rng.random((n, ic, h, w), dtype=np.float32)
+    x[rng.random(x.shape) < 0.5] = 0
+    f = tb.SparseFilter(filt, ic, oc, ks)
+    got = _run(tb, torch, f, x, stride, pad, False)
+    cols = torch.nn.functional.unfold(torch.from_numpy(x).cuda().double(), ks, padding=pad, stride=stride)
+    want = (torch.from_numpy(filt).cuda().double().reshape(oc, -1) @ cols).cpu().numpy().reshape(got.shape)
+    error = np.linalg.norm(got - want) / np.linalg.norm(want)
+    assert error < 0.36 * 2.0 ** -24 * 6 * steps + 3 * 2.0 ** -25, error
+    f.close()

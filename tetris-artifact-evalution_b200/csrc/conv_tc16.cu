@@ -64,7 +64,6 @@ namespace {
 constexpr int BM = 128, KC = 32;         // channels of a tile; K chunk (32 input channels)
 constexpr int kTW = 8;                   // a pixel group is 8 consecutive output columns
 constexpr int kXStagesMax = 6, kWStagesMax = 8;
-constexpr int kSuper = 8;                // K steps accumulated on the tensor core before the FP32 add outside
 constexpr int kSumWarps = 8;
 constexpr int kBands = 3, kBandBits = 16;  // second pass: bands of 16 binades below the largest activation
 // Per summing warp: two blocks of 16 pixels x 32 channels on their way to the output, and for
@@ -1062,6 +1061,30 @@ bool plan_geometry(const Tc16State &t, const ConvShape &s, Geometry *best) {
   return found;
 }
 
+// K steps the tensor core adds up before the sum is carried on outside: the error of an output, which is
+// that of the truncating adds inside a partial, grows with it (relative, against 64 bits, 256 channels and
+// more: 7.2e-7 with 8 steps, 4.0e-7 with 4, 2.4e-7 with 2, 1.6e-7 with 1; split TF32, whose K step is 12
+// MMAs instead of 6: 5.3e-7 with its 4 steps, 3.1e-7 with 2, 2.0e-7 with 1), and so does the speed: on VGG-19
+// at batch 16, 3x3 layers of 128 channels and more, 4 steps cost 1 to 11 % against 8, on 1x1 layers 0 to 4 %,
+// 2 steps 4 % more.  The rule keeps every layer at the error of the faster tensor-core kernel there was
+// for it before this one, or below:
+//   * larger filters than 1x1 at stride 1 with more than 32 channels and more than two waves of 128-pixel
+//     tiles: 8, as the split-FP16 kernel had that ran them (with fewer channels or tiles its fixed costs
+//     showed and split TF32 was faster: 24->128 at 112x112 batch 4 24.7 us against 26.7, 64->128 41.4 to 35.0);
+//   * others: 4, as the split-TF32 kernel that ran them has; 1x1 layers of few tiles, whose K range that
+//     kernel cuts into slices added up in FP32, no more steps than a slice has;
+//   * stacked filters do a K step in 4 MMAs and carry the same error over twice the steps (8: 4.7e-7).
+int partial_steps(const Tc16State &t, const ConvShape &s) {
+  const long long pixels = (long long)s.N * s.OH * s.OW, tiles = (pixels + 127) / 128 * t.oc_tiles;
+  if (s.KS > 1 && s.S == 1 && t.n_chunks > 1 && tiles > 2ll * t.sms) return 8;
+  int steps = 4;
+  if (s.KS == 1)
+    for (int d = 2; d <= 8 && tiles * d <= t.sms; ++d)
+      if (t.n_chunks % d == 0)
+        while (steps > 1 && steps > t.n_chunks / d) steps /= 2;
+  return t.stack && s.S == 1 ? 2 * steps : steps;
+}
+
 // The geometry of a shape, planned once (the caller holds the state's mutex).
 const Geometry *geometry_of(Tc16State *t, const ConvShape &s) {
   if (t->last_geo.mode < 0 || !same_conv(t->last_shape, s)) {
@@ -1181,9 +1204,7 @@ int launch_conv_tc16(const tetris_filter *f, const float *in, float *out, const 
       q.by_oc_tiles = fast_div(q.oc_tiles); q.by_tiles_w = fast_div(q.tiles_w); q.by_tiles_h = fast_div(q.tiles_h);
       q.by_PW = fast_div(q.PW); q.by_PHI = fast_div(q.PHI);
       q.n_chunks = t->n_chunks; q.d = g->d;
-      // (strided layers keep the shorter chain of the split-TF32 kernel that ran them before: relative
-      // error 3.4e-7 against 4.9e-7 on 128->256 at 52x52)
-      q.super = s.S > 1 ? kSuper / 2 : kSuper;
+      q.super = partial_steps(*t, s);
       q.total_pixels = (long long)s.N * s.OH * s.OW;
       q.out_scale = t->d_out_scale; q.error_flag = t->d_error; q.w_tiles = t->d_tiles;
       cuuint64_t dims[4], strides[3];
