@@ -108,3 +108,33 @@ def test_chain_graph_equals_synchronised_layers(tb, torch_cuda, oc):
         chain.replay()
     assert np.array_equal(chain.download(), want)
     chain.close()
+
+
+@pytest.mark.parametrize("n,h,ic,oc,ks", [(4, 28, 65, 128, 5), (16, 7, 515, 515, 3), (2, 52, 315, 72, 3), (16, 28, 129, 130, 3)])
+def test_list_kernel_spreads_over_the_device_back_to_back(tb, torch_cuda, n, h, ic, oc, ks):
+    """A launch placed early must not double up on the SMs that were free first (1.4 to 1.6 times the time): a
+    launch among others takes no longer than one that is waited for, which has the host's part on top."""
+    torch = torch_cuda
+    rng = np.random.default_rng(0)
+    w = rng.normal(0, 0.05, (oc, ic, ks, ks)).astype(np.float32)
+    w[rng.random(w.shape) < 0.875] = 0
+    f = tb.SparseFilter(w, ic, oc, ks)
+    x, y = torch.rand(n, h, h, ic, device="cuda"), torch.empty(n, h, h, oc, device="cuda")
+
+    def per_launch(count):
+        times = []
+        for _ in range(11):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            for _ in range(count):
+                tb.sparse_conv2d(f, x, y, n, h, h, 1, ks // 2, variant=tb.VARIANT_TILED, cuda_stream=torch.cuda.current_stream())
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b) / count)
+        return sorted(times)[5]
+
+    tb.tune_sparse_conv2d(f, x, y, n, h, h, 1, ks // 2)
+    per_launch(20)
+    assert per_launch(20) < 1.1 * per_launch(1)
+    f.close()

@@ -296,6 +296,7 @@ struct Plan {
   TiledParams p{};
   dim3 grid;
   size_t smem_bytes = 0;
+  bool overlapped = false;
 };
 
 // Row pitch in 8-byte slots: at least `need`, chosen so that the 16 lanes of a half-warp (one
@@ -320,6 +321,7 @@ int pick_row_slots(int need, int NSEG, int TH, int S) {
 }
 
 constexpr size_t kSmemLimit = (size_t)225 * 1024;
+constexpr size_t kSmemPerSm = (size_t)228 * 1024, kSmemReserved = 1024;  // of an SM; what a CTA takes beside its own
 
 struct Instance {
   int K, P2, WARPS, MINB;
@@ -382,7 +384,19 @@ double plan_cost(const tetris_filter *f, const ConvShape &s, const Instance &ins
     p.tic_shift = 0;
     while ((1 << p.tic_shift) < TIC) ++p.tic_shift;
     out->grid = dim3((unsigned)(tiles_w * tiles_h * n_pairs), (unsigned)ctas_y);
-    out->smem_bytes = smem;
+    // Overlapped with the launch before it only where all CTAs are resident at once and alike, and then with
+    // at least so much shared memory that no SM holds more of them than an even spread gives it.  A launch
+    // that is placed while another one drains takes the SMs as they come free, several CTAs on the first
+    // ones and none on the last: 65->128 5x5 at 28x28 batch 4 took 151 us among others, 89 with the floor, 92
+    // launched in the ordinary way; 515->515 3x3 at 7x7 batch 16 247, 173 and 174.  CTAs whose warps are
+    // partly idle (the last ones of a channel count that is no multiple of a CTA's) are spread evenly by
+    // their order only in an ordinary launch: 129->130 3x3 at 28x28 batch 16 106, 106 and 82; 27->75 1x1 at
+    // 100x100 batch 3 28.2, 28.2 and 22.7.
+    const bool alike = ctas_y == 1 || f->n_oc_blocks % inst.WARPS == 0;
+    out->overlapped = waves <= 1.0 && (alike || ctas <= sm_count);
+    const size_t share = (size_t)std::ceil(ctas / sm_count) + 1;
+    const size_t floor = kSmemPerSm / share > kSmemReserved ? kSmemPerSm / share - kSmemReserved + 16 : 0;
+    out->smem_bytes = std::max(smem, std::min(smem_limit, floor / 16 * 16));
   }
   return t;
 }
@@ -463,7 +477,12 @@ int launch_instance(const Plan &plan, const float *in, float *out, cudaStream_t 
   TiledParams p = plan.p;
   p.in = in;
   p.out = out;
-  TETRIS_CUDA_TRY(launch_overlapped(kern, plan.grid, WARPS * 32, plan.smem_bytes, st, 1, p));
+  if (plan.overlapped) {
+    TETRIS_CUDA_TRY(launch_overlapped(kern, plan.grid, WARPS * 32, plan.smem_bytes, st, 1, p));
+  } else {
+    kern<<<plan.grid, WARPS * 32, plan.smem_bytes, st>>>(p);
+    TETRIS_CUDA_TRY(cudaGetLastError());
+  }
   count_launch();
   return TETRIS_OK;
 }
