@@ -148,3 +148,25 @@ def test_error_against_64_bits(tb, torch_cuda, case, steps):
     error = np.linalg.norm(got - want) / np.linalg.norm(want)
     assert error < 0.36 * 2.0 ** -24 * 6 * steps + 3 * 2.0 ** -25, error
     f.close()
+
+
+@pytest.mark.parametrize("channels", [64, 160])  # stacked tiles, plain ones
+@pytest.mark.parametrize("top,bottom", [(13, -18), (13, -19), (13, -35), (-9, -40), (-9, -57), (100, 69), (-60, -108)])
+def test_bands_of_activations(tb, torch_cuda, channels, top, bottom):
+    """Activations of every binade from 2^top down to 2^bottom, each output reading one of them: the bands --
+    two for 32 binades, three below -- keep every activation's 22 bits down to 49 binades below the largest
+    (operand halves rounded to nearest at 11 bits each: 2^-22 of activation and of weight, the product of the
+    remainders left out 2^-22, and one truncated add of the three products 2^-23)."""
+    rng = np.random.default_rng(0)
+    weights = rng.uniform(0.5, 2, channels).astype(np.float32)
+    filt = np.zeros((channels, channels, 1, 1), np.float32)
+    filt[np.arange(channels), np.arange(channels), 0, 0] = weights
+    shape = (2, channels, 40, 33)
+    x = np.ldexp(rng.uniform(1, 2, shape), rng.integers(bottom, top + 1, shape)).astype(np.float32)
+    x[rng.random(shape) < 0.3] = 0
+    x = x * rng.choice(np.float32([-1, 1]), shape)
+    f = tb.SparseFilter(filt, channels, channels, 1)
+    got = _run(tb, torch_cuda, f, x, 1, 0, False).astype(np.float64)
+    want = x.astype(np.float64) * weights.reshape(1, -1, 1, 1)
+    assert (np.abs(got - want) <= 4 * 2.0 ** -22 * np.abs(want)).all()
+    f.close()

@@ -11,9 +11,9 @@
 //
 // Range.  FP16 has a window: |x| < 2048 after the fixed scale, absolute error of at most 2e-9 per
 // activation.  The converter warps of a CTA record the largest |x| they see; a CTA that finds it
-// outside [2^-8, 2048) runs its work items a second time with a scale taken from that maximum and
-// the activations cut into three bands of 16 binades, one pass over K per band, whose sums are
-// added up in FP32 (see kBands).  No second launch and no state between launches: what a CTA
+// outside [2^-8, 2048) runs its work items again with a scale taken from that maximum and the
+// activations cut into two bands, the upper one of 16 binades, with a pass over K per band, whose sums
+// are added up in FP32; where activations lie below 32 binades, a last time with three bands.  No second launch and no state between launches: what a CTA
 // recomputes is its own output.
 //
 // The tensor core truncates when it adds into its FP32 accumulator, so the accumulation chain is
@@ -65,7 +65,7 @@ constexpr int BM = 128, KC = 32;         // channels of a tile; K chunk (32 inpu
 constexpr int kTW = 8;                   // a pixel group is 8 consecutive output columns
 constexpr int kXStagesMax = 6, kWStagesMax = 8;
 constexpr int kSumWarps = 8;
-constexpr int kBands = 3, kBandBits = 16;  // second pass: bands of 16 binades below the largest activation
+constexpr int kBandBits = 16;            // banded passes: bands of 16 binades below the largest activation
 // Per summing warp: two blocks of 16 pixels x 32 channels on their way to the output, and for
 // stacked tiles 32 pixels x 32 accumulator lanes handed to the warp with the other half.
 __host__ __device__ constexpr int stage_bytes(bool stack) { return kSumWarps * (4096 + (stack ? 4096 : 0)); }
@@ -228,6 +228,69 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
 // Pixels of a tile that one CTA of a cluster of `d` adds up and stores: whole blocks of 16.
 __host__ __device__ constexpr int share_pixels(int npx, int d) { return ((npx >> 4) + d - 1) / d * 16; }
 
+// One 128-byte row of a patch, in place: 32 FP32 channels, each through `scaled`, to {x_hi[32], x_lo[32]} FP16.
+// `look` sees the 16-byte pieces before.
+template <typename F, typename G>
+__device__ __forceinline__ void convert_row(float4 *rp, int swz, F scaled, G look) {
+  float4 v[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) v[c] = rp[c ^ swz];
+  uint32_t hi[16], lo[16];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    look(v[c]);
+    const float x[4] = {scaled(v[c].x), scaled(v[c].y), scaled(v[c].z), scaled(v[c].w)};
+    const __half2 h01 = __floats2half2_rn(x[0], x[1]), h23 = __floats2half2_rn(x[2], x[3]);
+    const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
+    hi[2 * c] = *reinterpret_cast<const uint32_t *>(&h01);
+    hi[2 * c + 1] = *reinterpret_cast<const uint32_t *>(&h23);
+    lo[2 * c] = pack_half2(x[0] - f01.x, x[1] - f01.y);
+    lo[2 * c + 1] = pack_half2(x[2] - f23.x, x[3] - f23.y);
+  }
+  uint4 *wp = reinterpret_cast<uint4 *>(rp);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    wp[c ^ swz] = make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]);
+    wp[(c + 4) ^ swz] = make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]);
+  }
+}
+
+// The same in the passes behind the first, which few launches make: out of line, so that the first one's code and
+// registers stay as they are (inlined, the smallest launches took 2 % longer: 64->64 3x3 at 56x56, one image).
+// band < 0: all of it, `seen` becomes the bits of the largest finite |activation|.  band 0: what is not below `lo`
+// (infinities and NaN with it).  band > 0: what lies in [lo, hi); `seen` becomes 2 * bits - 1 of the smallest
+// |activation|, zeros last.
+__device__ __noinline__ unsigned convert_row_again(uint32_t saddr, int swz, float scale, float lo, float hi, unsigned seen, int band) {
+  float4 *rp = static_cast<float4 *>(__cvta_shared_to_generic(saddr));
+  auto nothing = [](const float4 &) {};
+  if (band < 0)
+    convert_row(rp, swz, [&](float x) {
+      if (fabsf(x) < __int_as_float(0x7F800000)) seen = max(seen, __float_as_uint(fabsf(x)));
+      return x * scale;
+    }, nothing);
+  else if (band == 0)
+    convert_row(rp, swz, [&](float x) { return fabsf(x) < lo ? 0.f : x * scale; }, nothing);
+  else
+    convert_row(rp, swz, [&](float x) {
+      seen = min(seen, 2u * __float_as_uint(x) - 1u);
+      return fabsf(x) < hi && !(fabsf(x) < lo) ? x * scale : 0.f;
+    }, nothing);
+  return seen;
+}
+
+// Sums of a lane in tensor memory, multiplied by f.
+__device__ __noinline__ void scale_columns(uint32_t taddr, int ncols, float f) {
+#pragma unroll 1
+  for (int c0 = 0; c0 < ncols; c0 += 16) {
+    uint32_t v[16];
+    tmem_ld16(taddr + c0, v);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * f);
+    tmem_st16(taddr + c0, v);
+  }
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 // NMAX: most pixels of a tile.  A summing warp keeps NMAX / 2 running sums per thread, which sets
 // the register count: 12 warps (2 of them converters) for 256 pixels, 16 warps (6 converters) for
 // 128.  STACK: at most 64 output channels, {w_hi, w_lo} stacked on the M side.
@@ -332,13 +395,20 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   int x_loads = 0, w_loads = 0;
   bool ok = true;
   // Pass 0: scale 16.  If it saw an infinity, pass 1 repeats it looking for the largest FINITE
-  // activation.  If the largest one lies outside FP16's window a last, banded pass follows.
-  bool first = true, banded = false;
-  int emax = 0;                       // exponent of the largest activation (banded pass)
+  // activation.  If the largest one lies outside FP16's window, a pass of two bands follows, and if that
+  // saw an activation too small for its lower band (22 bits down to 2^-33 of the largest) one of three.
+  // (Always three, and each element's band worked out from its exponent: 128->256 3x3 s2 at 104x104
+  // batch 16, all activations 1e-5, 574 us; 356 now.  64->64 3x3 at 56x56 batch 16 84 and 63,
+  // 512->512 1x1 at 14x14 batch 16 58.7 and 42.7.)
+  bool first = true;
+  int bands = 1;
+  int emax = 0;                       // exponent of the largest activation (banded passes)
   uint32_t total_at = 0;              // d > 1: a summing warp's columns of its sums
   float total_scale = 1.f;            // d > 1: what takes a summing lane's sums to the output's scale
+  // lower end of band b: 2^(emax - 15 - 16 b), zero below the normal numbers
+  auto band_end = [&](int b) { const int e = emax + 1 - kBandBits * (b + 1); return e < -126 ? 0.f : pow2f(e); };
   for (;;) {
-    const int bands = banded ? kBands : 1;
+    const bool banded = bands > 1;
     auto band_exp = [&](int b) { return banded ? min(127, 14 - emax + kBandBits * b) : 4; };  // scale of band b: 2^that
     if (warp == 0) {
       // ---- loads: two independent cursors (patches, weight images) polled in turn ----
@@ -509,56 +579,25 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       //      sit at piece ^ (r & 7) before and after, so the eight lanes of a quarter-warp touch
       //      eight different bank groups ----
       const int ct = (warp - 2) * 32 + lane;
-      float seen = 0.f;
-      auto split = [](const float (&x)[4], uint32_t *hi, uint32_t *lo) {
-        const __half2 h01 = __floats2half2_rn(x[0], x[1]), h23 = __floats2half2_rn(x[2], x[3]);
-        const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
-        hi[0] = *reinterpret_cast<const uint32_t *>(&h01);
-        hi[1] = *reinterpret_cast<const uint32_t *>(&h23);
-        lo[0] = pack_half2(x[0] - f01.x, x[1] - f01.y);
-        lo[1] = pack_half2(x[2] - f23.x, x[3] - f23.y);
-      };
+      // bits of the largest |activation|; banded passes: 2 * bits - 1 of the smallest one, zeros last
+      unsigned seen = banded ? ~0u : 0u;
+      auto note = [&](float a) { seen = __float_as_uint(fmaxf(__uint_as_float(seen), a)); };
       for (int t = tile0; t < p.total_tiles && ok; t += tile_step)
         for (int b = bands - 1; b >= 0 && ok; --b) {
           const float scale = pow2f(band_exp(b));
+          const float band_lo = b == bands - 1 ? 0.f : band_end(b), band_hi = band_end(b - 1);  // (infinities and NaN are in the upper band)
           for (int u = (chunk1 - chunk0) * phases * phases; u > 0; --u) {
             if (!(ok = mbar_wait_warp(bar_xfull(sx), px, abort_flag))) break;
             unsigned char *stage = xbase + (size_t)sx * p.x_stage_bytes;
             for (int row = ct; row < p.box_rows; row += 32 * kConv) {
               float4 *rp = reinterpret_cast<float4 *>(stage + (size_t)row * 128);
-              const int swz = row & 7;
-              float4 v[8];
-#pragma unroll
-              for (int c = 0; c < 8; ++c) v[c] = rp[c ^ swz];
-              uint32_t hi[16], lo[16];
-              if (first) {
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                  seen = fmaxf(seen, fmaxf(fabsf(v[c].x), fabsf(v[c].y)));
-                  seen = fmaxf(seen, fmaxf(fabsf(v[c].z), fabsf(v[c].w)));
-                  const float x[4] = {kXScale * v[c].x, kXScale * v[c].y, kXScale * v[c].z, kXScale * v[c].w};
-                  split(x, hi + 2 * c, lo + 2 * c);
-                }
-              } else {
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                  float x[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    const int ex = (int)((__float_as_uint(x[e]) >> 23) & 0xFFu) - 127;  // 128: infinity or NaN, kept in band 0
-                    if (ex < 128) seen = fmaxf(seen, fabsf(x[e]));
-                    const int mine = banded ? min(kBands - 1, max(0, emax - ex) / kBandBits) : 0;
-                    x[e] = mine == b ? x[e] * scale : 0.f;
-                  }
-                  split(x, hi + 2 * c, lo + 2 * c);
-                }
-              }
-              uint4 *wp = reinterpret_cast<uint4 *>(rp);
-#pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                wp[c ^ swz] = make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]);
-                wp[(c + 4) ^ swz] = make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]);
-              }
+              if (first)
+                convert_row(rp, row & 7, [](float x) { return kXScale * x; }, [&](const float4 &v) {
+                  note(fmaxf(fabsf(v.x), fabsf(v.y)));
+                  note(fmaxf(fabsf(v.z), fabsf(v.w)));
+                });
+              else
+                seen = convert_row_again(smem_u32(rp), row & 7, scale, band_lo, band_hi, seen, banded ? b : -1);
             }
             // the writes above go through the generic proxy, the MMAs read through the async proxy
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -567,7 +606,8 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (++sx == p.n_x) { sx = 0; px ^= 1u; }
           }
         }
-      unsigned m = __float_as_uint(seen);
+      unsigned m = seen;
+      if (banded) m = band_end(1) > 0.f && seen < 2u * __float_as_uint(band_end(1)) - 1u;  // (a third band would hold it)
       for (int s = 16; s; s >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, s));
       if (lane == 0) atomicMax(seen_slot, m);
     } else {
@@ -677,16 +717,7 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         if (banded) {
           const bool apart = channel_scale != 0.f && !(sc >= 1.17549435e-38f && sc <= 3.402823466e38f);
           if (__any_sync(0xffffffffu, apart)) {
-            const float f = apart ? unscale : 1.f;
-#pragma unroll 1
-            for (int c0 = 0; c0 < ncols; c0 += 16) {
-              uint32_t v[16];
-              tmem_ld16(ttotal + c0, v);
-#pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * f);
-              tmem_st16(ttotal + c0, v);
-            }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            scale_columns(ttotal, ncols, apart ? unscale : 1.f);
             if (apart) sc = channel_scale;
           }
         }
@@ -774,13 +805,17 @@ conv_tc16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned m = *reinterpret_cast<volatile unsigned *>(seen_slot);
-    const bool stop = *abort_flag != 0 || banded || (m < 0x45000000u && (m == 0u || m >= 0x3B800000u));
-    if (stop) break;
-    banded = m < 0x7F800000u;
-    emax = (int)(m >> 23) - 127;
+    const bool in_window = m < 0x45000000u && (m == 0u || m >= 0x3B800000u);
+    if (*abort_flag != 0 || bands == 3 || (bands == 2 ? m == 0u : in_window)) break;
+    if (bands == 2) {
+      bands = 3;
+    } else if (m < 0x7F800000u) {
+      bands = 2;
+      emax = (int)(m >> 23) - 127;
+    }
     first = false;
     __syncthreads();
-    if (tid == 0 && !banded) *seen_slot = 0u;
+    if (tid == 0) *seen_slot = 0u;
     __syncthreads();
   }
 
