@@ -170,3 +170,33 @@ def test_bands_of_activations(tb, torch_cuda, channels, top, bottom):
     want = x.astype(np.float64) * weights.reshape(1, -1, 1, 1)
     assert (np.abs(got - want) <= 4 * 2.0 ** -22 * np.abs(want)).all()
     f.close()
+
+
+@pytest.mark.parametrize("oc,sparsity", [(17, 0.875), (16, 0.8), (33, 0.8)])
+def test_untuned_choice_on_odd_channel_counts(tb, torch_cuda, oc, sparsity):
+    """Channel counts that are no multiple of four are stored value by value, which the estimate behind the
+    untuned choice has to know: the chosen kernel is the faster one, or not more than a quarter slower."""
+    torch = torch_cuda
+    n, h, ic = 4, 112, 32
+    rng = np.random.default_rng(0)
+    filt = rng.normal(0, 0.05, (oc, ic, 3, 3)).astype(np.float32)
+    filt[rng.random(filt.shape) < sparsity] = 0
+    f = tb.SparseFilter(filt, ic, oc, 3)
+    x, y = torch.rand(n, h, h, ic, device="cuda"), torch.empty(n, h, h, oc, device="cuda")
+
+    def per_launch(variant):
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            for _ in range(20):
+                tb.sparse_conv2d(f, x, y, n, h, h, 1, 1, variant=variant, cuda_stream=torch.cuda.current_stream())
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return sorted(times)[3]
+
+    kernels = {v: per_launch(v) for v in (tb.VARIANT_TILED, tb.VARIANT_TENSOR16)}
+    assert kernels[tb.auto_choice(f, n, h, h, 1, 1)] < 1.25 * min(kernels.values())
+    f.close()

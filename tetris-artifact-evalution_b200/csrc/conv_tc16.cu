@@ -945,8 +945,11 @@ struct Geometry {
   int box_w = 1, box_h = 1, box_n = 1, reach = 0;  // patch load; furthest row a window touches
   int d = 1, nmax = 128, n_x = 2, n_w = 3, x_stage = 0;
   size_t smem = 0;
-  double cost = 0.;  // estimated clocks, to compare with the list kernel's model
-  double rank = 0.;  // estimated clocks, to compare geometries
+  // Estimated clocks.  `cost` leaves out what loads cost and comes out a quarter below `rank`; the list kernel's
+  // model it is compared with comes out low as well, and with `rank` in its place that comparison chose worse
+  // (untuned layers, 356 of them: 1.6 % above the faster kernel on average, 3.5 % with `rank`).
+  double cost = 0.;  // to compare with the list kernel's model
+  double rank = 0.;  // to compare geometries
 };
 
 struct Tc16State {
@@ -1020,7 +1023,9 @@ bool finish_geometry(const Tc16State &t, const ConvShape &s, Geometry *g) {
   // (clusters of d CTAs live inside a GPC: on the 148-SM part 148 CTAs in pairs, 132 in fours, 120 in eights)
   const double slots = g->d <= 2 ? t.sms : g->d * std::floor(t.sms * (g->d == 4 ? 0.225 : 0.1015));
   const double waves = std::ceil(tiles * g->d / slots);
-  const double item = std::max(k_steps * step, 12. * g->npx) + 400.;
+  // (channel counts TMA stores do not take leave value by value: 32->17 3x3 at 112x112 batch 4, 26.9 us against
+  // 14.7 with 16 channels; with 12 clocks a pixel there, too, it was chosen before the list kernel's 15.4)
+  const double item = std::max(k_steps * step, ((s.OC & 3) == 0 || g->d > 1 ? 12. : 33.) * g->npx) + 400.;
   g->cost = waves * item + 5000. + 10. * g->npx + 0.3 * box_rows * 10. + (g->d > 1 ? 2500. + 8. * g->npx + (waves - 1.) * 5000. : 0.);
   // The geometries among themselves.  Measured on 26 layers, batch 1 to 16: loads reach an SM at about 30
   // bytes per clock, weights (which many CTAs ask for at once) slower than patches -- 1x1 96 pixels

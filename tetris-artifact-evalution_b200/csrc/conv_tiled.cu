@@ -455,8 +455,10 @@ int make_plan(const tetris_filter *f, const ConvShape &s, Plan *plan) {
   if (rc) return rc;
   fill_plan(f, s, cands[0], sm_count, plan);
   // The list kernel's wavefront model counts issue slots only and comes out 1.2-1.75x below the
-  // measured time (1.45x on the layers where the two kernels are close); the tensor-core figures
-  // are measured ones.
+  // measured time (1.45x on the layers where the two kernels are close); the split-TF32 figures are
+  // measured ones, the split-FP16 kernel's an estimate (see Geometry).  A strided layer goes to the latter
+  // even where split TF32 would be faster (5 of 117 strided layers, by 3 to 22 %, one 5 % faster than
+  // before): the split-TF32 figures leave out its cut K ranges, so they cannot tell; tuning does.
   const double tc16 = conv_tc16_cost(f, s);
   if (tc16 >= 0. && tc16 < 1.45 * cands[0].cost) plan->use_tc = 2;
   else plan->use_tc = tc16 < 0. && conv_tc_supported(f, s) && tc_cost(f, s, sm_count) < 1.45 * cands[0].cost ? 1 : 0;
