@@ -60,3 +60,25 @@ def test_filters_made_and_closed_in_turn(tb, torch_cuda):
             tb.release_workspace()
     for f, x, want in kept:
         assert np.array_equal(tb.cuda_sparse_conv2d(x, f, 1, 20, 20, 1, 0), want)
+
+
+def test_large_upload_small_download(tb, torch_cuda):
+    """Helpers that sleep while the layer computes must not leave the ring's lines in their caches: the copy engine
+    then took 500 us for 4 MB.  The yardstick is the same call on page-locked arrays, which are copied directly
+    (110 us): staging may add the time of a few memcpys, not multiples."""
+    import time
+    torch = torch_cuda
+    rng = np.random.default_rng(0)
+    f = tb.SparseFilter(rng.normal(0, 0.1, (4, 256, 1, 1)).astype(np.float32), 256, 4, 1)
+    arrays = [rng.random((1, 256, 64, 64), dtype=np.float32) for _ in range(4)]
+    pinned = [torch.from_numpy(a).pin_memory() for a in arrays]
+
+    def median(inputs):
+        times = []
+        for i in range(80):
+            t = time.perf_counter()
+            tb.cuda_sparse_conv2d(inputs[i % 4], f, 1, 64, 64, 1, 0)
+            times.append(time.perf_counter() - t)
+        return sorted(times[20:])[30]
+
+    assert median(arrays) < 3 * median([p.numpy() for p in pinned])
