@@ -7,6 +7,7 @@
 #include <string.h>
 #include <time.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -51,8 +52,9 @@ static void use_event(cudaEvent_t e) {
 static bool in_ring(const void *p) { return g_ring && (const char *)p >= g_ring && (const char *)p < g_ring + g_ring_bytes; }
 
 extern "C" {
-cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
-cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+static thread_local int t_device = 0;
+cudaError_t cudaGetDevice(int *d) { *d = t_device; return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { t_device = d; return cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "error"; }
@@ -213,6 +215,53 @@ static int no_memory() {
   return rc || y != x;
 }
 
+// While the device computes, the helpers of a download sleep: the call takes the processor time of its own thread
+static int idle_helpers() {
+  tetris_filter f = make_filter(16);
+  const int h = 200;
+  const auto x = ramp((size_t)16 * h * h);
+  std::vector<float> y(x.size());
+  if (tetris_conv2d_host(&f, x.data(), y.data(), 1, h, h, 1, 0, nullptr) || y != x) return 1;
+  const auto busy_until = std::chrono::steady_clock::now() + 400ms;
+  g_query = [&](cudaEvent_t) { return std::chrono::steady_clock::now() < busy_until ? cudaErrorNotReady : cudaSuccess; };
+  y.assign(y.size(), -1.f);
+  const clock_t before = clock();
+  if (tetris_conv2d_host(&f, x.data(), y.data(), 1, h, h, 1, 0, nullptr) || y != x) return 1;
+  const double used = (double)(clock() - before) / CLOCKS_PER_SEC;
+  fprintf(stderr, "%.2f s of processor time\n", used);
+  return used > 0.6;
+}
+
+static int threads_of_process() {
+  FILE *fh = fopen("/proc/self/status", "r");
+  char line[256];
+  int n = -1;
+  while (fh && fgets(line, sizeof(line), fh)) sscanf(line, "Threads: %d", &n);
+  if (fh) fclose(fh);
+  return n;
+}
+
+// The helpers of all devices together are at most a third of the cores, and a release gives them back
+static int helper_budget() {
+  const auto x = ramp((size_t)16 * 200 * 200);
+  std::vector<float> y(x.size());
+  const int most = std::max(1, (int)std::thread::hardware_concurrency() / 3);
+  for (int round = 0; round < 2; ++round) {
+    for (int dev = 0; dev < 8; ++dev) {
+      tetris_filter f = make_filter(16);
+      f.device = dev;
+      y.assign(y.size(), -1.f);
+      if (tetris_conv2d_host(&f, x.data(), y.data(), 1, 200, 200, 1, 0, nullptr) || y != x) return 1;
+    }
+    const int n = threads_of_process();
+    fprintf(stderr, "%d threads, %d cores\n", n, (int)std::thread::hardware_concurrency());
+    if (n < 2 || n > 1 + most) return 1;
+    tetris_release_workspace();
+    if (threads_of_process() != 1) return 1;
+  }
+  return 0;
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "release_race") return release_race();
@@ -220,6 +269,8 @@ int main(int argc, char **argv) {
   if (what == "download_error") return device_error(false);
   if (what == "upload_mark_error") return upload_mark_error();
   if (what == "no_memory") return no_memory();
+  if (what == "idle_helpers") return idle_helpers();
+  if (what == "helper_budget") return helper_budget();
   fprintf(stderr, "unknown scenario\n");
   return 2;
 }

@@ -38,3 +38,8 @@ def test_an_error_of_the_device_ends_a_staged_copy(harness, scenario):
 
 def test_staged_copies_take_no_memory(harness):
     _run(harness, "no_memory")
+
+
+@pytest.mark.parametrize("scenario", ["idle_helpers", "helper_budget"])
+def test_helpers_take_no_cores_they_do_not_use(harness, scenario):
+    _run(harness, scenario)

@@ -85,6 +85,7 @@ struct Job {
   std::atomic<unsigned char> done[kRing] = {};
   std::atomic<int> users{0};      // threads that hold a pointer to this job
 
+  bool available() const { return next.load() < n && next.load() < ready.load(); }
   // Takes and moves one chunk; false if none may be taken now.
   bool work() {
     int i = next.load(std::memory_order_relaxed);
@@ -125,12 +126,21 @@ class Stager {
         return false;
       }
     if (cudaEventCreateWithFlags(&uploaded_, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); release(); return false; }
-    // four cores move as much as the link carries; the caller is one more
-    const int n = (int)std::min(4u, std::max(1u, std::thread::hardware_concurrency() / 3));
+    // four cores move as much as the link carries; the caller is one more.  All devices together take a third
+    // of the host's cores; on a device that comes too late for them the caller moves the chunks alone.
+    const int most = std::max(1, (int)(std::thread::hardware_concurrency() / 3));
     stop_ = false;
     try {
-      for (int i = 0; i < n; ++i) threads_.emplace_back([this] { serve(); });
-    } catch (...) {  // (the caller then moves the chunks alone)
+      while (threads_.size() < 4) {
+        if (helpers_.fetch_add(1) >= most) { helpers_.fetch_sub(1); break; }
+        try {
+          threads_.emplace_back([this] { serve(); });
+        } catch (...) {
+          helpers_.fetch_sub(1);
+          throw;
+        }
+      }
+    } catch (...) {
     }
     return true;
   }
@@ -139,6 +149,7 @@ class Stager {
     { std::lock_guard<std::mutex> lock(mutex_); stop_ = true; }
     wake_.notify_all();
     for (std::thread &t : threads_) t.join();
+    helpers_.fetch_sub((int)threads_.size());
     threads_.clear();
     if (uploaded_) { cudaEventSynchronize(uploaded_); cudaEventDestroy(uploaded_); uploaded_ = nullptr; }
     for (cudaEvent_t &e : events_) { if (e) cudaEventDestroy(e); e = nullptr; }
@@ -153,7 +164,7 @@ class Stager {
     if (err != cudaSuccess) return err;
     Job job;
     prepare(&job, static_cast<char *>(const_cast<void *>(src)), ring_in_, bytes, true);
-    job.ready.store(std::min(job.n, kRing), std::memory_order_release);
+    job.ready.store(std::min(job.n, kRing));
     post(&job);
     for (int sent = 0, back = 0; sent < job.n && err == cudaSuccess;) {
       if (job.take_done(sent)) {
@@ -164,7 +175,7 @@ class Stager {
         ++sent;
       } else if (back < sent && back + kRing < job.n) {
         const cudaError_t q = cudaEventQuery(events_[back % kRing]);
-        if (q == cudaSuccess) job.ready.store(std::min(job.n, ++back + kRing), std::memory_order_release);  // that chunk of the ring is free again
+        if (q == cudaSuccess) make_ready(&job, std::min(job.n, ++back + kRing));  // that chunk of the ring is free again
         else if (q != cudaErrorNotReady) err = q;
         else if (!job.work()) relax();
       } else if (!job.work()) {
@@ -199,7 +210,7 @@ class Stager {
         ++moved;
       } else if (landed < sent) {
         const cudaError_t q = cudaEventQuery(events_[landed % kRing]);
-        if (q == cudaSuccess) job.ready.store(++landed, std::memory_order_release);
+        if (q == cudaSuccess) make_ready(&job, ++landed);
         else if (q != cudaErrorNotReady) err = q;
         else if (!job.work()) relax();
       } else if (!job.work()) {
@@ -219,25 +230,36 @@ class Stager {
     job->n = (int)((bytes + job->chunk - 1) / job->chunk);
   }
   void post(Job *job) {
-    { std::lock_guard<std::mutex> lock(mutex_); job_ = job; }
+    { std::lock_guard<std::mutex> lock(mutex_); job_ = job; ++jobs_; }
     wake_.notify_all();
+  }
+  void make_ready(Job *job, int chunks) {
+    job->ready.store(chunks);
+    if (sleepers_.load() == 0) return;
+    { std::lock_guard<std::mutex> lock(mutex_); }  // (a helper that has just found nothing to do is waiting by now)
+    wake_.notify_one();
   }
   void finish(Job *job) {  // nobody takes another chunk, and nobody is left inside the job
     job->next.store(job->n, std::memory_order_relaxed);
     { std::lock_guard<std::mutex> lock(mutex_); job_ = nullptr; }
     while (job->users.load(std::memory_order_acquire)) relax();
   }
+  // A helper joins each copy once and looks for chunks for about 250 us; when the device has not got that far
+  // it sleeps until there is one.
   void serve() {
     std::unique_lock<std::mutex> lock(mutex_);
-    for (;;) {
-      wake_.wait(lock, [this] { return stop_ || (job_ && job_->next.load(std::memory_order_relaxed) < job_->n); });
+    for (unsigned joined = 0;;) {
+      sleepers_.fetch_add(1);
+      wake_.wait(lock, [&] { return stop_ || (job_ && (jobs_ != joined || job_->available())); });
+      sleepers_.fetch_sub(1);
       if (stop_) return;
       Job *job = job_;
+      joined = jobs_;
       job->users.fetch_add(1, std::memory_order_relaxed);
       lock.unlock();
-      for (int idle = 0; job->next.load(std::memory_order_relaxed) < job->n;) {
-        if (job->work()) { idle = 0; continue; }
-        if (++idle > 2000) std::this_thread::yield(); else relax();  // (waiting for the device)
+      for (int idle = 0; idle < 5000 && job->next.load(std::memory_order_relaxed) < job->n;) {
+        if (job->work()) idle = 0;
+        else { ++idle; relax(); }
       }
       job->users.fetch_sub(1, std::memory_order_release);
       lock.lock();
@@ -247,11 +269,16 @@ class Stager {
   std::mutex mutex_;
   std::condition_variable wake_;
   Job *job_ = nullptr;
+  unsigned jobs_ = 0;             // copies so far
+  std::atomic<int> sleepers_{0};
+  static std::atomic<int> helpers_;  // of all devices
   bool stop_ = false;
   std::vector<std::thread> threads_;
   char *ring_in_ = nullptr, *ring_out_ = nullptr;
   cudaEvent_t events_[kRing] = {}, uploaded_ = nullptr;
 };
+
+std::atomic<int> Stager::helpers_{0};
 
 std::mutex g_stagers_mutex;
 Stager *g_stagers[kMaxDevices];
