@@ -262,6 +262,26 @@ static int helper_budget() {
   return 0;
 }
 
+// The last upload is still on its way on one stream: an upload on another stream does not wait for it
+static int busy_ring() {
+  tetris_filter f = make_filter(64);
+  f.out_channel = 1;
+  const auto x = ramp((size_t)64 * 64 * 64);
+  std::vector<float> y(64 * 64);
+  cudaStream_t a, b;
+  cudaStreamCreateWithFlags(&a, 0);
+  cudaStreamCreateWithFlags(&b, 0);
+  auto call = [&](cudaStream_t s) { return tetris_conv2d_host(&f, x.data(), y.data(), 1, 64, 64, 1, 0, s); };
+  if (call(a) || g_ring_copies == 0) return 1;
+  int waits = 0;
+  g_query = [](cudaEvent_t) { return cudaErrorNotReady; };
+  g_event_sync = [&](cudaEvent_t) { ++waits; return cudaSuccess; };
+  const int staged = g_ring_copies;
+  if (call(b) || g_ring_copies != staged || waits) return 1;  // by the driver, at once
+  if (call(a) || g_ring_copies == staged || !waits) return 1;  // behind its own upload
+  return g_faults;
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "release_race") return release_race();
@@ -271,6 +291,7 @@ int main(int argc, char **argv) {
   if (what == "no_memory") return no_memory();
   if (what == "idle_helpers") return idle_helpers();
   if (what == "helper_budget") return helper_budget();
+  if (what == "busy_ring") return busy_ring();
   fprintf(stderr, "unknown scenario\n");
   return 2;
 }

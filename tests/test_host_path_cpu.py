@@ -43,3 +43,7 @@ def test_staged_copies_take_no_memory(harness):
 @pytest.mark.parametrize("scenario", ["idle_helpers", "helper_budget"])
 def test_helpers_take_no_cores_they_do_not_use(harness, scenario):
     _run(harness, scenario)
+
+
+def test_an_upload_does_not_wait_for_another_streams(harness):
+    _run(harness, "busy_ring")

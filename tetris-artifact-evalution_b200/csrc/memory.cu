@@ -157,6 +157,10 @@ class Stager {
     ring_in_ = ring_out_ = nullptr;
   }
 
+  // Whether an upload on `st` may use the ring now: the last upload has left it, or is on `st` as well, where this one
+  // comes behind it whichever way it goes.  (On another stream it may stand behind any amount of work.)
+  bool ring_free(cudaStream_t st) { return st == last_ || cudaEventQuery(uploaded_) != cudaErrorNotReady; }
+
   // The caller's array -> device; when this returns the array may be reused, the last copies out of
   // the ring may still be under way on `st`.
   cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st) {
@@ -184,6 +188,7 @@ class Stager {
     }
     finish(&job);
     const cudaError_t marked = cudaEventRecord(uploaded_, st);
+    last_ = st;
     if (err == cudaSuccess) return marked;
     cudaStreamSynchronize(st);  // (copies out of the ring may be under way)
     return err;
@@ -276,6 +281,7 @@ class Stager {
   std::vector<std::thread> threads_;
   char *ring_in_ = nullptr, *ring_out_ = nullptr;
   cudaEvent_t events_[kRing] = {}, uploaded_ = nullptr;
+  cudaStream_t last_ = nullptr;   // of the last upload
 };
 
 std::atomic<int> Stager::helpers_{0};
@@ -343,6 +349,10 @@ void device_free(void *p) {
 // page-locked: then once `st` has passed).
 cudaError_t copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t st) {
   Stager *s = take_stager(src, bytes, kStagedUpload);
+  if (s && !s->ring_free(st)) {
+    s->in_use.unlock();
+    s = nullptr;
+  }
   if (!s) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
   const cudaError_t err = s->upload(dst, src, bytes, st);
   s->in_use.unlock();
