@@ -23,7 +23,8 @@
 
 // ---- the model ----------------------------------------------------------------------------------
 static std::mutex g_model;
-static std::set<void *> g_streams, g_events;
+static std::set<void *> g_streams, g_events, g_recorded;
+static cudaStream_t g_last_upload = nullptr;
 static std::atomic<size_t> g_handles{0x1000};
 static std::atomic<int> g_faults{0}, g_queries{0}, g_waits{0}, g_ring_copies{0}, g_direct_copies{0};
 static std::function<cudaError_t(cudaEvent_t)> g_query;          // answers cudaEventQuery
@@ -87,14 +88,27 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
 cudaError_t cudaEventDestroy(cudaEvent_t e) {
   use_event(e);
   std::lock_guard<std::mutex> lock(g_model);
-  g_events.erase(e);
+  g_events.erase(e); g_recorded.erase(e);
   return cudaSuccess;
 }
-cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { use_event(e); use_stream(s); return cudaSuccess; }
-cudaError_t cudaEventQuery(cudaEvent_t e) { use_event(e); ++g_queries; return g_query ? g_query(e) : cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  use_event(e); use_stream(s);
+  std::lock_guard<std::mutex> lock(g_model);
+  g_recorded.insert(e);
+  return cudaSuccess;
+}
+cudaError_t cudaEventQuery(cudaEvent_t e) {
+  use_event(e);
+  ++g_queries;
+  std::unique_lock<std::mutex> lock(g_model);
+  if (!g_recorded.count(e)) return cudaSuccess;
+  lock.unlock();
+  return g_query ? g_query(e) : cudaSuccess;
+}
 cudaError_t cudaEventSynchronize(cudaEvent_t e) { use_event(e); return g_event_sync ? g_event_sync(e) : cudaSuccess; }
-cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st) {
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind kind, cudaStream_t st) {
   use_stream(st);
+  if (kind == cudaMemcpyHostToDevice) g_last_upload = st;
   ++(in_ring(d) || in_ring(s) ? g_ring_copies : g_direct_copies);
   memcpy(d, s, n);
   return cudaSuccess;
@@ -282,6 +296,24 @@ static int busy_ring() {
   return g_faults;
 }
 
+// A slot that is used again while it works does not hold back the upload of an idle one
+static int slot_in_use() {
+  tetris_filter f = make_filter(4);
+  const auto x = ramp(4 * 9);
+  std::vector<float> y(x.size());
+  auto call = [&](int slot) { return tetris_conv2d_host_async(&f, x.data(), y.data(), 1, 3, 3, 1, 0, slot); };
+  if (call(0)) return 1;
+  const cudaStream_t shared = g_last_upload;
+  g_query = [](cudaEvent_t) { return cudaErrorNotReady; };
+  int waits = 0;
+  g_on_wait = [&](cudaStream_t s) { waits += s == shared; };
+  if (call(0) || g_last_upload == shared) return 1;  // on its own stream
+  if (call(1) || g_last_upload != shared) return 1;  // idle: on the shared one, which waits for nobody
+  g_query = nullptr;
+  if (call(0) || g_last_upload != shared) return 1;
+  return waits || g_faults;
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "release_race") return release_race();
@@ -292,6 +324,7 @@ int main(int argc, char **argv) {
   if (what == "idle_helpers") return idle_helpers();
   if (what == "helper_budget") return helper_budget();
   if (what == "busy_ring") return busy_ring();
+  if (what == "slot_in_use") return slot_in_use();
   fprintf(stderr, "unknown scenario\n");
   return 2;
 }

@@ -47,3 +47,7 @@ def test_helpers_take_no_cores_they_do_not_use(harness, scenario):
 
 def test_an_upload_does_not_wait_for_another_streams(harness):
     _run(harness, "busy_ring")
+
+
+def test_a_slot_at_work_does_not_hold_back_idle_slots(harness):
+    _run(harness, "slot_in_use")

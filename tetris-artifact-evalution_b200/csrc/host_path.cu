@@ -148,10 +148,13 @@ int tetris_conv2d_host_async(const tetris_filter_t *f, const float *h_input_nchw
   float *d_in_nchw = d, *d_in_nhwc = d + in_pad, *d_out_nhwc = d + 2 * in_pad, *d_out_nchw = d + 2 * in_pad + out_pad;
   cudaStream_t st = hs.stream;
   // (the slot's last call has read its input buffer once `computed` has passed, its output buffer once `left` has)
-  TETRIS_CUDA_TRY(cudaStreamWaitEvent(up, hs.computed, 0));
-  TETRIS_CUDA_TRY(cudaMemcpyAsync(d_in_nchw, h_input_nchw, in_elems * sizeof(float), cudaMemcpyHostToDevice, up));
-  TETRIS_CUDA_TRY(cudaEventRecord(hs.arrived, up));
-  TETRIS_CUDA_TRY(cudaStreamWaitEvent(st, hs.arrived, 0));
+  if (cudaEventQuery(hs.computed) == cudaSuccess) {
+    TETRIS_CUDA_TRY(cudaMemcpyAsync(d_in_nchw, h_input_nchw, in_elems * sizeof(float), cudaMemcpyHostToDevice, up));
+    TETRIS_CUDA_TRY(cudaEventRecord(hs.arrived, up));
+    TETRIS_CUDA_TRY(cudaStreamWaitEvent(st, hs.arrived, 0));
+  } else {  // behind the slot's own work: on the shared stream it would hold back the uploads of other slots
+    TETRIS_CUDA_TRY(cudaMemcpyAsync(d_in_nchw, h_input_nchw, in_elems * sizeof(float), cudaMemcpyHostToDevice, st));
+  }
   if ((rc = launch_nchw_to_nhwc(d_in_nchw, d_in_nhwc, s.N, s.IC, s.H, s.W, st))) return rc;
   if ((rc = conv_dispatch_auto(f, d_in_nhwc, d_out_nhwc, s, st))) return rc;
   TETRIS_CUDA_TRY(cudaStreamWaitEvent(st, hs.left, 0));
