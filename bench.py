@@ -32,8 +32,8 @@ from __graft_entry__ import load_package  # noqa: E402
 # of a launch over the algorithmic bytes of the captured layer); the bench scales it to its own
 # mean launch.  The captures are summarised under profiles/.
 NCU_TRAFFIC = {
-    "tensor16_3x3_s1": {"dram_over_algorithmic": 67.9 / 107.5,
-                        "note": "captured on VGG-19 conv3_3 batch 16: 67.9 MB per launch against 107.5 MB "
+    "tensor16_3x3_s1": {"dram_over_algorithmic": 61.1 / 103.5,
+                        "note": "captured on VGG-19 conv3_3 batch 16: 61.1 MB per launch against 103.5 MB "
                                 "algorithmic (outputs still in L2 at kernel end); scaled by algorithmic bytes"},
     "tensor_3x3_s1": {"dram_over_algorithmic": 65.7 / 107.5,
                       "note": "captured on VGG-19 conv3_3 batch 16: 65.7 MB per launch against 107.5 MB "
@@ -44,8 +44,8 @@ NCU_TRAFFIC = {
 }
 VARIANT_NAMES = {0: "auto", 1: "generic", 2: "tiled", 4: "tensor", 5: "tensor16"}
 ARITH = {"tensor16": "3xFP16 split on the tensor cores (x_hi*w_hi + x_lo*w_hi + x_hi*w_lo, 11-bit halves), FP32 "
-                     "accumulate, partial sums added on the CUDA cores every 48 MMAs; tiles with out-of-range "
-                     "activations computed again with fitted scales",
+                     "accumulate, partial sums added on the CUDA cores every 1 to 8 K steps of 6 MMAs (4 on stacked "
+                     "tiles); CTAs with out-of-range activations compute their tiles again with fitted scales",
          "tensor": "3xTF32 split on the tensor cores (x_hi*w_hi + x_lo*w_hi + x_hi*w_lo), FP32 accumulate, "
                    "partial sums added on the CUDA cores every 48 MMAs",
          "tiled": "FP32 FMA on the CUDA cores, taps added in the reference's (ic, r, s) order",

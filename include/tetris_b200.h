@@ -67,7 +67,7 @@ enum {
                                  16-byte aligned input.  Where the largest |activation| of
                                  all tiles that one CTA computes is 2048 or more (infinity) or
                                  below 2^-8, that CTA computes them again in the same launch,
-                                 with scales fitted to them: 2.6 to 3.9 times the time of an
+                                 with scales fitted to them: 1.8 to 3.9 times the time of an
                                  ordinary launch (TETRIS_VARIANT_TENSOR has no such window).
                                  Else an activation's error is at most 2^-22 of it or 2^-29   */
 };
@@ -153,9 +153,9 @@ int tetris_conv2d_launch_ex(const tetris_filter_t *f, const float *d_input_nhwc,
 
 /*
  * The same launch with options fused into the kernel's store.  flags: TETRIS_FUSE_RELU -- the
- * output is max(y, 0).  The tensor-core variants rectify at their own store (and do not split a
- * tile's K range for such a launch); the other kernels are followed by an in-place pass on the
- * same stream.  No counterpart in the reference, whose kernel writes the plain convolution
+ * output is max(y, 0).  The tensor-core variants and the depthwise kernels rectify at their own
+ * store (split TF32 does not split a tile's K range for such a launch); the other kernels are
+ * followed by an in-place pass on the same stream.  No counterpart in the reference, whose kernel writes the plain convolution
  * (Tetris/spconv2d_kernel.cu:140-158).
  */
 enum { TETRIS_FUSE_RELU = 1 };
@@ -220,7 +220,7 @@ int tetris_conv2d_tune(const tetris_filter_t *f, const float *d_input_nhwc, floa
 /*
  * Which kernel a TETRIS_VARIANT_AUTO launch of this shape uses at the moment (the tuned choice if
  * tetris_conv2d_tune ran for the shape, else the cost models'): *variant receives
- * TETRIS_VARIANT_TILED, _TENSOR or _GENERIC (TETRIS_VARIANT_AUTO for a depthwise filter, which
+ * TETRIS_VARIANT_TILED, _TENSOR, _TENSOR16 or _GENERIC (TETRIS_VARIANT_AUTO for a depthwise filter, which
  * has a single kernel).  No counterpart in the reference, which has one kernel.
  */
 int tetris_conv2d_choice(const tetris_filter_t *f, int batch_size, int img_h, int img_w, int stride,
@@ -238,9 +238,11 @@ int tetris_conv2d_host(const tetris_filter_t *f, const float *h_input_nchw,
                        int padding, void *stream);
 
 /*
- * The same data path without the final wait: the copies, transposes and the convolution are
- * queued on an internal stream selected by `slot` (0..3; each slot has its own stream and
- * workspace on the filter's device) and the call returns.  tetris_host_sync(device, slot) waits
+ * The same data path without the final wait: transposes and convolution are queued on an internal
+ * stream selected by `slot` (0..3; each slot has its own stream and workspace on the filter's
+ * device), the copies on two streams of the device that all slots share, one per direction, and the
+ * call returns.  Results leave in the order of the calls.  A slot that is used again before it has been
+ * waited for uploads behind its own work instead, a little slower.  tetris_host_sync(device, slot) waits
  * for a slot (slot < 0: all of them); until then neither host buffer may be touched.  Calls that
  * alternate between slots overlap the upload of one with the download of the other.  Host buffers
  * should be page-locked for the copies to be asynchronous.  No counterpart in the reference,

@@ -393,9 +393,9 @@ def test_tensor16_random_shapes(tb, torch_cuda, oracle, seed):
 def test_tensor16_value_ranges(tb, torch_cuda, oracle):
     """Split FP16 keeps FP32 accuracy over the range FP16 can hold -- large activations (up to
     ~3e4), tiny ones (1e-7: below FP16's normal range, the absolute error stays far under the
-    floor), weights of very different magnitudes (|w| from 1e-6 to 30) -- and a launch whose
-    activations do not fit FP16's window (2048 and more, or all below 2^-8) is recomputed by the
-    split-TF32 variant behind it: every case has to meet the bar of the path, with the absolute
+    floor), weights of very different magnitudes (|w| from 1e-6 to 30) -- and a CTA whose
+    activations do not fit FP16's window (2048 and more, or all below 2^-8) computes its tiles again in
+    the same launch, in bands scaled to them: every case has to meet the bar of the path, with the absolute
     floor scaled like the activations."""
     torch = torch_cuda
     rng = np.random.default_rng(77)
@@ -420,8 +420,8 @@ def test_tensor16_value_ranges(tb, torch_cuda, oracle):
     got = device_conv(tb, torch_cuda, f, x, 1, 1, VARIANTS["tensor16"])
     bad, max_rel, _ = oracle.compare(got, oracle.host_conv2d(x, filt, 1, 1))
     assert bad == 0, "plain launch after an out-of-range one: %d elements off (max rel %.3g)" % (bad, max_rel)
-    # output channels whose weights differ by seven orders of magnitude share one filter-wide
-    # scale; each channel is held to the bar of the path with the floor scaled like its weights
+    # output channels whose weights differ by seven orders of magnitude, each with a scale of its
+    # own; each channel is held to the bar of the path with the floor scaled like its weights
     # (against a floor of 1e-5 the CPU path's own FP32 rounding would show on the large channels)
     chan = np.exp(rng.uniform(np.log(2e-5), np.log(600.0), (oc, 1, 1, 1))).astype(np.float32)
     wide = filt * chan

@@ -1,7 +1,7 @@
 """GPU: the split-FP16 tensor-core kernel at the edges of its tile geometries -- strides 1 to 4 (input
 phases), stacked tiles (at most 64 channels), K ranges cut over a cluster, tiles of consecutive
 pixels, of whole padded rows and of 8-column blocks with several images, channel counts around
-the tiles' -- and its second pass for activations outside FP16's window."""
+the tiles' -- its passes for activations outside FP16's window, and its error against 64 bits."""
 import numpy as np
 import pytest
 
@@ -93,7 +93,13 @@ def test_activations_outside_the_window(tb, torch_cuda, oracle, case):
     want = oracle.host_conv2d(x, filt, stride, pad, threads=True)
     far = np.ones(got.shape, bool)
     far[0, :, max(0, 5 + pad - ks) // stride: (5 + pad) // stride + 1, max(0, 5 + pad - ks) // stride: (5 + pad) // stride + 1] = False
-    assert not np.isfinite(got[~far]).all()
+    reads = np.zeros(got.shape, bool)  # outputs with a nonzero weight on the infinity
+    for r in range(ks):
+        for s in range(ks):
+            p, q = 5 + pad - r, 5 + pad - s
+            if p % stride == 0 and q % stride == 0 and 0 <= p // stride < got.shape[2] and 0 <= q // stride < got.shape[3]:
+                reads[0, :, p // stride, q // stride] |= filt[:, 3, r, s] != 0
+    assert reads.any() and not np.isfinite(got[reads]).any()
     assert oracle.compare(got[far], want[far])[0] == 0
     f.close()
     g.close()
@@ -199,4 +205,22 @@ def test_untuned_choice_on_odd_channel_counts(tb, torch_cuda, oc, sparsity):
 
     kernels = {v: per_launch(v) for v in (tb.VARIANT_TILED, tb.VARIANT_TENSOR16)}
     assert kernels[tb.auto_choice(f, n, h, h, 1, 1)] < 1.25 * min(kernels.values())
+    f.close()
+
+
+def test_a_tiny_image_beside_ordinary_ones(tb, torch_cuda, oracle):
+    """One maximum per CTA decides about its scales, so an image of activations near 1e-6 may be computed at the
+    scale of the images that share its CTA.  Then each activation is held to 2^-29 (half the spacing of FP16's
+    subnormal numbers, 2^-25, at the scale 16), and an output to the sum of its |weights| times that, the
+    rounding of the tiny sum itself aside; the ordinary images keep the bar of the path."""
+    n, ic, h, oc = 48, 64, 28, 128  # several tiles per CTA
+    filt, x = _layer((n, ic, h, h, oc, 3, 1, 1), 11)
+    x[17] *= np.float32(2.0 ** -20)
+    f = tb.SparseFilter(filt, ic, oc, 3)
+    got = _run(tb, torch_cuda, f, x, 1, 1, False)
+    want = oracle.host_conv2d(x, filt, 1, 1, threads=True, skip_zero=True)
+    rest = np.arange(n) != 17
+    assert oracle.compare(got[rest], want[rest])[0] == 0
+    bound = np.abs(filt).sum((1, 2, 3)).reshape(-1, 1, 1) * 2.0 ** -29 + 1e-5 * np.abs(want[17]).max()
+    assert (np.abs(got[17] - want[17]) <= bound).all()
     f.close()

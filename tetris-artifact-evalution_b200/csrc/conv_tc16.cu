@@ -17,8 +17,9 @@
 // recomputes is its own output.
 //
 // The tensor core truncates when it adds into its FP32 accumulator, so the accumulation chain is
-// cut every 8 K steps (48 MMAs): the tensor core accumulates from zero into one of two partial
-// accumulators and CUDA-core warps add the partials to a running sum in registers.
+// cut every 1 to 8 K steps of 6 MMAs (4 on stacked tiles; see partial_steps): the tensor core accumulates
+// from zero into one of two partial accumulators and CUDA-core warps add the partials to a running sum
+// in registers.
 //
 // Structure.  D[channel][pixel]: the M side is 128 output channels (the weights), the N side up to
 // 256 output pixels (the activations), K = (32-channel chunk, filter tap).  Both operands are read
@@ -27,8 +28,9 @@
 // N = 128 needs the whole shared-memory pipe while N = 256 leaves a quarter of it for the weight
 // copies and the conversion; with the weights on the M side one 16 KB weight image serves 256
 // pixels (L2 -> SM weight traffic halved against 128-pixel tiles), and an accumulator row is an
-// output channel, so a warp stores one pixel's 32 consecutive channels as one 128-byte line
-// without staging, whatever the channel count or alignment.
+// output channel, so a warp turns 16 pixels x 32 consecutive channels over in a small staging block, from
+// where TMA stores carry 8 pixels at a time on, or, where the channel count is no multiple of 4 or the
+// output not 16-byte aligned, the warp itself, a pixel's 32 channels as one line.
 //   * warp 0 (one thread): TMA loads of activation patches (tile + halo, 32 channels, out-of-range
 //     coordinates zero-filled = the padding) and bulk copies of weight images, each into a ring;
 //   * converter warps: a landed patch, once, in place: each 128-byte row of 32 FP32 channels
@@ -294,6 +296,8 @@ __device__ __noinline__ void scale_columns(uint32_t taddr, int ncols, float f) {
 // NMAX: most pixels of a tile.  A summing warp keeps NMAX / 2 running sums per thread, which sets
 // the register count: 12 warps (2 of them converters) for 256 pixels, 16 warps (6 converters) for
 // 128.  STACK: at most 64 output channels, {w_hi, w_lo} stacked on the M side.
+// The 256-pixel instances spill: 168 registers a thread hold 128 running sums, and ptxas reports 32 (stacked 64)
+// bytes of spill stores and 52 (100) of loads.
 template <int NMAX> struct Roles {
   static constexpr int kConv = NMAX == 256 ? 2 : 6;
   static constexpr int kFirstSum = 2 + kConv;
