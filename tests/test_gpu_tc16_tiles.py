@@ -224,3 +224,13 @@ def test_a_tiny_image_beside_ordinary_ones(tb, torch_cuda, oracle):
     bound = np.abs(filt).sum((1, 2, 3)).reshape(-1, 1, 1) * 2.0 ** -29 + 1e-5 * np.abs(want[17]).max()
     assert (np.abs(got[17] - want[17]) <= bound).all()
     f.close()
+
+
+@pytest.mark.parametrize("n,h,w,ks,pad", [(2 ** 31 - 300, 1, 1, 1, 0), (1, 2 ** 31 - 300, 1, 3, 1), (1, 1, 2 ** 31 - 300, 3, 1)])
+def test_shapes_past_32_bit_coordinates_are_refused(tb, torch_cuda, n, h, w, ks, pad):
+    """Refused on the host, before anything is launched: the last tile would reach past 2^31."""
+    f = tb.SparseFilter(np.ones((8, 8, ks, ks), np.float32), 8, 8, ks)
+    buf = torch_cuda.zeros(64, device="cuda")
+    with pytest.raises(tb.TetrisError, match="split-FP16"):
+        tb.sparse_conv2d(f, buf, buf, n, h, w, 1, pad, variant=tb.VARIANT_TENSOR16)
+    f.close()

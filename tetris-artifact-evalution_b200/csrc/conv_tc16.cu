@@ -1071,6 +1071,7 @@ bool plan_geometry(const Tc16State &t, const ConvShape &s, Geometry *best) {
       continue;
     }
     // whole padded rows
+    if ((long long)s.OH * (s.OW + amax) >= (1ll << 31) - 1024) continue;
     g.mode = kFlat;
     g.PW = s.OW + amax;
     g.TH = s.OH;
@@ -1201,7 +1202,9 @@ int conv_tc16_prepare(tetris_filter *f, const float *d_dense, WeightImages *w) {
 bool conv_tc16_supported(const tetris_filter *f, const ConvShape &s) {
   if (!f->tc16_state || f->groups != 1) return false;
   if (s.S < 1 || s.S > 4 || s.N < 1 || s.OH < 1 || s.OW < 1) return false;
-  return (long long)s.N * s.OH * s.OW < (1ll << 31);
+  // (pixel numbers and image coordinates are 32-bit, and a tile reaches up to 256 of them past the last one)
+  constexpr long long kMost = (1ll << 31) - 1024;
+  return (long long)s.N * s.OH * s.OW < kMost && s.H + 2ll * s.P < kMost && s.W + 2ll * s.P < kMost;
 }
 
 // Estimated clocks of a launch (negative: the shape is not covered).
